@@ -55,18 +55,18 @@ am24_status make_map(am24_handle h, CUtensorMap *map, const float *base, int K, 
 }
 
 // K-major 16-bit operand [rows][ld] (ld in elements; BF16, or FP16 when
-// fp16), loaded as 32 x box_rows tiles (64-byte rows, 64-byte swizzle), as the
-// 16-bit pair GEMMs read them.
+// fp16), loaded as 64 x box_rows tiles (128-byte rows, 128-byte swizzle: two K
+// blocks), as the 16-bit pair GEMMs read them.
 am24_status make_map_bf16(am24_handle h, CUtensorMap *map, const uint16_t *base, int K, int rows,
                           int ld, int box_rows, bool fp16) {
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)ld * sizeof(uint16_t)};
-  cuuint32_t box[2] = {(cuuint32_t)PAIR_BK_BF16, (cuuint32_t)box_rows};
+  cuuint32_t box[2] = {2u * (cuuint32_t)PAIR_BK_BF16, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = h->encode(map, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
                          2, const_cast<uint16_t *>(base),
                          dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
     return fail(AM24_ERR_CUDA, "cuTensorMapEncodeTiled (BF16) failed with code " +
@@ -764,7 +764,7 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
   // candidates (AM24_SELECT_LIST=0 leaves the gather to the select kernels)
   bool lists = is_constrained(settings->formulation);
   if (const char *e = getenv("AM24_SELECT_LIST")) lists = lists && atoi(e) != 0;
-  const int bk2 = d.pair2 ? PAIR_BK_TF32 : d.bk;  // K box of the TF32 maps of V = B^T Z
+  const int bk2 = d.pair2 ? 2 * PAIR_BK_TF32 : d.bk;  // K box of the TF32 maps of V = B^T Z
   const int kb_total1 = (M.n + d.bk - 1) / d.bk;
   choose_splits(d.m_tiles1 * d.n_tiles1, kb_total1, num_sms(), &d.splits1, &d.kbps1);
   d.ws_len = ws_floats(d.splits1, d.m_tiles1, d.n_tiles1, d.bn1);

@@ -2362,16 +2362,16 @@ cudaError_t dispatch_gemm2(const BatchDev &b, const TensorMaps &tm, const GemmSh
       GemmShape s2 = sh;
       s2.row_scale = b.row_scale;
       if (l1_variance)  // B = sgn(z), exact
-        return run_gemm_pair<PairFP16x2A, 256, 8>(tm.a2_h0, tm.a2_h1, tm.b2_h0, tm.b2_h0, s2, epi,
+        return run_gemm_pair<PairFP16x2A, 256, 4>(tm.a2_h0, tm.a2_h1, tm.b2_h0, tm.b2_h0, s2, epi,
                                                   st);
       s2.col_scale = b.z_scale;
-      return run_gemm_pair<PairFP16x3, 256, 6>(tm.a2_h0, tm.a2_h1, tm.b2_h0, tm.b2_h1, s2, epi,
+      return run_gemm_pair<PairFP16x3, 256, 3>(tm.a2_h0, tm.a2_h1, tm.b2_h0, tm.b2_h1, s2, epi,
                                                st);
     }
     if (b.bf16_2 && l1_variance)
-      return run_gemm_pair<PairBF16x3A, 256, 6>(tm.a2_b0, tm.a2_b1, tm.a2_b2, tm.b2_b, sh, epi,
+      return run_gemm_pair<PairBF16x3A, 256, 3>(tm.a2_b0, tm.a2_b1, tm.a2_b2, tm.b2_b, sh, epi,
                                                 st);
-    return run_gemm_pair<PairTF32x3, 256, 6>(tm.a2_hi, tm.a2_lo, tm.b2_hi, tm.b2_lo, sh, epi, st);
+    return run_gemm_pair<PairTF32x3, 256, 3>(tm.a2_hi, tm.a2_lo, tm.b2_hi, tm.b2_lo, sh, epi, st);
   }
   return dispatch_gemm(b.bn2, b.bk, tm.a2_hi, tm.a2_lo, tm.b2_hi, tm.b2_lo, sh, epi, st);
 }
@@ -2632,7 +2632,7 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
     GemmShape gp = g1;
     gp.row_scale = b.bt_row_scale;
     gp.col_scale = b.v_scale;
-    e = run_gemm_pair<PairFP16x3, 256, 6>(tm.a1_h0, tm.a1_h1, tm.b1_h0, tm.b1_h1, gp, ep, st,
+    e = run_gemm_pair<PairFP16x3, 256, 3>(tm.a1_h0, tm.a1_h1, tm.b1_h0, tm.b1_h1, gp, ep, st,
                                           b.splits1p);
   } else {
     e = dispatch_gemm(b.bn1, b.bk, tm.a1_hi, tm.a1_lo, tm.b1_hi, tm.b1_lo, g1, ep, st);
@@ -2687,10 +2687,10 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
       if (b.mixed_fp16) {
         gl.row_scale = b.row_scale;
         gl.col_scale = is_l1_variance(f) ? nullptr : b.z_scale;  // sgn(z) is exact
-        e2 = run_gemm_pair<PairFP16x1, 256, 12>(tm.a2_h0, tm.b2_h0, tm.a2_h0, tm.b2_h0, gl, epi,
+        e2 = run_gemm_pair<PairFP16x1, 256, 6>(tm.a2_h0, tm.b2_h0, tm.a2_h0, tm.b2_h0, gl, epi,
                                                 st);
       } else {
-        e2 = run_gemm_pair<PairBF16x1, 256, 12>(tm.a2_b0, tm.b2_b, tm.a2_b0, tm.b2_b, gl, epi,
+        e2 = run_gemm_pair<PairBF16x1, 256, 6>(tm.a2_b0, tm.b2_b, tm.a2_b0, tm.b2_b, gl, epi,
                                                 st);
       }
       if (e2 != cudaSuccess) return e2;

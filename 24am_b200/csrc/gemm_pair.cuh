@@ -18,8 +18,12 @@
 // and accumulates 128 rows x BN columns into each CTA's tensor memory.  The
 // tensor-core work per SM is that of a one-CTA kernel with a 128 x BN tile,
 // but each SM streams 128 + BN/2 operand rows per K slab instead of 128 + BN.
-// Shared-memory rows are 64 bytes of K (64-byte swizzle) in both schemes, so a
-// stage is 32 KB either way.
+// A shared-memory row is 128 bytes of K (128-byte swizzle) in every scheme.
+// With one MMA per K step (PairFP16x1) the loads bound the kernel: 64-byte rows
+// took 4.72 ms at 65536 x 8192 x 4096, 128-byte rows (whole L2 lines per
+// request, half the barrier traffic) take 3.59 ms; the split schemes gain 2-4 %
+// and run at the rate the power limit allows.  A stage holds a slab of PAIR_SLAB = 2 K blocks of 64 bytes, and a unit whose
+// blocks are odd in number issues the MMAs of the last slab's first block only.
 //
 // The tensor-core FP32 accumulation does not round to nearest; as in
 // gemm_tf32x3.cuh each TMEM buffer takes PROMO K slabs (S::PROMO_K elements: 48
@@ -62,9 +66,12 @@ __device__ __forceinline__ Unit decode_pair_unit(const GemmShape &s, int u, int 
   return r;
 }
 
+// Shared-memory descriptor code of the 128-byte swizzle.
+constexpr uint32_t PAIR_SWIZZLE = 2u;
+
 // Operand schemes.  NA + NB <= 4 planes, passed as the kernel's first tensor
 // maps (A planes first; the others are not read); BK = K elements per 64-byte
-// shared-memory row.
+// half shared-memory row.
 struct PairTF32x3 {
   static constexpr int NA = 2, NB = 2, BK = PAIR_BK_TF32;
   // K elements per TMEM chunk before the FP32 promotion: 48 MMAs accumulate
@@ -78,10 +85,10 @@ struct PairTF32x3 {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      const uint64_t dah = sdesc_kmajor(a[0] + off, sbo, 4u);
-      const uint64_t dal = sdesc_kmajor(a[1] + off, sbo, 4u);
-      const uint64_t dbh = sdesc_kmajor(b[0] + off, sbo, 4u);
-      const uint64_t dbl = sdesc_kmajor(b[1] + off, sbo, 4u);
+      const uint64_t dah = sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE);
+      const uint64_t dal = sdesc_kmajor(a[1] + off, sbo, PAIR_SWIZZLE);
+      const uint64_t dbh = sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE);
+      const uint64_t dbl = sdesc_kmajor(b[1] + off, sbo, PAIR_SWIZZLE);
       mma_tf32_pair(d, dal, dbh, ID, (first && kk == 0) ? 0u : 1u);
       mma_tf32_pair(d, dah, dbl, ID, 1u);
       mma_tf32_pair(d, dah, dbh, ID, 1u);
@@ -101,10 +108,10 @@ struct PairBF16x3A {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      const uint64_t db = sdesc_kmajor(b[0] + off, sbo, 4u);
-      mma_bf16_pair(d, sdesc_kmajor(a[2] + off, sbo, 4u), db, ID, (first && kk == 0) ? 0u : 1u);
-      mma_bf16_pair(d, sdesc_kmajor(a[1] + off, sbo, 4u), db, ID, 1u);
-      mma_bf16_pair(d, sdesc_kmajor(a[0] + off, sbo, 4u), db, ID, 1u);
+      const uint64_t db = sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE);
+      mma_bf16_pair(d, sdesc_kmajor(a[2] + off, sbo, PAIR_SWIZZLE), db, ID, (first && kk == 0) ? 0u : 1u);
+      mma_bf16_pair(d, sdesc_kmajor(a[1] + off, sbo, PAIR_SWIZZLE), db, ID, 1u);
+      mma_bf16_pair(d, sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE), db, ID, 1u);
     }
   }
   static constexpr uint32_t FMT = 1u;
@@ -126,10 +133,10 @@ struct PairFP16x3 {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      const uint64_t da0 = sdesc_kmajor(a[0] + off, sbo, 4u);
-      const uint64_t db0 = sdesc_kmajor(b[0] + off, sbo, 4u);
-      mma_f16_pair(d, sdesc_kmajor(a[1] + off, sbo, 4u), db0, ID, (first && kk == 0) ? 0u : 1u);
-      mma_f16_pair(d, da0, sdesc_kmajor(b[1] + off, sbo, 4u), ID, 1u);
+      const uint64_t da0 = sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE);
+      const uint64_t db0 = sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE);
+      mma_f16_pair(d, sdesc_kmajor(a[1] + off, sbo, PAIR_SWIZZLE), db0, ID, (first && kk == 0) ? 0u : 1u);
+      mma_f16_pair(d, da0, sdesc_kmajor(b[1] + off, sbo, PAIR_SWIZZLE), ID, 1u);
       mma_f16_pair(d, da0, db0, ID, 1u);
     }
   }
@@ -146,9 +153,9 @@ struct PairFP16x2A {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      const uint64_t db = sdesc_kmajor(b[0] + off, sbo, 4u);
-      mma_f16_pair(d, sdesc_kmajor(a[1] + off, sbo, 4u), db, ID, (first && kk == 0) ? 0u : 1u);
-      mma_f16_pair(d, sdesc_kmajor(a[0] + off, sbo, 4u), db, ID, 1u);
+      const uint64_t db = sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE);
+      mma_f16_pair(d, sdesc_kmajor(a[1] + off, sbo, PAIR_SWIZZLE), db, ID, (first && kk == 0) ? 0u : 1u);
+      mma_f16_pair(d, sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE), db, ID, 1u);
     }
   }
   static constexpr uint32_t FMT = 0u;
@@ -166,7 +173,7 @@ struct PairBF16x1 {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      mma_bf16_pair(d, sdesc_kmajor(a[0] + off, sbo, 4u), sdesc_kmajor(b[0] + off, sbo, 4u), ID,
+      mma_bf16_pair(d, sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE), sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE), ID,
                     (first && kk == 0) ? 0u : 1u);
     }
   }
@@ -189,16 +196,19 @@ struct PairFP16x1 {
 #pragma unroll
     for (int kk = 0; kk < 2; kk++) {
       const uint32_t off = kk * 32;
-      mma_f16_pair(d, sdesc_kmajor(a[0] + off, sbo, 4u), sdesc_kmajor(b[0] + off, sbo, 4u), ID,
+      mma_f16_pair(d, sdesc_kmajor(a[0] + off, sbo, PAIR_SWIZZLE), sdesc_kmajor(b[0] + off, sbo, PAIR_SWIZZLE), ID,
                    (first && kk == 0) ? 0u : 1u);
     }
   }
   static constexpr uint32_t FMT = 0u;
 };
 
+// K blocks (S::BK elements, 64 bytes a row) per stage.
+constexpr int PAIR_SLAB = 2;
+
 template <class S, int BN, int STAGES>
 struct PairSmem {
-  static constexpr int ROW = 64;  // bytes of K per shared-memory row
+  static constexpr int ROW = 64 * PAIR_SLAB;  // bytes of K per shared-memory row
   static constexpr int A_BYTES = GEMM_BM * ROW;
   static constexpr int B_BYTES = (BN / 2) * ROW;
   static constexpr int STAGE_BYTES = S::NA * A_BYTES + S::NB * B_BYTES;
@@ -217,6 +227,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
   using L = PairSmem<S, BN, STAGES>;
   constexpr int BK = S::BK;
   static_assert(S::NA + S::NB <= 4, "at most four operand planes");
+  static_assert(PROMO % PAIR_SLAB == 0, "a promotion chunk is whole slabs");
   static_assert(BN % 32 == 0 && BN >= 64 && BN <= 256, "BN must be a multiple of 32 in [64,256]");
   constexpr uint32_t SBO = L::ROW * 8;  // bytes between 8-row core-matrix groups
   constexpr uint32_t TMEM_COLS = (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
@@ -278,7 +289,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       uint32_t armed_parity = 0;
       for (int u = pair; u < shape.num_units && !*abort; u += pairs) {
         const Unit t = decode_pair_unit(shape, u, rank);
-        for (int kb = t.kb0; kb < t.kb1; kb++) {
+        for (int kb = t.kb0; kb < t.kb1; kb += PAIR_SLAB) {
           if (!mbar_wait_bounded(&empty[stage], phase ^ 1u, abort, shape.status,
                                  DEV_ERR_TIMEOUT_PRODUCER, tmo))
             break;
@@ -339,7 +350,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-          for (int kb = c0; kb < c1; kb++) {
+          for (int kb = c0; kb < c1; kb += PAIR_SLAB) {
             if (!mbar_wait_bounded(&full[stage], phase, abort, shape.status,
                                    DEV_ERR_TIMEOUT_MMA_SMEM, tmo)) {
               ok = false;
@@ -353,6 +364,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 #pragma unroll
             for (int i = 0; i < S::NB; i++) b[i] = base + S::NA * L::A_BYTES + i * L::B_BYTES;
             S::template k_block<IDESC>(d_tmem, a, b, SBO, kb == c0);
+            if (kb + 1 < c1) {
+#pragma unroll
+              for (int i = 0; i < S::NA; i++) a[i] += 64;
+#pragma unroll
+              for (int i = 0; i < S::NB; i++) b[i] += 64;
+              S::template k_block<IDESC>(d_tmem, a, b, SBO, false);
+            }
             mma_commit_pair(&empty[stage], BOTH);
             if (++stage == STAGES) {
               stage = 0;

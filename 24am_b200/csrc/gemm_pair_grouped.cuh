@@ -47,7 +47,7 @@ __device__ __forceinline__ void tensormap_acquire(const CUtensorMap *map) {
 
 template <int BN>
 struct GPairSmem {
-  static constexpr int ROW = 64;
+  static constexpr int ROW = 64 * PAIR_SLAB;
   static constexpr int A_BYTES = GEMM_BM * ROW;
   static constexpr int B_BYTES = (BN / 2) * ROW;
   static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
@@ -253,7 +253,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         for (int i = 0; i < nb; i++) tensormap_acquire(mb[i]);
         const uint32_t bytes = 2u * (uint32_t)(na * L::A_BYTES + nb * L::B_BYTES);
         const Unit &t = gu.t;
-        for (int kb = t.kb0; kb < t.kb1; kb++) {
+        for (int kb = t.kb0; kb < t.kb1; kb += PAIR_SLAB) {
           if (!mbar_wait_bounded(&empty[stage], phase ^ 1u, abort, status,
                                  DEV_ERR_TIMEOUT_PRODUCER, tmo))
             break;
@@ -310,7 +310,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-          for (int kb = c0; kb < c1; kb++) {
+          for (int kb = c0; kb < c1; kb += PAIR_SLAB) {
             if (!mbar_wait_bounded(&full[stage], phase, abort, status, DEV_ERR_TIMEOUT_MMA_SMEM,
                                    tmo)) {
               ok = false;
@@ -318,18 +318,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
             }
             tc_fence_after();
             const uint32_t base = smem_u32(smem + stage * L::STAGE_BYTES);
-            const uint32_t a[2] = {base, base + L::A_BYTES};
-            const uint32_t bq = base + 2 * L::A_BYTES;
-            const bool first = kb == c0;
-            if (gu.scheme == GS_FP16X3) {
-              const uint32_t b[2] = {bq, bq + L::B_BYTES};
-              PairFP16x3::k_block<ID_F16>(d_tmem, a, b, SBO, first);
-            } else if (gu.scheme == GS_FP16X2A) {
-              const uint32_t b[1] = {bq};
-              PairFP16x2A::k_block<ID_F16>(d_tmem, a, b, SBO, first);
-            } else {
-              const uint32_t a1[1] = {base}, b[1] = {bq};
-              PairFP16x1::k_block<ID_F16>(d_tmem, a1, b, SBO, first);
+            for (int h = 0; h < PAIR_SLAB && kb + h < c1; h++) {
+              const uint32_t ao = base + 64 * h;
+              const uint32_t a[2] = {ao, ao + L::A_BYTES};
+              const uint32_t bq = ao + 2 * L::A_BYTES;
+              const bool first = kb + h == c0;
+              if (gu.scheme == GS_FP16X3) {
+                const uint32_t b[2] = {bq, bq + L::B_BYTES};
+                PairFP16x3::k_block<ID_F16>(d_tmem, a, b, SBO, first);
+              } else if (gu.scheme == GS_FP16X2A) {
+                const uint32_t b[1] = {bq};
+                PairFP16x2A::k_block<ID_F16>(d_tmem, a, b, SBO, first);
+              } else {
+                const uint32_t a1[1] = {ao}, b[1] = {bq};
+                PairFP16x1::k_block<ID_F16>(d_tmem, a1, b, SBO, first);
+              }
             }
             mma_commit_pair(&empty[stage], BOTH);
             if (++stage == STAGES) {

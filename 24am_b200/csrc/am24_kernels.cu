@@ -1239,9 +1239,77 @@ __device__ void bitonic_desc(T *a, int len) {
   }
 }
 
+constexpr int SELECT_THREADS = 256;  // block size of both selects
+
+// Descending sort of a[0..c) (zeros taken beyond, up to the next power of two),
+// E = 1, 2, 4, 8 or 16 elements per thread of a SELECT_THREADS block in
+// registers: a bitonic network whose exchanges run inside a thread (distances
+// below E), by shuffles (below 32 E) and only beyond that through shared memory.
+// Bound by instruction issue: the same network on shared memory pays a block
+// barrier and two round trips for every one of its stages.
+template <int E>
+__device__ __noinline__ void sort_desc_regs(uint64_t *a, int c, int len) {
+  const int t = threadIdx.x;
+  uint64_t v[E];
+#pragma unroll
+  for (int e = 0; e < E; e++) {
+    const int i = e * SELECT_THREADS + t;
+    v[e] = i < c ? a[i] : 0ull;
+  }
+  auto pick = [](uint64_t x, uint64_t y, bool larger) { return (x > y) == larger ? x : y; };
+  // element t * E + e; the one at distance j is in this thread, lane or warp
+  for (int k = 2; k <= len; k <<= 1) {
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= 32 * E) {
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < E; e++) a[e * SELECT_THREADS + t] = v[e];
+        __syncthreads();
+        const int o = t ^ (j / E);
+        const bool larger = ((t * E & k) == 0) == ((t * E & j) == 0);
+#pragma unroll
+        for (int e = 0; e < E; e++) v[e] = pick(v[e], a[e * SELECT_THREADS + o], larger);
+      } else if (j >= E) {
+        const bool larger = (((t * E) & k) == 0) == (((t * E) & j) == 0);
+#pragma unroll
+        for (int e = 0; e < E; e++)
+          v[e] = pick(v[e], __shfl_xor_sync(FULL, v[e], j / E), larger);
+      } else {
+#pragma unroll
+        for (int q = 1; q < E; q <<= 1) {
+          if (j != q) continue;
+#pragma unroll
+          for (int e = 0; e < E; e++) {
+            if (e & q) continue;
+            const bool desc = ((t * E + e) & k) == 0;
+            const uint64_t x = v[e], y = v[e | q];
+            v[e] = pick(x, y, desc);
+            v[e | q] = pick(x, y, !desc);
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < E; e++) a[t * E + e] = v[e];
+  __syncthreads();
+}
+// a[0..c) descending, c <= cap (a power of two, at most 16 * SELECT_THREADS; a
+// has room for max(cap, SELECT_THREADS)).
+__device__ __forceinline__ void sort_pairs_desc(uint64_t *a, int c, int cap) {
+  int len = 1;
+  while (len < c) len <<= 1;
+  if (len <= SELECT_THREADS) sort_desc_regs<1>(a, c, len);
+  else if (len == 2 * SELECT_THREADS) sort_desc_regs<2>(a, c, len);
+  else if (len == 4 * SELECT_THREADS) sort_desc_regs<4>(a, c, len);
+  else if (len == 8 * SELECT_THREADS || cap <= 8 * SELECT_THREADS) sort_desc_regs<8>(a, c, len);
+  else sort_desc_regs<16>(a, c, len);
+}
+
 // The (|v| key << 32 | ~index) pairs of the entries whose bit is set in a
-// column's mask (words 32-bit words), the first `cap` of them in index order,
-// into out; returns how many bits are set.  Each thread owns a contiguous run
+// column's mask (words 32-bit words) in index order into out, when there are at
+// most `cap`; returns how many bits are set.  Each thread owns a contiguous run
 // of words, so an exclusive scan of their counts places the entries in order.
 // scratch: one word of shared memory per warp of the block.
 __device__ uint32_t pairs_from_mask(const uint32_t *__restrict__ mk, int words,
@@ -1266,6 +1334,7 @@ __device__ uint32_t pairs_from_mask(const uint32_t *__restrict__ mk, int words,
     if (i < w) off += scratch[i];
     total += scratch[i];
   }
+  if (total > cap) return total;  // not listed: nobody reads a part of the set
   for (int q = w0; q < w1; q++) {
     uint32_t bits = mk[q];
     while (bits) {
@@ -1285,10 +1354,14 @@ constexpr int HARD_THREADS = 256;
 constexpr int HARD_CAND = 2048;  // hinted (key, index) candidates resolved in shared memory
 
 // One streaming pass over a column in global memory (16-byte loads, four in
-// flight per thread): the entries with |v| key >= bound go to cand as
+// flight per thread): the entries with |v| key >= bound (>= 1) go to cand as
 // (key << 32 | ~index), the first `cap` of them in any order; returns how many
-// there are (it may exceed cap) and leaves in counter[1] the largest key below
-// the bound (0 if none).  Entries past n are not taken.
+// there are (it may exceed cap) and, BELOW, leaves in counter[1] the largest
+// key below the bound (0 if none).  Entries past n are not taken (the padding
+// read with the last 16 bytes is zero).  The bound leaves a few hundred entries
+// of a column, so a quad of them is tested by its largest key and the taken
+// ones placed by single shared-memory atomics.
+template <bool BELOW>
 __device__ uint32_t gather_pairs_above(const float *__restrict__ colg, int n, uint32_t bound,
                                        uint64_t *cand, uint32_t cap, uint32_t *counter) {
   if (threadIdx.x == 0) {
@@ -1297,54 +1370,95 @@ __device__ uint32_t gather_pairs_above(const float *__restrict__ colg, int n, ui
   }
   __syncthreads();
   uint32_t below = 0;
-  const int lane = threadIdx.x & 31;
   const int n4 = (n + 3) >> 2;
   const float4 *c4 = reinterpret_cast<const float4 *>(colg);
   constexpr int U = 4;
-  for (int base = (threadIdx.x & ~31); base < n4; base += U * blockDim.x) {
+  for (int base = threadIdx.x; base < n4; base += U * blockDim.x) {
     float4 v[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int i = base + u * blockDim.x + lane;
+      const int i = base + u * blockDim.x;
       v[u] = (i < n4) ? __ldg(c4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      const int e0 = 4 * (base + u * blockDim.x + lane);
-      const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
-      uint32_t take = 0;
+      const uint32_t k[4] = {abs_key(v[u].x), abs_key(v[u].y), abs_key(v[u].z), abs_key(v[u].w)};
+      if (BELOW) {
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t key = abs_key(x[q]);
-        const bool in = e0 + q < n;
-        take |= (uint32_t)(in && key >= bound) << q;
-        if (in && key < bound) below = max(below, key);
+        for (int q = 0; q < 4; q++) below = max(below, k[q] < bound ? k[q] : 0u);
       }
-      if (!__any_sync(FULL, take != 0)) continue;
-      const uint32_t mine = __popc(take);
-      uint32_t incl = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += t;
-      }
-      uint32_t wbase = 0;
-      if (lane == 31) wbase = atomicAdd(&counter[0], incl);
-      wbase = __shfl_sync(FULL, wbase, 31);
-      uint32_t pos = wbase + incl - mine;
+      if (max(max(k[0], k[1]), max(k[2], k[3])) < bound) continue;
+      const int e0 = 4 * (base + u * (int)blockDim.x);
 #pragma unroll
       for (int q = 0; q < 4; q++)
-        if (take & (1u << q)) {
-          if (pos < cap)
-            cand[pos] = ((uint64_t)abs_key(x[q]) << 32) | (uint32_t)~(uint32_t)(e0 + q);
-          pos++;
+        if (k[q] >= bound && e0 + q < n) {
+          const uint32_t pos = atomicAdd(&counter[0], 1u);
+          if (pos < cap) cand[pos] = ((uint64_t)k[q] << 32) | (uint32_t)~(uint32_t)(e0 + q);
         }
     }
   }
-  below = __reduce_max_sync(FULL, below);
-  if (lane == 0) atomicMax(&counter[1], below);
+  if (BELOW) {
+    below = __reduce_max_sync(FULL, below);
+    if ((threadIdx.x & 31) == 0) atomicMax(&counter[1], below);
+  }
   __syncthreads();
   return counter[0];
+}
+
+// A bound on |v| keys that about `target` to a few times as many of a column's
+// entries reach, from a sample of SAMPLE_KEYS evenly spaced ones (twice as
+// many from long columns; every entry of a short one): the sample's r-th
+// largest key to 8 significant bits, r the sample's share of `target` plus
+// 2.5 standard deviations of that count and 3, and at most 0.85 of its share of
+// `most` (0 when that is none).  For columns whose level has no usable
+// hint; reading 8 KB of a column in place of a histogram pass over all of it.
+// smp: room for 2 * SAMPLE_KEYS keys; cnt: 16 words.  The bound only decides how many
+// candidates are looked at, not the result.
+constexpr int SAMPLE_KEYS = 2048, SAMPLE_LONG = 65536;
+__device__ uint32_t sampled_bound(const float *__restrict__ colg, int n, uint32_t target,
+                                  uint32_t most, uint32_t *smp, uint32_t *cnt) {
+  const int n4 = n >> 2;  // whole quads
+  const int s4 = min(n4, (n > SAMPLE_LONG ? 2 : 1) * SAMPLE_KEYS / 4);
+  if (s4 == 0) return 1u;
+  const float f = (float)(4 * s4) / (float)n;
+  const float x = (float)target * f;
+  const float rf = fminf(s4 == n4 ? (float)target : x + 2.5f * sqrtf(x) + 3.f,
+                         fminf(0.85f * f * (float)most, (float)(4 * s4)));
+  const uint32_t r = (uint32_t)rf;
+  if (r == 0u) return 0u;
+  __syncthreads();  // smp and cnt may still be read by their previous users
+  if (threadIdx.x < 16) cnt[threadIdx.x] = 0u;
+  const float4 *c4 = reinterpret_cast<const float4 *>(colg);
+  for (int i = threadIdx.x; i < s4; i += blockDim.x) {
+    const float4 v = __ldg(c4 + (s4 == n4 ? i : (int)(((int64_t)i * n4) / s4)));
+    reinterpret_cast<uint4 *>(smp)[i] =
+        make_uint4(abs_key(v.x), abs_key(v.y), abs_key(v.z), abs_key(v.w));
+  }
+  __syncthreads();
+  uint32_t bound = 0u;
+  for (int bit = 30; bit >= 15; bit--) {
+    const uint32_t t = bound | (1u << bit);
+    uint32_t c = 0;
+    for (int i = threadIdx.x; i < s4; i += blockDim.x) {
+      const uint4 k = reinterpret_cast<const uint4 *>(smp)[i];
+      c += (k.x >= t) + (k.y >= t) + (k.z >= t) + (k.w >= t);
+    }
+    c = __reduce_add_sync(FULL, c);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&cnt[30 - bit], c);
+    __syncthreads();
+    if (cnt[30 - bit] >= r) bound = t;
+  }
+  __syncthreads();
+  return max(bound, 1u);
+}
+
+// The hint that makes the next step's candidate bound the key of rank `want`
+// of this step's sorted candidates (a little below the last of them when
+// there are fewer), and at most HINT_FRACTION of the level.
+__device__ __forceinline__ float next_hint(const uint64_t *sorted, uint32_t c, uint32_t want,
+                                           float level) {
+  const float b = __uint_as_float((uint32_t)(sorted[min(c - 1, want)] >> 32));
+  return fminf(level, (c <= want ? 0.85f * b : b) / HINT_FRACTION);
 }
 
 // One streaming pass over a column: every |v| with key >= bound goes to
@@ -1381,24 +1495,29 @@ __device__ uint32_t gather_keys_above(const float *__restrict__ colg, int n, uin
 // s-th largest |v| (with multiplicity, as the sorting variant :92-98 defines
 // it), keep |v| >= level, then x <- x / ||x|| (c++/src/gpower/gpower_commons.h:111).
 //
-// One block per column, reading it from global memory.  (a) With the previous
-// step's level as a hint, a streaming pass gathers the entries with
-// |v| >= HINT_FRACTION * hint together with their indices; if fewer than s,
-// a second pass gathers down to the largest key below that bound (exactly
-// the kept set when one entry was missing).  When that holds s to HARD_CAND
-// entries, sorting them gives the exact level, the norm and the kept entries,
-// and the column is written sparsely (its mask words cleared, then the kept
-// entries' bits and values set).  Otherwise (b) a histogram of the top 11 bits
-// of |v| finds the bin holding rank s, keys above it are kept for sure, keys
-// in it are gathered and sorted; a bin too full for shared memory falls back
-// to (c) the exact three-level radix select; the column is then written by a
-// full pass.
+// One block per column, reading it from global memory.  (a) The entries with
+// |v| at or above a bound, with their indices: the previous step's hint, whose
+// entries V = B^T Z's epilogue marked (or a streaming pass gathers), or, when
+// the hinted set is short of s or too large, or there is no hint, a bound from
+// a sample of the column.  When that gives s to HARD_CAND entries, sorting them
+// gives the exact level, the norm and the kept entries, and the column is
+// written sparsely (its mask words cleared, then the kept entries' bits and
+// values set).  Otherwise (b) a histogram of the top 11 bits of |v| finds the
+// bin holding rank s, keys above it are kept for sure, keys in it are gathered
+// and sorted; a bin too full for shared memory falls back to (c) the exact
+// three-level radix select; the column is then written by a full pass.
+// What bounds it: with a hint, the latency of the candidates' loads and sort;
+// without, one read of V (205 MB at 1024 columns of 50000, 31 us at the copy
+// rate).  Measured there: 84 us unhinted (704 with the histogram of every
+// column), 31 us hinted with a few columns falling back (265 when a hint that
+// came up short streamed the column twice).
 __device__ __forceinline__ void hard_select_body(
     const float *__restrict__ Vraw, int ldv, int n, unsigned s, float *__restrict__ Vx,
     uint32_t *__restrict__ nnz_out, int *status, uint32_t *__restrict__ vmask,
     float *__restrict__ hints, const uint32_t *stop, const uint32_t *__restrict__ cmask, int j) {
   if (*stop) return;
-  __shared__ uint64_t cand[HARD_CAND];  // also 2 * HARD_CAND keys for (b)
+  // also 2 * HARD_CAND keys for (b), and the sample, read 16 bytes at a time
+  __shared__ __align__(16) uint64_t cand[HARD_CAND];
   __shared__ uint32_t hist[2048];
   __shared__ uint32_t res[8];
   __shared__ double red[32];
@@ -1410,49 +1529,34 @@ __device__ __forceinline__ void hard_select_body(
   double ss = 0.0, cnt = 0.0;
   bool done = false;
   const float hint = hints[j];
-  uint32_t bound = hinted_bound(hint);
-  for (int attempt = 0; attempt < 2 && hint > 0.f && !done; attempt++) {
-    uint32_t c = 0, below = 0;
-    bool listed = false;
-    if (attempt == 0 && cmask) {
-      // V = B^T Z's epilogue marked the entries at or above the same bound
-      // (it keeps no largest key below the bound: with fewer than s entries the
-      // column is gathered here as before)
-      c = pairs_from_mask(cmask + (size_t)j * (ldv >> 5), ldv >> 5, colg, cand, HARD_CAND,
-                          &res[0]);
-      listed = c >= s;
-    }
-    if (!listed) {
-      c = gather_pairs_above(colg, n, bound, cand, HARD_CAND, &res[0]);
-      below = res[1];
-    }
-    if (c > (uint32_t)HARD_CAND) break;  // too many: the histogram path
-    if (c < s) {
-      // short by one: the s-th largest is the largest key below the bound, so
-      // gathering down to it takes exactly the kept entries; otherwise widen
-      bound = (s - c == 1) ? below : abs_key(HINT_FRACTION * __uint_as_float(below));
-      if (bound == 0) break;
-    } else {
-      int len = 1;
-      while (len < (int)c) len <<= 1;
-      for (int q = c + threadIdx.x; q < len; q += blockDim.x) cand[q] = 0ull;
-      __syncthreads();
-      bitonic_desc(cand, len);
-      thr = (uint32_t)(cand[s - 1] >> 32);
-      // kept: the sorted prefix with key >= thr (ties with the s-th included)
-      if (threadIdx.x == 0) res[1] = 0;
-      __syncthreads();
-      for (int q = threadIdx.x; q < (int)c; q += blockDim.x) {
-        const uint32_t key = (uint32_t)(cand[q] >> 32);
-        if (key >= thr && (q + 1 == (int)c || (uint32_t)(cand[q + 1] >> 32) < thr))
-          res[1] = q + 1;
-        if (key >= thr) {
-          const double v = (double)__uint_as_float(key);
-          ss += v * v;
-        }
+  float new_hint = 0.f;
+  // the bound that is wanted next time: about twice s entries reach it
+  const uint32_t want = s + min(s + 32u, 192u);
+  uint32_t c = 0;
+  if (hint > 0.f)
+    c = cmask ? pairs_from_mask(cmask + (size_t)j * (ldv >> 5), ldv >> 5, colg, cand, HARD_CAND,
+                                &res[0])
+              : gather_pairs_above<false>(colg, n, hinted_bound(hint), cand, HARD_CAND, &res[0]);
+  if ((c < s || c > (uint32_t)HARD_CAND) && s <= (uint32_t)HARD_CAND) {
+    const uint32_t bound = sampled_bound(colg, n, want, HARD_CAND, cand32, hist);
+    c = bound ? gather_pairs_above<false>(colg, n, bound, cand, HARD_CAND, &res[0]) : 0u;
+  }
+  if (c >= s && c <= (uint32_t)HARD_CAND) {
+    __syncthreads();
+    sort_pairs_desc(cand, (int)c, HARD_CAND);
+    thr = (uint32_t)(cand[s - 1] >> 32);
+    // kept: the sorted prefix with key >= thr (ties with the s-th included)
+    for (int q = threadIdx.x; q < (int)c; q += blockDim.x) {
+      const uint32_t key = (uint32_t)(cand[q] >> 32);
+      if (key >= thr && (q + 1 == (int)c || (uint32_t)(cand[q + 1] >> 32) < thr))
+        res[1] = q + 1;
+      if (key >= thr) {
+        const double v = (double)__uint_as_float(key);
+        ss += v * v;
       }
-      done = true;
     }
+    new_hint = next_hint(cand, c, want, __uint_as_float(thr));
+    done = true;
     __syncthreads();
   }
   if (done) {
@@ -1463,8 +1567,11 @@ __device__ __forceinline__ void hard_select_body(
     __syncthreads();
     for (int q = threadIdx.x; q < (int)kept; q += blockDim.x) {
       const uint32_t i = ~(uint32_t)cand[q];
-      vx[i] = __ldg(colg + i) * inv;
-      atomicOr(&mk[i >> 5], 1u << (i & 31));
+      const float x = __ldg(colg + i) * inv;
+      if (x != 0.f) {
+        vx[i] = x;
+        atomicOr(&mk[i >> 5], 1u << (i & 31));
+      }
     }
     cnt = (double)kept;
   } else {
@@ -1519,7 +1626,7 @@ __device__ __forceinline__ void hard_select_body(
                         [=](float v) { return (abs_key(v) >= thr) ? v * inv : 0.f; });
   }
   if (threadIdx.x == 0) {
-    hints[j] = __uint_as_float(thr);
+    hints[j] = done ? new_hint : __uint_as_float(thr);
     nnz_out[j] = (uint32_t)cnt;
   }
 }
@@ -1631,6 +1738,22 @@ __device__ void eval_chunk(const float *cand, const double *p1, const double *p2
     const double hi = (double)cand[q];
     const double lov = (q + 1 < total) ? (double)cand[q + 1] : lo_after;
     const double S1i = p1[q], S2i = p2[q];
+    // Ranks that cannot stop are passed over without the predicates' roots and
+    // quotients.  With R(l) = num / sqrt(den) at the segment's lower end below
+    // sqrt(s) by 5e-6 relative, the segment lies strictly between the roots of
+    // the stopping quadratic (or, t < s, its discriminant -4 (s - t) s D is
+    // negative), at a distance of 5e-6 of their spacing or more; den and D, the
+    // spreads that rounding is measured against, are large enough here that the
+    // predicates' own rounding moves a root by less than a tenth of that.  Equal
+    // or nearly equal leading values (den, D near 0), where the last bit
+    // decides, and NaN all fail these tests and are evaluated.
+    {
+      const double num = S1i - t * lov, den = S2i - 2.0 * lov * S1i + t * lov * lov;
+      const double lead = S2i - 2.0 * hi * S1i + t * hi * hi;  // sum (v_i - v_t)^2
+      if (num >= 0.0 && num * num < 0.99999 * sq2 * den && lead > 1e-6 * S2i && g + 1 != n &&
+          (EXACT || sq2 * (t * S2i - S1i * S1i) > 1e-8 * S1i * S1i * fmax(t, sq2)))
+        continue;
+    }
     if (!EXACT) {
       // Same operations, order and (unfused) rounding as the reference's
       // expressions at thresh_functions.h:193-213; several of its stops are
@@ -1838,27 +1961,43 @@ __device__ __forceinline__ void soft_select_body(
   bool sparse = false;     // ... and the gathered pairs hold every kept entry
   uint32_t c_pairs = 0;
   double ss = 0.0, cnt = 0.0;
-  // ---- hinted path: gather (key, index) with |v| >= HINT_FRACTION * (previous level)
+  float new_hint = 0.f;
+  // ---- candidate sets (1024 columns of 50000, s = 128: 186 us on the first
+  // step where the histogram and the chunked walk took 780; 90 to 190 later,
+  // where columns that outran the hint took 690): the (key, index) pairs with
+  // |v| at or above a bound,
+  // sorted and scanned a chunk of SOFT_C ranks at a time.  Attempt 0 takes the
+  // hinted set; when that is empty, too large or ends before the stop, attempts
+  // 1 and 2 take bounds from a sample of the column (4 s + 64 entries or twice
+  // the set that was too small; then as many as fit)
   const float hint = hints[j];
   uint32_t c_hint = 0;  // entries at or above the hinted bound
-  if (hint > 0.f) {
-    uint32_t c, below_key = 0;
-    const bool listed = cmask != nullptr;
+  constexpr uint32_t MOST = SOFT_HINT_CAP;
+  uint32_t want = s < MOST / 4u ? 4u * s + 64u : MOST;
+  for (int attempt = hint > 0.f ? 0 : 1; attempt < 3 && brk == NONE; attempt++) {
+    uint32_t c = 0, below_key = 0;
+    const bool listed = attempt == 0 && cmask != nullptr;
     if (listed) {  // marked by V = B^T Z's epilogue, with the same bound
       c = pairs_from_mask(cmask + (size_t)j * (ldv >> 5), ldv >> 5, colg, pairs, SOFT_HINT_CAP,
                           res);
     } else {
-      c = gather_pairs_above(colg, n, hinted_bound(hint), pairs, SOFT_HINT_CAP, res);
-      below_key = res[1];
+      uint32_t bound = 0;
+      if (attempt == 0) {
+        bound = hinted_bound(hint);
+      } else if (attempt == 2 || want < MOST / 2u) {
+        if (attempt == 2) want = MOST;
+        bound = sampled_bound(colg, n, want, SOFT_HINT_CAP, reinterpret_cast<uint32_t *>(pairs),
+                              res);
+      }
+      if (bound) {
+        c = gather_pairs_above<true>(colg, n, bound, pairs, SOFT_HINT_CAP, res);
+        below_key = res[1];
+      }
     }
-    c_hint = c;
+    if (attempt == 0) c_hint = c;
     __syncthreads();
     if (c > 0 && c <= (uint32_t)SOFT_HINT_CAP) {
-      int len = 1;
-      while (len < (int)c) len <<= 1;
-      for (int q = c + threadIdx.x; q < len; q += blockDim.x) pairs[q] = 0ull;
-      __syncthreads();
-      bitonic_desc(pairs, len);
+      sort_pairs_desc(pairs, (int)c, SOFT_HINT_CAP);
       // the sorted set, a chunk of SOFT_C ranks at a time; every position sees
       // its next value in the set, except the set's last: for a listed set
       // (no largest value below it) that one is left to the paths below
@@ -1911,6 +2050,9 @@ __device__ __forceinline__ void soft_select_body(
         have_norm = true;
         sparse = true;
         c_pairs = c;
+        new_hint = next_hint(pairs, c, brk + brk / 2u + 32u, (float)w);
+      } else {
+        want = max(want, 2u * c);
       }
     }
     __syncthreads();
@@ -2010,7 +2152,7 @@ __device__ __forceinline__ void soft_select_body(
     brk = exact_walk<EXACT>(ColumnSrc{colg}, (uint32_t)n, (uint32_t)n, 0.0, cand, p1, p2, hist,
                             res, red, misc, w_sh, sq, sq2, &w);
 
-  if (threadIdx.x == 0) hints[j] = (float)w;
+  if (threadIdx.x == 0) hints[j] = sparse ? new_hint : (float)w;
   // x = sgn(v)(|v| - w)_+ with w kept in double: a level that lands within
   // rounding of the largest |v| still leaves that entry non-zero, as in the
   // reference's double arithmetic.

@@ -332,6 +332,7 @@ struct SparseBatchDev {
   uint32_t *vmask = nullptr; // k x ldn / 32
   float *Vraw = nullptr;     // k x ldn raw V = B^T Z (and the staging of loads)
   float *Vt = nullptr;       // n x kp
+  uint32_t *xmask = nullptr; // per tile of starts, a bit per row of Vt: not zero in the tile
   float *Zs = nullptr;       // k x ldm
   float *Zt = nullptr;       // m x kp
   float *fz = nullptr, *val = nullptr, *err = nullptr, *max_err = nullptr;

@@ -3065,21 +3065,26 @@ cudaError_t launch_grouped_condition(const GroupDev &g, unsigned long long handl
 
 namespace {
 // One product on the compressed arrays: the tile kernel for the outer entries
-// of at most SP_LONG entries, the segment and combine kernels for the others.
+// and the segments of the long ones, the combine kernel for the long ones' sums.
 // gate (may be null): the launches do their work only when *gate >= gate_min.
+// xmask (may be null): the rows of X that are not zero, per tile of starts.
+template <bool SKIP>
 void sparse_product(const int32_t *ptr, const int32_t *idx, const float *val, int ncols,
                     const SparseLong &L, const float *X, float *part, const SparseBatchDev &b,
                     float *out, int ld_out, const float *cvec, const double *a, const double *bv,
-                    const uint32_t *gate, uint32_t gate_min, cudaStream_t st) {
-  sp_spmm_kernel<<<dim3((ncols + SP_TILE - 1) / SP_TILE, b.kp / SP_TILE), SP_THREADS, 0, st>>>(
-      ptr, idx, val, ncols, X, b.kp, b.k, out, ld_out, cvec, a, bv, b.ctl, gate, gate_min);
+                    const uint32_t *gate, uint32_t gate_min, const uint32_t *xmask,
+                    cudaStream_t st) {
+  const int tiles = (b.kp + SP_WIDE - 1) / SP_WIDE;
+  const int seg_blocks = L.count ? (L.segs + SP_OUTER - 1) / SP_OUTER : 0;
+  sp_spmm_kernel<SKIP>
+      <<<dim3(seg_blocks + (ncols + SP_OUTER - 1) / SP_OUTER, tiles), SP_THREADS, 0, st>>>(
+          ptr, idx, val, ncols, X, b.kp, b.k, out, ld_out, cvec, a, bv, b.ctl, gate, gate_min,
+          xmask, b.ldn / 32, L.seg_e0, L.seg_e1, L.segs, seg_blocks, part);
   if (L.count == 0) return;
-  constexpr int WARPS = SP_THREADS / 32;
-  sp_spmm_seg_kernel<<<dim3((L.segs + WARPS - 1) / WARPS, b.kp / SP_TILE), SP_THREADS, 0, st>>>(
-      L.seg_e0, L.seg_e1, L.segs, idx, val, X, b.kp, part, b.ctl, gate, gate_min);
   sp_spmm_long_kernel<<<dim3(L.count, b.kp / SP_TILE), SP_TILE, 0, st>>>(
       L.outer, L.seg_first, part, b.kp, b.k, out, ld_out, cvec, a, bv, b.ctl, gate, gate_min);
 }
+
 }  // namespace
 
 cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, const StepParams &p,
@@ -3106,12 +3111,13 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
       b.max_nnz, (uint32_t)SP_SCATTER_CAP, b.work,
       S.comps > 0 ? -1.0 : SP_SCATTER_PER_STEP * (double)S.nnz * (double)(b.kp / 32), b.zgate,
       b.ctl);
-  sp_transpose_v_kernel<<<dim3((S.n + SP_TILE - 1) / SP_TILE, b.kp / SP_TILE), SP_THREADS, 0,
-                          st>>>(b.Vx, b.vmask, b.ldn, S.n, b.k, b.Vt, b.kp, b.ctl, b.zgate, 1u,
-                                S.defl, S.comps, b.defl_a);
-  sparse_product(S.row_ptr, S.col_ind, S.rvals, S.m, S.long_rows, b.Vt, b.part_rows, b, b.Zs,
-                 b.ldm, S.row_means, S.row_means ? b.sum_v : nullptr,
-                 S.means ? b.dot_mu : nullptr, b.zgate, 1u, st);
+  sp_transpose_v_kernel<<<dim3((S.n + SP_TILE - 1) / SP_TILE, (b.kp + SP_WIDE - 1) / SP_WIDE),
+                          SP_THREADS, 0, st>>>(b.Vx, b.vmask, b.ldn, S.n, b.k, b.Vt, b.kp,
+                                               b.xmask, b.ctl, b.zgate, 1u, S.defl, S.comps,
+                                               b.defl_a);
+  sparse_product<true>(S.row_ptr, S.col_ind, S.rvals, S.m, S.long_rows, b.Vt, b.part_rows, b,
+                       b.Zs, b.ldm, S.row_means, S.row_means ? b.sum_v : nullptr,
+                       S.means ? b.dot_mu : nullptr, b.zgate, 1u, b.xmask, st);
   sp_scatter_z_kernel<<<b.k, SP_THREADS, 0, st>>>(
       S.col_ptr, S.row_ind, S.cvals, b.Vx, b.vmask, b.ldn, b.Zs, b.ldm, S.m, S.row_means,
       S.row_means ? b.sum_v : nullptr, S.means ? b.dot_mu : nullptr, b.zgate, 0u, b.ctl);
@@ -3121,9 +3127,9 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
   sp_transpose_z_kernel<<<dim3((S.m + SP_TILE - 1) / SP_TILE, b.kp / SP_TILE), SP_THREADS, 0,
                           st>>>(b.Zs, b.ldm, S.m, b.k, b.Zt, b.kp, b.ctl);
   // 3. V = (B - 1 mu^T - r 1^T)^T Z: CSC columns against Z transposed
-  sparse_product(S.col_ptr, S.row_ind, S.cvals, S.n, S.long_cols, b.Zt, b.part_cols, b, b.Vraw,
-                 b.ldn, S.means, S.means ? b.zsum : nullptr, S.row_means ? b.zdot : nullptr,
-                 nullptr, 0, st);
+  sparse_product<false>(S.col_ptr, S.row_ind, S.cvals, S.n, S.long_cols, b.Zt, b.part_cols, b,
+                        b.Vraw, b.ldn, S.means, S.means ? b.zsum : nullptr,
+                        S.row_means ? b.zdot : nullptr, nullptr, 0, nullptr, st);
   if (S.comps > 0)
     sp_defl_vraw_kernel<<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, S.defl, S.comps, S.gram,
                                                     b.ctl);

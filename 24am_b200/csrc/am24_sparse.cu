@@ -274,6 +274,7 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   AM24_TRY(A.get(&b.vmask, (size_t)k * (b.ldn / 32)));
   AM24_TRY(A.get(&b.Vraw, (size_t)k * b.ldn));
   AM24_TRY(A.get(&b.Vt, (size_t)n * b.kp));
+  AM24_TRY(A.get(&b.xmask, (size_t)(b.kp / 32) * (b.ldn / 32)));
   AM24_TRY(A.get(&b.Zs, (size_t)k * b.ldm));
   AM24_TRY(A.get(&b.Zt, (size_t)S.m * b.kp));
   AM24_TRY(A.get(&b.fz, k));

@@ -14,35 +14,94 @@
 // The per-column passes around them (selects, finalize) are the dense path's.
 
 constexpr int SP_TILE = 32;        // outer entries x starts per tile
-constexpr int SP_THREADS = 256;    // 8 warps, 4 outer entries each
+constexpr int SP_THREADS = 256;
+// outer entries per block of the products, one per warp: lengths vary with the
+// terms' popularity, and a warp that takes several long ones in turn holds the
+// launch (B^T Z of 6 M entries, 512 starts: 1.58 ms with four per warp, 0.48 with
+// one, the segments of the longest aside)
+constexpr int SP_OUTER = SP_THREADS / 32;
+// starts per lane of the products, and per tile.  Four also for batches that
+// leave lanes idle: a step's time at 32 starts 0.46 ms, against 0.48 with one
+// start per lane, and 1.6 against 3.1 at 512
+constexpr int SP_VEC = 4, SP_WIDE = 32 * SP_VEC;
 
-// sum over entries e in [e0, e1) of val[e] * X[idx[e] * kp + j], in entry
-// order with FP32 FMAs, for the lane's start j.  The warp loads 32 (index,
-// value) pairs at once, one per lane, and broadcasts them, so the X loads of
-// consecutive entries do not wait on one another.
-__device__ __forceinline__ float sp_dot(const int32_t *__restrict__ idx,
-                                        const float *__restrict__ val,
-                                        const float *__restrict__ X, int kp, int j, int e0,
-                                        int e1) {
+// acc = sum over entries e in [e0, e1) of val[e] * X[idx[e] * kp + j ...], in
+// entry order with FP32 FMAs, for the lane's SP_VEC starts from j.  The warp loads
+// 32 (index, value) pairs at once, one per lane, so the X loads of consecutive
+// entries do not wait on one another.  SKIP: xmask has a bit per row of X, clear
+// where the row is zero in all of the warp's starts; entries that meet such a
+// row (and whose own value is finite) add nothing and are left out: the others
+// are queued in order in the warp's part of shared memory (64 pairs) and taken
+// 32 at a time.
+template <bool SKIP>
+__device__ __forceinline__ void sp_dot(const int32_t *__restrict__ idx,
+                                       const float *__restrict__ val,
+                                       const float *__restrict__ X, int kp, int j, int e0, int e1,
+                                       const uint32_t *__restrict__ xmask, int2 *queue,
+                                       float4 &acc) {
   const int lane = threadIdx.x & 31;
-  float acc = 0.f;
+  acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float *Xj = X + j;
+  auto add = [&](int i, float v) {
+    const float4 x = *reinterpret_cast<const float4 *>(Xj + (size_t)i * kp);
+    acc.x = fmaf(v, x.x, acc.x);
+    acc.y = fmaf(v, x.y, acc.y);
+    acc.z = fmaf(v, x.z, acc.z);
+    acc.w = fmaf(v, x.w, acc.w);
+  };
+  if (!SKIP) {
+    for (int base = e0; base < e1; base += 32) {
+      const int e = base + lane;
+      int ii = 0;
+      float vv = 0.f;
+      if (e < e1) {
+        ii = idx[e];
+        vv = val[e];
+      }
+      const int cnt = min(32, e1 - base);
+#pragma unroll 8
+      for (int t = 0; t < cnt; t++) {
+        const int i = __shfl_sync(0xFFFFFFFFu, ii, t);
+        const float v = __shfl_sync(0xFFFFFFFFu, vv, t);
+        add(i, v);
+      }
+    }
+    return;
+  }
+  int have = 0;  // queued pairs (uniform over the warp)
+  auto take = [&](int first, int cnt) {
+#pragma unroll 8
+    for (int t = 0; t < cnt; t++) {
+      const int2 p = queue[first + t];
+      add(p.x, __int_as_float(p.y));
+    }
+  };
   for (int base = e0; base < e1; base += 32) {
     const int e = base + lane;
+    bool use = false;
     int ii = 0;
     float vv = 0.f;
     if (e < e1) {
       ii = idx[e];
       vv = val[e];
+      use = ((xmask[ii >> 5] >> (ii & 31)) & 1u) || !isfinite(vv);
     }
-    const int cnt = min(32, e1 - base);
-#pragma unroll 8
-    for (int t = 0; t < cnt; t++) {
-      const int i = __shfl_sync(0xFFFFFFFFu, ii, t);
-      const float v = __shfl_sync(0xFFFFFFFFu, vv, t);
-      acc = fmaf(v, X[(size_t)i * kp + j], acc);
+    const uint32_t bits = __ballot_sync(0xFFFFFFFFu, use);
+    if (use)
+      queue[have + __popc(bits & ((1u << lane) - 1u))] = make_int2(ii, __float_as_int(vv));
+    have += __popc(bits);
+    __syncwarp();
+    if (have >= 32) {
+      take(0, 32);
+      const int2 rest = queue[32 + lane];
+      __syncwarp();
+      have -= 32;
+      if (lane < have) queue[lane] = rest;
+      __syncwarp();
     }
   }
-  return acc;
+  take(0, have);
+  __syncwarp();  // the queue is refilled by the warp's next outer entry
 }
 
 // The rank-one centring of one output: acc - (cvec ? cvec[c] a[j] : 0) - (b ? b[j] : 0) in FP64.
@@ -57,43 +116,63 @@ __device__ __forceinline__ float sp_correct(float acc, int c, int j, const float
 
 // out[j][c] (j < k, c < ncols) = sum_e val[e] X[idx[e] * kp + j]
 //                                - (cvec ? cvec[c] * a[j] : 0) - (b ? b[j] : 0)
-// One warp per outer entry, a lane per start: every entry reads one 128-byte
-// row segment of X.  Each sum runs over the outer entry's entries in storage
-// order with FP32 FMAs (deterministic); the correction is applied in FP64.
-// Outer entries longer than SP_LONG are left to sp_spmm_seg_kernel and
-// sp_spmm_long_kernel.
+// One warp per outer entry, SP_VEC starts per lane: every entry reads one row
+// segment of X, 512 bytes.  Each sum runs over the outer entry's entries in
+// storage order with FP32 FMAs (deterministic); the correction is applied in
+// FP64.  Outer entries longer than SP_LONG are summed in segments: the launch's
+// first `seg_blocks` blocks take one segment per warp (the longest work goes
+// first) and write its sum to part[s][j], and sp_spmm_long_kernel adds them up.
+// What bounds it: the L2 reads of X's segments
+// (17.6 TB/s for B^T Z of 6 M entries, 512 starts: 0.69 ms; with one start per
+// lane the instructions did: 2.8 ms), and where rows are left out the scan of the
+// entries (0.34 ms once supports are sparse; 2.0 ms when every row was read).
+template <bool SKIP>
 __global__ void __launch_bounds__(SP_THREADS) sp_spmm_kernel(
     const int32_t *__restrict__ ptr, const int32_t *__restrict__ idx,
     const float *__restrict__ val, int ncols, const float *__restrict__ X, int kp, int k,
     float *__restrict__ out, int ld_out, const float *__restrict__ cvec,
     const double *__restrict__ a, const double *__restrict__ b, const uint32_t *stop,
-    const uint32_t *gate, uint32_t gate_min) {
+    const uint32_t *gate, uint32_t gate_min, const uint32_t *__restrict__ xmask, int xwords,
+    const int32_t *__restrict__ seg_e0, const int32_t *__restrict__ seg_e1, int segs,
+    int seg_blocks, float *__restrict__ part) {
   if (*stop || (gate && *gate < gate_min)) return;
-  __shared__ float tile[SP_TILE][SP_TILE + 1];
-  __shared__ int skip[SP_TILE];
+  __shared__ float tile[SP_WIDE][SP_OUTER + 1];
+  __shared__ int skip[SP_OUTER];
+  __shared__ int2 queues[SKIP ? SP_OUTER : 1][64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int c0 = blockIdx.x * SP_TILE, j0 = blockIdx.y * SP_TILE;
-  const int j = j0 + lane;  // < kp always (kp is a multiple of 32)
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int c = c0 + r;
-    float acc = 0.f;
-    bool own = false;
-    if (c < ncols) {
-      const int e0 = ptr[c], e1 = ptr[c + 1];
-      own = e1 - e0 <= SP_LONG;
-      if (own) {
-        acc = sp_dot(idx, val, X, kp, j, e0, e1);
-        if (j < k) acc = sp_correct(acc, c, j, cvec, a, b);
-      }
+  const int j0 = blockIdx.y * SP_WIDE, j = j0 + SP_VEC * lane;
+  const int jl = j < kp ? j : j0;  // lanes past the last start repeat the tile's first
+  const uint32_t *xm = SKIP ? xmask + (size_t)blockIdx.y * xwords : nullptr;
+  int2 *queue = queues[SKIP ? warp : 0];
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if ((int)blockIdx.x < seg_blocks) {
+    const int s = blockIdx.x * SP_OUTER + warp;
+    if (s >= segs) return;  // whole warps leave together
+    sp_dot<SKIP>(idx, val, X, kp, jl, seg_e0[s], seg_e1[s], xm, queue, acc);
+    if (j < kp) *reinterpret_cast<float4 *>(part + (size_t)s * kp + j) = acc;
+    return;
+  }
+  const int c0 = ((int)blockIdx.x - seg_blocks) * SP_OUTER;
+  const int c = c0 + warp;
+  bool own = false;
+  if (c < ncols) {
+    const int e0 = ptr[c], e1 = ptr[c + 1];
+    own = e1 - e0 <= SP_LONG;
+    if (own) {
+      sp_dot<SKIP>(idx, val, X, kp, jl, e0, e1, xm, queue, acc);
     }
-    tile[lane][r] = acc;
-    if (lane == 0) skip[r] = !own;
   }
+  const float y[SP_VEC] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+  for (int i = 0; i < SP_VEC; i++)
+    tile[SP_VEC * lane + i][warp] =
+        own && j + i < k ? sp_correct(y[i], c, j + i, cvec, a, b) : 0.f;
+  if (lane == 0) skip[warp] = !own;
   __syncthreads();
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int jj = j0 + r, c = c0 + lane;
-    if (jj < k && c < ncols && !skip[lane]) out[(size_t)jj * ld_out + c] = tile[r][lane];
-  }
+  const int cw = threadIdx.x % SP_OUTER;  // a start's row of the tile: one 32-byte sector
+  if (c0 + cw >= ncols || skip[cw]) return;
+  for (int r = threadIdx.x / SP_OUTER; r < SP_WIDE; r += SP_THREADS / SP_OUTER)
+    if (j0 + r < k) out[(size_t)(j0 + r) * ld_out + c0 + cw] = tile[r][cw];
 }
 
 // Z = (B - centring) V once V is sparse (when sp_zgate_kernel chose this path:
@@ -171,22 +250,7 @@ __global__ void __launch_bounds__(SP_THREADS) sp_scatter_z_kernel(
   }
 }
 
-// Long outer entries, step 1: one warp per (segment, 32 starts), the
-// segment's sum into part[s][j].
-__global__ void __launch_bounds__(SP_THREADS) sp_spmm_seg_kernel(
-    const int32_t *__restrict__ seg_e0, const int32_t *__restrict__ seg_e1, int segs,
-    const int32_t *__restrict__ idx, const float *__restrict__ val,
-    const float *__restrict__ X, int kp, float *__restrict__ part, const uint32_t *stop,
-    const uint32_t *gate, uint32_t gate_min) {
-  if (*stop || (gate && *gate < gate_min)) return;
-  const int s = blockIdx.x * (SP_THREADS / 32) + (threadIdx.x >> 5);
-  const int j = blockIdx.y * SP_TILE + (threadIdx.x & 31);
-  if (s >= segs) return;  // whole warps leave together
-  part[(size_t)s * kp + j] = sp_dot(idx, val, X, kp, j, seg_e0[s], seg_e1[s]);
-}
-
-// Long outer entries, step 2: per (entry, start) the segments' sums in
-// segment order, then the centring, into out[j][c].
+// Long outer entries: per (entry, start) the segments' sums in segment order, then the centring, into out[j][c].
 __global__ void __launch_bounds__(SP_TILE) sp_spmm_long_kernel(
     const int32_t *__restrict__ outer, const int32_t *__restrict__ seg_first,
     const float *__restrict__ part, int kp, int k, float *__restrict__ out, int ld_out,
@@ -204,39 +268,52 @@ __global__ void __launch_bounds__(SP_TILE) sp_spmm_long_kernel(
 
 // Vt[q][j] = V's column j at row q (zero where its mask bit is clear), for
 // q < n, j < kp (columns k..kp-1 zero): the row-major X of Z = B V (dense
-// steps only: *gate >= gate_min).
+// steps only: *gate >= gate_min).  A block takes 32 rows and the SP_WIDE starts
+// of one tile of the product and writes xmask[tile][q / 32]: the rows in which
+// any of the tile's starts has a loading.
 // With deflations (comps > 0) the column is the projected one,
-// v - sum_c a[j][c] x_c (sp_defl_coef_kernel's coefficients).
+// v - sum_c a[j][c] x_c (sp_defl_coef_kernel's coefficients), and every row counts.
 __global__ void __launch_bounds__(SP_THREADS) sp_transpose_v_kernel(
     const float *__restrict__ Vx, const uint32_t *__restrict__ mask, int ldn, int n, int k,
-    float *__restrict__ Vt, int kp, const uint32_t *stop, const uint32_t *gate,
-    uint32_t gate_min, const float *__restrict__ defl, int comps,
-    const double *__restrict__ defl_a) {
+    float *__restrict__ Vt, int kp, uint32_t *__restrict__ xmask,
+    const uint32_t *stop, const uint32_t *gate, uint32_t gate_min,
+    const float *__restrict__ defl, int comps, const double *__restrict__ defl_a) {
   if (*stop || *gate < gate_min) return;
   __shared__ float tile[SP_TILE][SP_TILE + 1];
+  __shared__ uint32_t any;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int q0 = blockIdx.x * SP_TILE, j0 = blockIdx.y * SP_TILE;
+  const int q0 = blockIdx.x * SP_TILE;
   const int words = ldn >> 5;
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int j = j0 + r, q = q0 + lane;
-    float v = 0.f;
-    if (j < k && q < n) {
-      const uint32_t w = mask[(size_t)j * words + (q >> 5)];
-      if ((w >> (q & 31)) & 1u) v = Vx[(size_t)j * ldn + q];
-      if (comps > 0) {
-        double d = (double)v;
-        for (int c = 0; c < comps; c++)
-          d -= defl_a[(size_t)j * SP_DEFL_MAX + c] * (double)defl[(size_t)c * n + q];
-        v = (float)d;
+  if (threadIdx.x == 0) any = comps > 0 ? 0xFFFFFFFFu : 0u;
+  uint32_t mine = 0u;
+  const int j1 = min(kp, (int)(blockIdx.y + 1) * SP_WIDE);
+  for (int j0 = blockIdx.y * SP_WIDE; j0 < j1; j0 += SP_TILE) {
+    __syncthreads();  // `any` set, or the previous tile stored
+    for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
+      const int j = j0 + r, q = q0 + lane;
+      float v = 0.f;
+      if (j < k && q < n) {
+        const uint32_t w = mask[(size_t)j * words + (q >> 5)];
+        mine |= w;
+        if ((w >> (q & 31)) & 1u) v = Vx[(size_t)j * ldn + q];
+        if (comps > 0) {
+          double d = (double)v;
+          for (int c = 0; c < comps; c++)
+            d -= defl_a[(size_t)j * SP_DEFL_MAX + c] * (double)defl[(size_t)c * n + q];
+          v = (float)d;
+        }
       }
+      tile[r][lane] = v;
     }
-    tile[r][lane] = v;
+    __syncthreads();
+    for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
+      const int q = q0 + r;
+      if (q < n) Vt[(size_t)q * kp + j0 + lane] = tile[lane][r];
+    }
   }
+  if (lane == 0 && mine) atomicOr(&any, mine);
   __syncthreads();
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int q = q0 + r;
-    if (q < n) Vt[(size_t)q * kp + j0 + lane] = tile[lane][r];
-  }
+  if (threadIdx.x == 0) xmask[(size_t)blockIdx.y * words + blockIdx.x] = any;
 }
 
 // Zt[i][j] = Zs[j][i] for i < m, j < kp (columns k..kp-1 zero): the row-major
@@ -313,13 +390,14 @@ __global__ void __launch_bounds__(SP_THREADS) sp_vstats_kernel(
 // within its list (the previous step's largest count, *max_nnz, at most cap)
 // and must touch fewer matrix entries (*work over all starts) than csr_steps:
 // SP_SCATTER_PER_STEP times the steps of the CSR product's warps (nnz x k / 32,
-// one 32-start row segment per entry and chunk of starts).  A scattered entry
-// (a coalesced read of its row and value, one update of a z row that stays in
-// cache) costs about a quarter of such a warp step: measured on B200 with
-// 1024 starts, a support work of 1.4x the warp steps ran faster scattered
-// (6.5 against 9.3 ms per step), while a corpus whose supports hold its most
-// common terms (an estimated 5x) ran slower (26.9 against 24.0).
-constexpr double SP_SCATTER_PER_STEP = 4.0;
+// one entry for 32 starts).  Below that a support's columns hold under 1/128 of
+// the matrix's entries.  Measured on B200, time per step scattered against the
+// CSR product, by the support work per warp step: 0.02 (20000 x 50000, 1 %,
+// 1024 starts, s = 32) 2.57 against 3.03 ms, 0.01 (150000 x 60000, 5 entries a
+// column) 0.88 against 0.97; 1.6 (a corpus whose supports hold its most common
+// terms, 64 starts, s = 4) 0.74 against 0.36, 7 (the same, 512 starts, s = 32)
+// 4.9 against 1.4.
+constexpr double SP_SCATTER_PER_STEP = 0.25;
 __global__ void sp_zgate_kernel(const uint32_t *max_nnz, uint32_t cap,
                                 const unsigned long long *work, double csr_steps,
                                 uint32_t *zgate, const uint32_t *stop) {

@@ -19,15 +19,13 @@ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; 
 // by the host-side capacity checks through the same rules.
 __device__ int plan_items(const GProblem &P, int l, uint32_t gate, uint32_t scheme) {
   const bool dense = gate > P.sparse_cap;
-  const bool grouped = !dense && gate <= min(P.sparse_cap, GATHER_GROUP_MAX_NNZ);
+  const bool wide = P.m > GATHER_NARROW;
   const int pairs1 = (P.m_tiles1 + 1) >> 1, pairs2 = (P.m_tiles2 + 1) >> 1;
   switch (l) {
-    case GL_GG0: case GL_GG1: case GL_GG2:
-      return (P.mode == l - GL_GG0 && grouped) ? ceil_div(P.k, GATHER_GROUP) : 0;
-    case GL_GA0: case GL_GA1: case GL_GA2:
-      return (P.mode == l - GL_GA0 && !dense && !grouped) ? P.k : 0;
-    case GL_DN0: case GL_DN1: case GL_DN2:
-      return (P.mode == l - GL_DN0 && dense) ? P.k : 0;
+    case GL_GATHER: return !dense && !wide ? P.k : 0;
+    case GL_LIST: case GL_FINISH: return !dense && wide ? P.k : 0;
+    case GL_TILE: return !dense && wide ? gather_tiles(P.ldm) * gather_groups(P.k) : 0;
+    case GL_DENSE: return dense ? P.k : 0;
     case GL_SEL_HARD: return P.formulation <= 1 ? P.k : 0;
     case GL_SEL_SCAN: return (P.formulation == 2 || P.formulation == 3) && !P.l1_exact ? P.k : 0;
     case GL_SEL_EXACT: return (P.formulation == 2 || P.formulation == 3) && P.l1_exact ? P.k : 0;
@@ -126,7 +124,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) group_plan_kernel(GroupDev g) {
       __syncthreads();
     }
   }
-  if (tid < GL_COUNT + 3) g.plan->next[tid] = 0;
+  if (tid < GL_COUNT + 1) g.plan->next[tid] = 0;
   if (tid < GL_COUNT) {
     g.plan->n[tid] = carry_n[tid];
     g.plan->total[tid] = carry_t[tid];
@@ -169,41 +167,45 @@ __device__ __forceinline__ void for_items(const GroupDev &g, int l, Fn fn, int c
   }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(GATHER_THREADS) g_gather_group_kernel(GroupDev g) {
-  for_items(g, GL_GG0 + MODE, [](const GProblem &P, int item) {
-    gather_bv_group_body<MODE>(P.Bc, P.ldm, P.m, P.ldn, P.k, P.Vx, P.vmask, P.Z_hi, P.Z_lo, P.fz,
-                               P.ctl + GCTL_GATE, P.sparse_cap, P.Z_b, P.Z_h, P.zplane,
-                               P.z_scale, P.ctl + CTL_STOP, item);
+__device__ __forceinline__ ZOut z_out(const GProblem &P, int j) {
+  return z_out(j, P.ldm, P.Z_hi, P.Z_lo, P.Z_b, P.Z_h, P.zplane, P.z_scale, P.fz);
+}
+
+__global__ void __launch_bounds__(GATHER_THREADS) g_gather_narrow_kernel(GroupDev g) {
+  for_items(g, GL_GATHER, [](const GProblem &P, int j) {
+    gather_narrow_body(P.mode, P.Bc, P.ldm, P.m, P.ldn, P.Vx, P.vmask, z_out(P, j), j);
   });
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(GATHER_THREADS) g_gather_kernel(GroupDev g) {
-  for_items(g, GL_GA0 + MODE, [](const GProblem &P, int j) {
-    gather_bv_body<MODE>(P.Bc, P.ldm, P.m, P.ldn, P.Vx, P.vmask, P.Z_hi, P.Z_lo, P.fz,
-                         P.ctl + GCTL_GATE, P.sparse_cap, P.Z_b, P.Z_h, P.zplane, P.z_scale,
-                         P.ctl + CTL_STOP, j);
+// the lists take the dense planes' place (not read on sparse steps)
+__global__ void __launch_bounds__(GATHER_THREADS) g_gather_list_kernel(GroupDev g) {
+  for_items(g, GL_LIST, [](const GProblem &P, int j) {
+    gather_list_body(P.ldn, P.Vx, P.vmask, P.sparse_cap, reinterpret_cast<int2 *>(P.V_h), j);
   });
 }
 
-// dense steps before Z = B V: the FP16 planes of V (the problems of mode `mode`)
+__global__ void __launch_bounds__(GATHER_THREADS) g_gather_tile_kernel(GroupDev g) {
+  for_items(g, GL_TILE, [](const GProblem &P, int item) {
+    gather_tile_body(P.Bc, P.ldm, P.ldn, P.k, reinterpret_cast<const int2 *>(P.V_h), P.Z_hi, item);
+  });
+}
+
+// dense steps before Z = B V: the FP16 planes of V
 __global__ void __launch_bounds__(DENSIFY_THREADS, DENSIFY_BLOCKS_PER_SM)
-    g_densify_kernel(GroupDev g, int mode) {
-  for_items(g, GL_DN0 + mode, [](const GProblem &P, int j) {
+    g_densify_kernel(GroupDev g) {
+  for_items(g, GL_DENSE, [](const GProblem &P, int j) {
     densify_fp16_body(P.Vx, P.vmask, P.ldn, P.n, P.V_h, (size_t)P.k * P.ldn, P.v_scale,
                       P.ctl + GCTL_GATE, P.sparse_cap, P.ctl + CTL_STOP, j);
   });
 }
 
-// dense steps after Z = B V: the split-K sum and the sign / norm / normalise
-template <int MODE>
+// after Z = B V: the split-K sum of dense steps, the end of the tiled gathers
 __global__ void __launch_bounds__(256) g_z_reduce_kernel(GroupDev g) {
-  for_items(g, GL_DN0 + MODE, [](const GProblem &P, int j) {
-    z_reduce_body<MODE>(P.ws, P.splits1, P.m_tiles1, P.n_tiles1, P.bn, P.m, P.Z_hi, P.Z_lo,
-                        P.ldm, P.fz, P.ctl + GCTL_GATE, P.sparse_cap, P.Z_b, P.Z_h, P.zplane,
-                        P.z_scale, P.ctl + CTL_STOP, j);
-  }, GL_COUNT + MODE);
+  for_items(g, GL_DENSE, [](const GProblem &P, int j) {
+    z_reduce_body(P.mode, P.ws, P.splits1, P.m_tiles1, P.n_tiles1, P.bn, P.m, z_out(P, j), j);
+  }, GL_COUNT);
+  for_items(g, GL_FINISH,
+            [](const GProblem &P, int j) { z_finish_body(P.mode, P.m, z_out(P, j)); });
 }
 
 __global__ void __launch_bounds__(HARD_THREADS) g_hard_select_kernel(GroupDev g) {

@@ -129,8 +129,9 @@ struct StepParams {
   int stop_check = 0;  // the step sets the stop word when the batch loop would end
 };
 
-// The sparse Z = B V runs four starts per block while no column has more
-// than this many non-zeros (and the sparse bound allows the gather at all).
+// The sparse Z = B V of matrices with few samples is one launch, which
+// am24_batch_step_timed names AM24_KERNEL_GATHER_BV_GROUP up to this many
+// non-zeros per column and AM24_KERNEL_GATHER_BV above.
 constexpr uint32_t GATHER_GROUP_MAX_NNZ = 1024;
 
 // Run-ahead control words of a batch (BatchDev::ctl).  Every step kernel
@@ -164,15 +165,11 @@ struct TensorMaps {
 // a function of that problem alone (its own tiles, split-K and reduction
 // order), so its result is the same bit for bit whatever else runs beside it.
 enum GList : int {
-  GL_GG0 = 0,  // sparse V with at most 1024 non-zeros: ceil(k / 4) items, by mode 0..2
-  GL_GG1,
-  GL_GG2,
-  GL_GA0,      // sparse V with more non-zeros: k items, by mode
-  GL_GA1,
-  GL_GA2,
-  GL_DN0,      // dense V (densify, then the split-K reduction): k items, by mode
-  GL_DN1,
-  GL_DN2,
+  GL_GATHER = 0,  // sparse V, few samples: k
+  GL_LIST,        // sparse V, many samples: k (the starts' non-zeros listed) ...
+  GL_TILE,        // ... (tiles of 128 samples) x (groups of 8 starts) ...
+  GL_FINISH,      // ... and k (norms and output planes)
+  GL_DENSE,       // dense V (densify, then the split-K reduction): k
   GL_SEL_HARD,   // k (top-s)
   GL_SEL_SCAN,   // k (L1 ball, the reference's scan)
   GL_SEL_EXACT,  // k (L1 ball, exact)
@@ -254,10 +251,10 @@ struct GPlan {
   int loops;            // steps run since the last launch began
   int loop_cap;         // the launch stops after this many steps
   int status;           // a device-side wait of a grouped kernel gave up
-  // per list, the next item a per-column kernel's block takes; the dense lists
-  // are walked twice a step (densify, then the split-K reduction), which the
-  // last three counters serve
-  int next[GL_COUNT + 3];
+  // per list, the next item a per-column kernel's block takes; the dense list
+  // is walked twice a step (densify, then the split-K reduction), which the
+  // last counter serves
+  int next[GL_COUNT + 1];
 };
 
 // Device arrays of a group, sized for `cap` problems.
@@ -276,7 +273,7 @@ struct GroupDev {
 // One grouped AM step of every live, unstopped problem; the plan kernel first.
 // grids: per-kernel persistent grid sizes (from grouped_grids()).
 struct GroupGrids {
-  int plan_threads, col, select_hard, select_soft, gather, gather_group, fin, pairs;
+  int plan_threads, col, select_hard, select_soft, gather, gather_tile, fin, pairs;
 };
 cudaError_t grouped_grids(GroupGrids *g);
 cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &grids, cudaStream_t st);
@@ -359,6 +356,8 @@ cudaError_t launch_sparse_ev(const SparseDev &S, const float *x, double *scratch
                              cudaStream_t st);
 inline size_t sparse_ev_scratch(const SparseDev &S) { return (size_t)(S.m + 255) / 256 + 2; }
 int num_sms();
+// Whether the sparse Z = B V of m samples is the listed, tiled form.
+bool gather_is_wide(int m);
 // Fills M's TF32 planes (Bc_hi/lo, Bt_hi/lo) from M.Bc.
 cudaError_t launch_prep_tf32_planes(MatrixDev &M, cudaStream_t st);
 // Fills M.Bc_b3 from M.Bc (its M.bf16_planes planes).

@@ -525,25 +525,76 @@ __global__ void __launch_bounds__(DENSIFY_THREADS, DENSIFY_BLOCKS_PER_SM) densif
 }
 
 // ------------------------------------------------------------ Z reduction
-// MODE 0: L2 variance, constrained  -> z = y, fz = ||y||_2  (gpower_commons.h:100)
-// MODE 1: L1 variance               -> z = sgn(y), fz = ||y||_1 (:85-86, :156)
-// MODE 2: L2 variance, penalized    -> z = y * (1/||y||_2)     (:163-164)
-template <int MODE>
-__device__ __forceinline__ void z_reduce_body(const float *__restrict__ ws, int splits,
+// What becomes of y = B v, by mode:
+// 0: L2 variance, constrained  -> z = y, fz = ||y||_2  (gpower_commons.h:100)
+// 1: L1 variance               -> z = sgn(y), fz = ||y||_1 (:85-86, :156)
+// 2: L2 variance, penalized    -> z = y * (1/||y||_2)     (:163-164)
+struct ZOut {
+  float *hi, *lo;     // one start's FP32 planes (hi + lo = z), ldm each
+  uint16_t *b;        // its BF16 z (null: not wanted)
+  uint16_t *h;        // its FP16 z (null: not wanted); second plane at h + plane
+  size_t plane;
+  float *scale, *fz;  // the start's words
+};
+__device__ __forceinline__ ZOut z_out(int j, int ldm, float *Z_hi, float *Z_lo, uint16_t *Zb,
+                                      uint16_t *Zh, size_t zplane, float *zscale, float *fz) {
+  const size_t o = (size_t)j * ldm;
+  return ZOut{Z_hi + o, Z_lo + o, Zb ? Zb + o : nullptr, Zh ? Zh + o : nullptr, zplane,
+              zscale ? zscale + j : nullptr, fz + j};
+}
+// Sample i's y before the norm is known: its share of the norm into acc, and
+// what can be stored already.  In mode 2 the planes are stored only when `keep`
+// (the second pass reads y back from them).
+__device__ __forceinline__ void z_emit(const ZOut &z, int mode, int i, float y, bool keep,
+                                       double &acc) {
+  if (mode == 1) {
+    acc += (double)fabsf(y);
+    z.hi[i] = sgnf(y);
+    z.lo[i] = 0.f;
+    if (z.b) z.b[i] = bf16_sign(y);
+    if (z.h) z.h[i] = f16_sign(y);
+  } else {
+    acc += (double)y * (double)y;
+    if (mode == 0 || keep) split_store(y, z.hi + i, z.lo + i);
+    if (mode == 0 && z.b) z.b[i] = bf16_bits(y);
+  }
+}
+__device__ __forceinline__ bool z_second_pass(const ZOut &z, int mode) {
+  return mode == 2 || (mode == 0 && z.h);
+}
+// Second pass over sample i: mode 2 normalises; both write the FP16 planes of
+// z * 2^s, s from a bound on |z| (||y||_2, or 1 for the normalised z).
+struct ZScale {
+  float inv, sc;
+  int s;
+};
+__device__ __forceinline__ ZScale z_scales(int mode, double tot) {
+  ZScale r;
+  r.inv = mode == 2 ? 1.0f / (float)sqrt(tot) : 1.0f;
+  r.s = fp16_shift(mode == 2 ? 1.0f : (float)sqrt(tot));
+  r.sc = pow2f(r.s);
+  return r;
+}
+__device__ __forceinline__ void z_emit2(const ZOut &z, int mode, const ZScale &c, int i, float y) {
+  const float v = mode == 2 ? y * c.inv : y;
+  if (mode == 2) {
+    split_store(v, z.hi + i, z.lo + i);
+    if (z.b) z.b[i] = bf16_bits(v);
+  }
+  if (z.h) fp16_split(v * c.sc, z.h + i, z.h + z.plane + i);
+}
+__device__ __forceinline__ void z_close(const ZOut &z, int mode, double tot) {  // one thread
+  if (z_second_pass(z, mode) && z.h) *z.scale = pow2f(-z_scales(mode, tot).s);
+  if (mode != 2) *z.fz = (mode == 1) ? (float)tot : (float)sqrt(tot);
+}
+
+// Dense steps: y from the split-K partial tiles of Z = B V.
+__device__ __forceinline__ void z_reduce_body(int mode, const float *__restrict__ ws, int splits,
                                               int m_tiles, int n_tiles, int bn, int m,
-                                              float *__restrict__ Z_hi, float *__restrict__ Z_lo,
-                                              int ldm, float *__restrict__ fz,
-                                              const uint32_t *gate, uint32_t gate_max,
-                                              uint16_t *__restrict__ Zb,
-                                              uint16_t *__restrict__ Zh, size_t zplane,
-                                              float *__restrict__ zscale, const uint32_t *stop,
-                                              int j) {
+                                              const ZOut &z, int j) {
   __shared__ double red[32];
-  if (*stop || *gate <= gate_max) return;  // the gather kernel produced Z this step
   const int nt = j / bn, c = j - nt * bn;
   const size_t unit_stride = (size_t)bn * BM;
-  float *zh = Z_hi + (size_t)j * ldm;
-  float *zl = Z_lo + (size_t)j * ldm;
   double acc = 0.0;
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     const int mt = i >> 7, r = i & 127;
@@ -552,51 +603,61 @@ __device__ __forceinline__ void z_reduce_body(const float *__restrict__ ws, int 
       const size_t u = ((size_t)s * m_tiles + mt) * n_tiles + nt;
       y += ws[u * unit_stride + (size_t)c * BM + r];
     }
-    if (MODE == 1) {
-      acc += (double)fabsf(y);
-      zh[i] = sgnf(y);
-      zl[i] = 0.f;
-      if (Zb) Zb[(size_t)j * ldm + i] = bf16_sign(y);
-      if (Zh) Zh[(size_t)j * ldm + i] = f16_sign(y);
-    } else {
-      acc += (double)y * (double)y;
-      split_store(y, zh + i, zl + i);
-      if (MODE == 0 && Zb) Zb[(size_t)j * ldm + i] = bf16_bits(y);
-    }
+    z_emit(z, mode, i, y, true, acc);
   }
   const double tot = block_sum(acc, red);
-  if (MODE == 2 || (MODE == 0 && Zh)) {
-    // second pass: MODE 2 normalises; both write the FP16 planes of z * 2^s,
-    // s from a bound on |z| (||y||_2, or 1 for the normalised z)
-    const float inv = MODE == 2 ? 1.0f / (float)sqrt(tot) : 1.0f;
-    const int s = fp16_shift(MODE == 2 ? 1.0f : (float)sqrt(tot));
-    const float sc = pow2f(s);
-    for (int i = threadIdx.x; i < m; i += blockDim.x) {
-      const float y = zh[i] + zl[i];  // exact: this thread wrote both planes
-      const float z = MODE == 2 ? y * inv : y;
-      if (MODE == 2) {
-        split_store(z, zh + i, zl + i);
-        if (Zb) Zb[(size_t)j * ldm + i] = bf16_bits(z);
-      }
-      if (Zh) fp16_split(z * sc, Zh + (size_t)j * ldm + i, Zh + zplane + (size_t)j * ldm + i);
-    }
-    if (Zh && threadIdx.x == 0) zscale[j] = pow2f(-s);
+  if (z_second_pass(z, mode)) {
+    const ZScale sc = z_scales(mode, tot);
+    for (int i = threadIdx.x; i < m; i += blockDim.x)
+      z_emit2(z, mode, sc, i, z.hi[i] + z.lo[i]);  // exact: this thread wrote both planes
   }
-  if (MODE != 2 && threadIdx.x == 0) fz[j] = (MODE == 1) ? (float)tot : (float)sqrt(tot);
+  if (threadIdx.x == 0) z_close(z, mode, tot);
 }
-template <int MODE>
-__global__ void __launch_bounds__(256) z_reduce_kernel(const float *__restrict__ ws, int splits,
-                                                       int m_tiles, int n_tiles, int bn, int m,
-                                                       float *__restrict__ Z_hi,
+
+// Sparse steps of matrices with more than GATHER_NARROW samples: y from the
+// plane gather_tile_body left it in (z.hi).  256 threads, 4 consecutive samples
+// each, 2048 samples per round.
+__device__ __forceinline__ void z_finish_body(int mode, int m, const ZOut &z) {
+  __shared__ double red[32];
+  double acc = 0.0;
+  for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x) {
+    const float4 y = *reinterpret_cast<const float4 *>(z.hi + i);
+    const float e[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+      if (i + c < m) z_emit(z, mode, i + c, e[c], true, acc);
+  }
+  const double tot = block_sum(acc, red);
+  if (z_second_pass(z, mode)) {
+    const ZScale sc = z_scales(mode, tot);
+    for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x)
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+        if (i + c < m) z_emit2(z, mode, sc, i + c, z.hi[i + c] + z.lo[i + c]);
+  }
+  if (threadIdx.x == 0) z_close(z, mode, tot);
+}
+
+// One block per start: the dense step's reduction, or the end of a sparse
+// step's tiled gather (`wide`).
+__global__ void __launch_bounds__(256) z_reduce_kernel(int mode, const float *__restrict__ ws,
+                                                       int splits, int m_tiles, int n_tiles,
+                                                       int bn, int m, float *__restrict__ Z_hi,
                                                        float *__restrict__ Z_lo, int ldm,
                                                        float *__restrict__ fz,
                                                        const uint32_t *gate, uint32_t gate_max,
                                                        uint16_t *__restrict__ Zb,
                                                        uint16_t *__restrict__ Zh, size_t zplane,
-                                                       float *__restrict__ zscale,
+                                                       float *__restrict__ zscale, bool wide,
                                                        const uint32_t *stop) {
-  z_reduce_body<MODE>(ws, splits, m_tiles, n_tiles, bn, m, Z_hi, Z_lo, ldm, fz, gate, gate_max,
-                      Zb, Zh, zplane, zscale, stop, blockIdx.x);
+  if (*stop) return;
+  const bool dense = *gate > gate_max;
+  if (!dense && !wide) return;  // gather_narrow_kernel produced Z this step
+  const ZOut z = z_out(blockIdx.x, ldm, Z_hi, Z_lo, Zb, Zh, zplane, zscale, fz);
+  if (dense)
+    z_reduce_body(mode, ws, splits, m_tiles, n_tiles, bn, m, z, blockIdx.x);
+  else
+    z_finish_body(mode, m, z);
 }
 
 // ------------------------------------------------------------ sparse Z = B V
@@ -608,7 +669,6 @@ __device__ __forceinline__ uint32_t mixed_next_phase(uint32_t ph, bool stable_en
   if (ph >= 2u) return ph == 2u ? 0u : ph - 1u;
   return (ph == 0u && stable_enough) ? 1u : ph;
 }
-constexpr int GATHER_ROWS = 8;  // samples per thread per pass
 constexpr int GATHER_CAP = 4096;
 
 // MIXED precision bookkeeping, after the step's non-zero masks are written:
@@ -649,32 +709,36 @@ __global__ void __launch_bounds__(256) support_kernel(const uint32_t *__restrict
   }
 }
 
-// Z = B V for one start when V's column has few non-zeros: runs instead of
-// gemm1 + z_reduce when the previous step left at most gate_max non-zeros in
-// every column (*gate).  The column's non-zero rows are listed in index order
-// from its bitmask, then z = sum_q v_q B[:, q] is accumulated with FP32 FMAs in
-// that fixed order (deterministic), and the same sign / norm / normalise
-// step as z_reduce_kernel<MODE> finishes the column.
-template <int MODE>
-__device__ __forceinline__ void gather_bv_body(
-    const float *__restrict__ Bc, int ldm, int m, int ldn,
-    const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi,
-    float *__restrict__ Z_lo, float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max,
-    uint16_t *__restrict__ Zb, uint16_t *__restrict__ Zh, size_t zplane,
-    float *__restrict__ zscale, const uint32_t *stop, int j) {
-  __shared__ int idx[GATHER_CAP];
-  __shared__ float val[GATHER_CAP];
-  __shared__ uint32_t wsum[GATHER_THREADS / 32];
-  __shared__ double red[32];
-  // dense V (gemm1 + z_reduce), or few enough non-zeros for gather_bv_group_kernel
-  if (*stop || *gate > gate_max || *gate <= min(gate_max, GATHER_GROUP_MAX_NNZ)) return;
+// The sparse Z = B V: z = sum_q v_q B[:, q] over the column's non-zeros, in index
+// order with FP32 FMAs (deterministic), on steps whose previous step left at
+// most gate_max non-zeros in every column (*gate); the FP32 rows of Bc are read.
+// Two forms, by the matrix's number of samples:
+//   up to GATHER_NARROW   one block per start and one launch: the list of
+//       non-zeros in shared memory, four samples per thread, the norm and the
+//       output planes from registers.  A chain of loads bounds it.
+//   above                 gather_list_kernel writes every start's list to
+//       memory once; gather_tile_kernel gives each (start, 128 samples) a warp
+//       that reads one 512-byte row segment per non-zero, the tiles of 128
+//       samples one after another over all starts, so that the segments in use
+//       (512 bytes per feature) stay in L2; z_finish_body closes the columns.
+//       L2 reads bound it (12.5 TB/s at 8192 samples, 4096 starts).
+// Measured against one kernel of four starts per block walking whole rows:
+// 8192 x 65536, 4096 starts of 128 non-zeros 2.47 -> 1.38 ms; 2000 x 50000, 1024
+// starts of 240 to 400: 204..302 -> 155..243 us (beyond 1024 non-zeros, 638 ->
+// 360); 400 samples, 64 starts of 16: 14 -> 5.4 us; 1000 samples, 256 starts of
+// 40 to 100: 54..100 -> 14..23 us, where the listed form takes 6 + 20..36.
+// The list of start j: a header {count, 0}, then (row, value bits) pairs.
+
+// The non-zeros of a column (its mask words) in index order through
+// put(position, row); returns their number.  Each thread of the block
+// owns a contiguous run of words, so an exclusive scan of their counts places
+// the entries.  wsum: a word per warp.
+template <class Put>
+__device__ __forceinline__ uint32_t list_column(const uint32_t *__restrict__ mk, int words,
+                                                uint32_t *wsum, Put put) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int words = ldn >> 5;
-  const uint32_t *mk = vmask + (size_t)j * words;
-  // each thread owns a contiguous run of mask words, so the block-wide
-  // exclusive scan of their popcounts lists rows in index order
   const int per = (words + GATHER_THREADS - 1) / GATHER_THREADS;
-  const int w0 = min(words, threadIdx.x * per), w1 = min(words, w0 + per);
+  const int w0 = min(words, (int)threadIdx.x * per), w1 = min(words, w0 + per);
   uint32_t cnt = 0;
   for (int q = w0; q < w1; q++) cnt += __popc(mk[q]);
   uint32_t incl = cnt;
@@ -685,367 +749,168 @@ __device__ __forceinline__ void gather_bv_body(
   }
   if (lane == 31) wsum[w] = incl;
   __syncthreads();
-  uint32_t off = incl - cnt;
-  for (int i = 0; i < w; i++) off += wsum[i];
-  uint32_t total = 0;
-  for (int i = 0; i < GATHER_THREADS / 32; i++) total += wsum[i];
-  if (total > (uint32_t)GATHER_CAP) total = GATHER_CAP;  // cannot happen below the gate
-  const float *vx = Vx + (size_t)j * ldn;
-  for (int q = w0; q < w1; q++) {
-    uint32_t bits = mk[q];
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1;
-      const int r = q * 32 + b;
-      if (off < (uint32_t)GATHER_CAP) {
-        idx[off] = r;
-        val[off] = vx[r];
-      }
-      off++;
-    }
+  uint32_t off = incl - cnt, total = 0;
+#pragma unroll
+  for (int i = 0; i < GATHER_THREADS / 32; i++) {
+    if (i < w) off += wsum[i];
+    total += wsum[i];
   }
+  for (int q = w0; q < w1; q++)
+    for (uint32_t bits = mk[q]; bits; bits &= bits - 1) put(off++, q * 32 + __ffs(bits) - 1);
   __syncthreads();
-  // Each thread accumulates 2 x 4 consecutive samples per pass (16-byte loads);
-  // the rows of four non-zeros are loaded before their FMAs, which still run in
-  // index order per sample.  Samples in [m, ldm) read B's zero padding.
-  constexpr int G4 = GATHER_ROWS / 4;
-  double acc = 0.0;
-  float4 y[G4];
-  float *zh = Z_hi + (size_t)j * ldm;
-  float *zl = Z_lo + (size_t)j * ldm;
-  uint16_t *zb = Zb ? Zb + (size_t)j * ldm : nullptr;
-  uint16_t *zh0 = Zh ? Zh + (size_t)j * ldm : nullptr;
-  const int chunk = GATHER_THREADS * GATHER_ROWS;
-  const int ld4 = ldm >> 2;
-  const bool one_pass = m <= chunk;
-  auto sample = [&](int base, int r) { return base + 4 * (r * GATHER_THREADS + (int)threadIdx.x); };
-  auto fma4 = [](float v, const float4 &b, float4 &acc4) {
-    acc4.x = fmaf(v, b.x, acc4.x);
-    acc4.y = fmaf(v, b.y, acc4.y);
-    acc4.z = fmaf(v, b.z, acc4.z);
-    acc4.w = fmaf(v, b.w, acc4.w);
-  };
-  // the final value of sample i (c of the float4), stored as Z needs it
-  auto emit = [&](int i, float yv) {
-    if (MODE == 1) {
-      acc += (double)fabsf(yv);
-      zh[i] = sgnf(yv);
-      zl[i] = 0.f;
-      if (zb) zb[i] = bf16_sign(yv);
-      if (zh0) zh0[i] = f16_sign(yv);
-    } else {
-      acc += (double)yv * (double)yv;
-      if (!(MODE == 2 && one_pass)) split_store(yv, zh + i, zl + i);
-      if (MODE == 0 && zb) zb[i] = bf16_bits(yv);
-    }
-  };
-  for (int base = 0; base < m; base += chunk) {
-    int i4[G4];
-    bool ok[G4];
-#pragma unroll
-    for (int r = 0; r < G4; r++) {
-      y[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-      i4[r] = sample(base, r) >> 2;
-      ok[r] = i4[r] < ld4;
-    }
-    uint32_t q = 0;
-    for (; q + 4 <= total; q += 4) {
-      float4 bq[4][G4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const float4 *row4 = reinterpret_cast<const float4 *>(Bc + (size_t)idx[q + u] * ldm);
-#pragma unroll
-        for (int r = 0; r < G4; r++)
-          bq[u][r] = ok[r] ? __ldg(row4 + i4[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const float v = val[q + u];
-#pragma unroll
-        for (int r = 0; r < G4; r++) fma4(v, bq[u][r], y[r]);
-      }
-    }
-    for (; q < total; q++) {
-      const float4 *row4 = reinterpret_cast<const float4 *>(Bc + (size_t)idx[q] * ldm);
-      const float v = val[q];
-#pragma unroll
-      for (int r = 0; r < G4; r++)
-        if (ok[r]) fma4(v, __ldg(row4 + i4[r]), y[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < G4; r++) {
-      const int i = sample(base, r);
-      const float e[4] = {y[r].x, y[r].y, y[r].z, y[r].w};
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-        if (i + c < m) emit(i + c, e[c]);
-    }
-  }
-  const double tot = block_sum(acc, red);
-  if (MODE == 2 || (MODE == 0 && zh0)) {
-    // as in z_reduce_kernel: MODE 2 normalises, both write the FP16 planes
-    const float inv = MODE == 2 ? 1.0f / (float)sqrt(tot) : 1.0f;
-    const int s = fp16_shift(MODE == 2 ? 1.0f : (float)sqrt(tot));
-    const float sc = pow2f(s);
-    for (int base = 0; base < m; base += chunk) {
-#pragma unroll
-      for (int r = 0; r < G4; r++) {
-        const int i = sample(base, r);
-        const float e[4] = {y[r].x, y[r].y, y[r].z, y[r].w};
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          if (i + c >= m) continue;
-          // one pass: the sums are still in registers; else re-read what this
-          // thread wrote (hi + lo is exact)
-          const float v = one_pass ? e[c] : zh[i + c] + zl[i + c];
-          const float z = MODE == 2 ? v * inv : v;
-          if (MODE == 2) {
-            split_store(z, zh + i + c, zl + i + c);
-            if (zb) zb[i + c] = bf16_bits(z);
-          }
-          if (zh0) fp16_split(z * sc, zh0 + i + c, zh0 + zplane + i + c);
-        }
-      }
-    }
-    if (zh0 && threadIdx.x == 0) zscale[j] = pow2f(-s);
-  }
-  if (MODE != 2 && threadIdx.x == 0) fz[j] = (MODE == 1) ? (float)tot : (float)sqrt(tot);
-}
-template <int MODE>
-__global__ void __launch_bounds__(GATHER_THREADS) gather_bv_kernel(
-    const float *__restrict__ Bc, int ldm, int m, int ldn,
-    const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi,
-    float *__restrict__ Z_lo, float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max,
-    uint16_t *__restrict__ Zb, uint16_t *__restrict__ Zh, size_t zplane,
-    float *__restrict__ zscale, const uint32_t *stop) {
-  gather_bv_body<MODE>(Bc, ldm, m, ldn, Vx, vmask, Z_hi, Z_lo, fz, gate, gate_max, Zb, Zh, zplane,
-                       zscale, stop, blockIdx.x);
+  return total;
 }
 
-// The sparse Z = B V for GATHER_GROUP starts per block, while every column
-// has at most GATHER_CAP / GATHER_GROUP non-zeros (*gate): the block lists the
-// union of the group's non-zero rows in index order, loads each row once, and
-// adds it to the sums of the starts it belongs to.  Every start's FMAs still
-// run over its own non-zeros in index order, so the result is bit for bit that
-// of gather_bv_kernel, with a quarter of the row loads where supports overlap.
-// Above the group bound this kernel returns at once and gather_bv_kernel runs.
-constexpr int GATHER_GROUP = 4;
-static_assert(GATHER_GROUP_MAX_NNZ == GATHER_CAP / GATHER_GROUP, "group bound");
-constexpr size_t GATHER_GROUP_SMEM =
-    (size_t)GATHER_CAP * (sizeof(int) + GATHER_GROUP * sizeof(float) + 1);
+__device__ __forceinline__ void fma4(float v, const float4 &b, float4 &acc) {
+  acc.x = fmaf(v, b.x, acc.x);
+  acc.y = fmaf(v, b.y, acc.y);
+  acc.z = fmaf(v, b.z, acc.z);
+  acc.w = fmaf(v, b.w, acc.w);
+}
 
-template <int MODE>
-__device__ __forceinline__ void gather_bv_group_body(
-    const float *__restrict__ Bc, int ldm, int m, int ldn, int k,
-    const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi,
-    float *__restrict__ Z_lo, float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max,
-    uint16_t *__restrict__ Zb, uint16_t *__restrict__ Zh, size_t zplane,
-    float *__restrict__ zscale, const uint32_t *stop, int group) {
-  constexpr int G = GATHER_GROUP;
-  extern __shared__ __align__(16) uint8_t gsm[];
-  int *idx = reinterpret_cast<int *>(gsm);                                  // GATHER_CAP
-  float *val = reinterpret_cast<float *>(gsm + sizeof(int) * GATHER_CAP);   // G x GATHER_CAP
-  uint8_t *memb = gsm + (sizeof(int) + G * sizeof(float)) * GATHER_CAP;     // GATHER_CAP
+constexpr int GATHER_NARROW = 4 * GATHER_THREADS;  // samples one block holds in registers
+__device__ __forceinline__ void gather_narrow_body(int mode, const float *__restrict__ Bc, int ldm,
+                                                   int m, int ldn, const float *__restrict__ Vx,
+                                                   const uint32_t *__restrict__ vmask,
+                                                   const ZOut &z, int j) {
+  __shared__ int list[GATHER_CAP];
+  __shared__ float val[GATHER_CAP];
   __shared__ uint32_t wsum[GATHER_THREADS / 32];
   __shared__ double red[32];
-  // dense V (gemm1 + z_reduce), or gather_bv_kernel's case
-  if (*stop || *gate > min(gate_max, GATHER_GROUP_MAX_NNZ)) return;
-  const int j0 = group * G;
-  const int ng = min(G, k - j0);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int words = ldn >> 5;
-  const uint32_t *mk[G];
-  const float *vx[G];
+  const float *vx = Vx + (size_t)j * ldn;
+  uint32_t total = list_column(vmask + (size_t)j * words, words, wsum, [&](uint32_t at, int r) {
+    if (at < (uint32_t)GATHER_CAP) list[at] = r;
+  });
+  total = min(total, (uint32_t)GATHER_CAP);  // more cannot happen below the gate
+  // a batch of rows is loaded before its FMAs (a short list's values with them);
+  // samples in [m, ldm) read B's zeros
+  constexpr uint32_t SHORT = 16, U = 8;
+  const int i4 = threadIdx.x;
+  const bool on = i4 < (ldm >> 2);
+  const float4 *B4 = reinterpret_cast<const float4 *>(Bc) + (on ? i4 : 0);
+  const size_t ld4 = (size_t)ldm >> 2;
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (total <= SHORT) {
+    float4 b[SHORT];
+    float v[SHORT];
 #pragma unroll
-  for (int g = 0; g < G; g++) {
-    const int j = j0 + min(g, ng - 1);  // past the last start: a repeat, never a member
-    mk[g] = vmask + (size_t)j * words;
-    vx[g] = Vx + (size_t)j * ldn;
-  }
-  auto word = [&](int g, int q) { return g < ng ? mk[g][q] : 0u; };
-  // the union's rows in index order: an exclusive scan over threads' word runs
-  const int per = (words + GATHER_THREADS - 1) / GATHER_THREADS;
-  const int w0 = min(words, threadIdx.x * per), w1 = min(words, w0 + per);
-  uint32_t cnt = 0;
-  for (int q = w0; q < w1; q++) {
-    uint32_t u = 0;
-#pragma unroll
-    for (int g = 0; g < G; g++) u |= word(g, q);
-    cnt += __popc(u);
-  }
-  uint32_t incl = cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) wsum[w] = incl;
-  __syncthreads();
-  uint32_t off = incl - cnt;
-  for (int i = 0; i < w; i++) off += wsum[i];
-  uint32_t total = 0;
-  for (int i = 0; i < GATHER_THREADS / 32; i++) total += wsum[i];
-  if (total > (uint32_t)GATHER_CAP) total = GATHER_CAP;  // cannot happen below the gate
-  for (int q = w0; q < w1; q++) {
-    uint32_t wg[G], u = 0;
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      wg[g] = word(g, q);
-      u |= wg[g];
-    }
-    while (u) {
-      const int b = __ffs(u) - 1;
-      u &= u - 1;
-      const int r = q * 32 + b;
-      if (off < (uint32_t)GATHER_CAP) {
-        idx[off] = r;
-        uint32_t mb = 0;
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-          const bool in = (wg[g] >> b) & 1u;
-          mb |= (uint32_t)in << g;
-          val[g * GATHER_CAP + off] = in ? vx[g][r] : 0.f;
-        }
-        memb[off] = (uint8_t)mb;
+    for (uint32_t u = 0; u < SHORT; u++)
+      if (on && u < total) {
+        b[u] = __ldg(B4 + list[u] * ld4);
+        v[u] = vx[list[u]];
       }
-      off++;
-    }
-  }
-  __syncthreads();
-  constexpr int G4 = GATHER_ROWS / 4;
-  double acc[G];
-  float4 y[G][G4];
-  const int chunk = GATHER_THREADS * GATHER_ROWS;
-  const int ld4 = ldm >> 2;
-  const bool one_pass = m <= chunk;
-  auto sample = [&](int base, int r) { return base + 4 * (r * GATHER_THREADS + (int)threadIdx.x); };
-  auto fma4 = [](float v, const float4 &b, float4 &acc4) {
-    acc4.x = fmaf(v, b.x, acc4.x);
-    acc4.y = fmaf(v, b.y, acc4.y);
-    acc4.z = fmaf(v, b.z, acc4.z);
-    acc4.w = fmaf(v, b.w, acc4.w);
-  };
 #pragma unroll
-  for (int g = 0; g < G; g++) acc[g] = 0.0;
-  // sample i of start g, as gather_bv_kernel's emit stores it
-  auto emit = [&](int g, int i, float yv) {
-    const size_t o = (size_t)(j0 + g) * ldm + i;
-    if (MODE == 1) {
-      acc[g] += (double)fabsf(yv);
-      Z_hi[o] = sgnf(yv);
-      Z_lo[o] = 0.f;
-      if (Zb) Zb[o] = bf16_sign(yv);
-      if (Zh) Zh[o] = f16_sign(yv);
-    } else {
-      acc[g] += (double)yv * (double)yv;
-      if (!(MODE == 2 && one_pass)) split_store(yv, Z_hi + o, Z_lo + o);
-      if (MODE == 0 && Zb) Zb[o] = bf16_bits(yv);
-    }
-  };
-  for (int base = 0; base < m; base += chunk) {
-    int i4[G4];
-    bool ok[G4];
-#pragma unroll
-    for (int r = 0; r < G4; r++) {
-      i4[r] = sample(base, r) >> 2;
-      ok[r] = i4[r] < ld4;
-#pragma unroll
-      for (int g = 0; g < G; g++) y[g][r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+    for (uint32_t u = 0; u < SHORT; u++)
+      if (on && u < total) fma4(v[u], b[u], y);
+  } else {
+    for (uint32_t q = threadIdx.x; q < total; q += GATHER_THREADS) val[q] = vx[list[q]];
+    __syncthreads();
     uint32_t q = 0;
-    for (; q + 4 <= total; q += 4) {
-      float4 bq[4][G4];
+    for (; on && q + U <= total; q += U) {
+      float4 b[U];
 #pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const float4 *row4 = reinterpret_cast<const float4 *>(Bc + (size_t)idx[q + u] * ldm);
+      for (uint32_t u = 0; u < U; u++) b[u] = __ldg(B4 + list[q + u] * ld4);
 #pragma unroll
-        for (int r = 0; r < G4; r++)
-          bq[u][r] = ok[r] ? __ldg(row4 + i4[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        const uint32_t mb = memb[q + u];
-#pragma unroll
-        for (int g = 0; g < G; g++) {
-          if (!((mb >> g) & 1u)) continue;
-          const float v = val[g * GATHER_CAP + q + u];
-#pragma unroll
-          for (int r = 0; r < G4; r++) fma4(v, bq[u][r], y[g][r]);
-        }
-      }
+      for (uint32_t u = 0; u < U; u++) fma4(val[q + u], b[u], y);
     }
-    for (; q < total; q++) {
-      const float4 *row4 = reinterpret_cast<const float4 *>(Bc + (size_t)idx[q] * ldm);
-      const uint32_t mb = memb[q];
-      float4 b[G4];
+    float4 b[U];
 #pragma unroll
-      for (int r = 0; r < G4; r++) b[r] = ok[r] ? __ldg(row4 + i4[r]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t u = 0; u < U; u++)
+      if (on && q + u < total) b[u] = __ldg(B4 + list[q + u] * ld4);
 #pragma unroll
-      for (int g = 0; g < G; g++) {
-        if (!((mb >> g) & 1u)) continue;
-        const float v = val[g * GATHER_CAP + q];
-#pragma unroll
-        for (int r = 0; r < G4; r++)
-          if (ok[r]) fma4(v, b[r], y[g][r]);
-      }
-    }
-#pragma unroll
-    for (int g = 0; g < G; g++) {
-      if (g >= ng) continue;
-#pragma unroll
-      for (int r = 0; r < G4; r++) {
-        const int i = sample(base, r);
-        const float e[4] = {y[g][r].x, y[g][r].y, y[g][r].z, y[g][r].w};
-#pragma unroll
-        for (int c = 0; c < 4; c++)
-          if (i + c < m) emit(g, i + c, e[c]);
-      }
-    }
+    for (uint32_t u = 0; u < U; u++)
+      if (on && q + u < total) fma4(val[q + u], b[u], y);
   }
+  const float e[4] = {y.x, y.y, y.z, y.w};
+  double acc = 0.0;
 #pragma unroll
-  for (int g = 0; g < G; g++) {
-    if (g >= ng) continue;  // uniform over the block
-    const int j = j0 + g;
-    const double tot = block_sum(acc[g], red);
-    float *zh = Z_hi + (size_t)j * ldm, *zl = Z_lo + (size_t)j * ldm;
-    uint16_t *zb = Zb ? Zb + (size_t)j * ldm : nullptr;
-    uint16_t *zh0 = Zh ? Zh + (size_t)j * ldm : nullptr;
-    if (MODE == 2 || (MODE == 0 && zh0)) {
-      const float inv = MODE == 2 ? 1.0f / (float)sqrt(tot) : 1.0f;
-      const int s = fp16_shift(MODE == 2 ? 1.0f : (float)sqrt(tot));
-      const float sc = pow2f(s);
-      for (int base = 0; base < m; base += chunk) {
+  for (int c = 0; c < 4; c++)
+    if (4 * i4 + c < m) z_emit(z, mode, 4 * i4 + c, e[c], false, acc);
+  const double tot = block_sum(acc, red);
+  if (z_second_pass(z, mode)) {
+    const ZScale sc = z_scales(mode, tot);
 #pragma unroll
-        for (int r = 0; r < G4; r++) {
-          const int i = sample(base, r);
-          const float e[4] = {y[g][r].x, y[g][r].y, y[g][r].z, y[g][r].w};
-#pragma unroll
-          for (int c = 0; c < 4; c++) {
-            if (i + c >= m) continue;
-            const float v = one_pass ? e[c] : zh[i + c] + zl[i + c];
-            const float z = MODE == 2 ? v * inv : v;
-            if (MODE == 2) {
-              split_store(z, zh + i + c, zl + i + c);
-              if (zb) zb[i + c] = bf16_bits(z);
-            }
-            if (zh0) fp16_split(z * sc, zh0 + i + c, zh0 + zplane + i + c);
-          }
-        }
-      }
-      if (zh0 && threadIdx.x == 0) zscale[j] = pow2f(-s);
-    }
-    if (MODE != 2 && threadIdx.x == 0) fz[j] = (MODE == 1) ? (float)tot : (float)sqrt(tot);
+    for (int c = 0; c < 4; c++)
+      if (4 * i4 + c < m) z_emit2(z, mode, sc, 4 * i4 + c, e[c]);
   }
+  if (threadIdx.x == 0) z_close(z, mode, tot);
 }
-template <int MODE>
-__global__ void __launch_bounds__(GATHER_THREADS) gather_bv_group_kernel(
-    const float *__restrict__ Bc, int ldm, int m, int ldn, int k,
-    const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi,
-    float *__restrict__ Z_lo, float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max,
-    uint16_t *__restrict__ Zb, uint16_t *__restrict__ Zh, size_t zplane,
-    float *__restrict__ zscale, const uint32_t *stop) {
-  gather_bv_group_body<MODE>(Bc, ldm, m, ldn, k, Vx, vmask, Z_hi, Z_lo, fz, gate, gate_max, Zb,
-                             Zh, zplane, zscale, stop, blockIdx.x);
+__global__ void __launch_bounds__(GATHER_THREADS) gather_narrow_kernel(
+    int mode, const float *__restrict__ Bc, int ldm, int m, int ldn, const float *__restrict__ Vx,
+    const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi, float *__restrict__ Z_lo,
+    float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max, uint16_t *__restrict__ Zb,
+    uint16_t *__restrict__ Zh, size_t zplane, float *__restrict__ zscale, const uint32_t *stop) {
+  if (*stop || *gate > gate_max) return;  // dense V: gemm1 + z_reduce
+  gather_narrow_body(mode, Bc, ldm, m, ldn, Vx, vmask,
+                     z_out(blockIdx.x, ldm, Z_hi, Z_lo, Zb, Zh, zplane, zscale, fz), blockIdx.x);
+}
+
+// int2 entries between the lists of consecutive starts: the plane they live in
+// holds ldn floats per start, and a list at most n / 32 + 1 pairs.
+__device__ __forceinline__ size_t list_stride(int ldn) { return (size_t)ldn / 2; }
+__device__ __forceinline__ void gather_list_body(int ldn, const float *__restrict__ Vx,
+                                                 const uint32_t *__restrict__ vmask, uint32_t cap,
+                                                 int2 *__restrict__ lists, int j) {
+  __shared__ uint32_t wsum[GATHER_THREADS / 32];
+  const int words = ldn >> 5;
+  int2 *list = lists + (size_t)j * list_stride(ldn);
+  const float *vx = Vx + (size_t)j * ldn;
+  const uint32_t total =
+      list_column(vmask + (size_t)j * words, words, wsum, [&](uint32_t at, int r) {
+        if (at < cap) list[1 + at] = make_int2(r, __float_as_int(vx[r]));
+      });
+  if (threadIdx.x == 0) list[0] = make_int2((int)min(total, cap), 0);
+}
+__global__ void __launch_bounds__(GATHER_THREADS) gather_list_kernel(
+    int ldn, const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, const uint32_t *gate,
+    uint32_t gate_max, int2 *__restrict__ lists, const uint32_t *stop) {
+  if (*stop || *gate > gate_max) return;
+  gather_list_body(ldn, Vx, vmask, gate_max, lists, blockIdx.x);
+}
+
+constexpr int GATHER_STARTS = GATHER_THREADS / 32;  // starts per block, a warp each
+__host__ __device__ __forceinline__ int gather_groups(int k) {
+  return (k + GATHER_STARTS - 1) / GATHER_STARTS;
+}
+__host__ __device__ __forceinline__ int gather_tiles(int ldm) { return (ldm + 127) / 128; }
+// Item: tile * gather_groups(k) + group of starts.  No block barrier: warps of
+// starts past k return.
+__device__ __forceinline__ void gather_tile_body(const float *__restrict__ Bc, int ldm, int ldn,
+                                                 int k, const int2 *__restrict__ lists,
+                                                 float *__restrict__ Z_hi, int item) {
+  const int groups = gather_groups(k);
+  const int tile = item / groups;
+  const int j = (item - tile * groups) * GATHER_STARTS + ((int)threadIdx.x >> 5);
+  if (j >= k) return;
+  const int lane = threadIdx.x & 31;
+  const int i4 = tile * 32 + lane;
+  const bool on = i4 < (ldm >> 2);
+  const float4 *B4 = reinterpret_cast<const float4 *>(Bc) + (on ? i4 : tile * 32);
+  const size_t ld4 = (size_t)ldm >> 2;
+  const int2 *list = lists + (size_t)j * list_stride(ldn);
+  const int total = list[0].x;
+  float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+  auto pair = [&](int e) { return e < total ? list[1 + e] : make_int2(0, 0); };
+  int2 next = pair(lane);
+  for (int base = 0; base < total; base += 32) {
+    const int2 mine = next;
+    next = pair(base + 32 + lane);  // in flight while this chunk's rows are read
+    const int cnt = min(32, total - base);
+#pragma unroll 16
+    for (int t = 0; t < cnt; t++) {
+      const int q = __shfl_sync(FULL, mine.x, t);
+      const float v = __int_as_float(__shfl_sync(FULL, mine.y, t));
+      fma4(v, __ldg(B4 + q * ld4), y);
+    }
+  }
+  if (on) reinterpret_cast<float4 *>(Z_hi + (size_t)j * ldm)[i4] = y;
+}
+__global__ void __launch_bounds__(GATHER_THREADS) gather_tile_kernel(
+    const float *__restrict__ Bc, int ldm, int ldn, int k, const int2 *__restrict__ lists,
+    float *__restrict__ Z_hi, const uint32_t *gate, uint32_t gate_max, const uint32_t *stop) {
+  if (*stop || *gate > gate_max) return;
+  gather_tile_body(Bc, ldm, ldn, k, lists, Z_hi, blockIdx.x);
 }
 
 // ------------------------------------------------------------ radix select
@@ -2533,6 +2398,8 @@ int num_sms() {
   return sms;
 }
 
+bool gather_is_wide(int m) { return m > GATHER_NARROW; }
+
 int pick_bn(int k) { return k > 128 ? 256 : (k > 64 ? 128 : 64); }
 
 size_t ws_floats(int splits, int m_tiles, int n_tiles, int bn) {
@@ -2682,25 +2549,6 @@ cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double
   return cudaGetLastError();
 }
 
-template <int MODE>
-cudaError_t launch_gather_group_mode(const MatrixDev &M, const BatchDev &b, size_t zplane,
-                                     cudaStream_t st) {
-  const cudaError_t e = kernel_setup(gather_bv_group_kernel<MODE>, (int)GATHER_GROUP_SMEM, false);
-  if (e != cudaSuccess) return e;
-  gather_bv_group_kernel<MODE><<<(b.k + GATHER_GROUP - 1) / GATHER_GROUP, GATHER_THREADS,
-                                 GATHER_GROUP_SMEM, st>>>(
-      M.Bc, M.ldm, M.m, M.ldn, b.k, b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz, b.max_nnz,
-      b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_gather_group(const MatrixDev &M, const BatchDev &b, int mode, size_t zplane,
-                                cudaStream_t st) {
-  if (mode == 0) return launch_gather_group_mode<0>(M, b, zplane, st);
-  if (mode == 1) return launch_gather_group_mode<1>(M, b, zplane, st);
-  return launch_gather_group_mode<2>(M, b, zplane, st);
-}
-
 cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm,
                            const StepParams &p, cudaStream_t st, int *launches, cudaEvent_t *ev,
                            int *kinds) {
@@ -2736,27 +2584,29 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   const int mode = is_l1_variance(f) ? 1 : (is_constrained(f) ? 0 : 2);
   const size_t zplane = (size_t)b.k * M.ldm;  // second FP16 plane of Z
   // 1a. sparse V (every column <= sparse_cap non-zeros last step): gather
+  const bool wide = gather_is_wide(M.m);
   if ((e = mark(9)) != cudaSuccess) return e;
-  if ((e = launch_gather_group(M, b, mode, zplane, st)) != cudaSuccess) return e;
-  nl++;
-  if ((e = mark(5)) != cudaSuccess) return e;
-  if (mode == 0)
-    gather_bv_kernel<0><<<b.k, GATHER_THREADS, 0, st>>>(M.Bc, M.ldm, M.m, M.ldn,
-                                                        b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz,
-                                                        b.max_nnz, b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale,
-                                                        b.ctl);
-  else if (mode == 1)
-    gather_bv_kernel<1><<<b.k, GATHER_THREADS, 0, st>>>(M.Bc, M.ldm, M.m, M.ldn,
-                                                        b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz,
-                                                        b.max_nnz, b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale,
-                                                        b.ctl);
-  else
-    gather_bv_kernel<2><<<b.k, GATHER_THREADS, 0, st>>>(M.Bc, M.ldm, M.m, M.ldn,
-                                                        b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz,
-                                                        b.max_nnz, b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale,
-                                                        b.ctl);
+  if (wide) {
+    // the lists take the dense planes' place (not read on sparse steps)
+    int2 *lists = reinterpret_cast<int2 *>(b.fp16_1 ? (void *)b.V_h : (void *)b.V_hi);
+    gather_list_kernel<<<b.k, GATHER_THREADS, 0, st>>>(M.ldn, b.Vx, b.vmask, b.max_nnz,
+                                                       b.sparse_cap, lists, b.ctl);
+    nl++;
+    if ((e = mark(5)) != cudaSuccess) return e;
+    gather_tile_kernel<<<gather_tiles(M.ldm) * gather_groups(b.k), GATHER_THREADS, 0, st>>>(
+        M.Bc, M.ldm, M.ldn, b.k, lists, b.Z_hi, b.max_nnz, b.sparse_cap, b.ctl);
+    nl++;
+  } else {
+    gather_narrow_kernel<<<b.k, GATHER_THREADS, 0, st>>>(
+        mode, M.Bc, M.ldm, M.m, M.ldn, b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz, b.max_nnz,
+        b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
+    nl++;
+    if (ev) {  // one launch serves both kinds: am24_batch_step_timed names it by the counts
+      if ((e = mark(5)) != cudaSuccess) return e;
+      nl++;
+    }
+  }
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  nl++;
   // 1b. dense V: TF32 hi/lo planes, tensor-core Z = B V (split-K partials) ...
   if ((e = mark(6)) != cudaSuccess) return e;
   if (b.fp16_1)
@@ -2784,18 +2634,9 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   // 2. ... then reduce + sign / normalise
   const int splits1 = b.fp16_1 ? b.splits1p : b.splits1;
   if ((e = mark(1)) != cudaSuccess) return e;
-  if (mode == 0)
-    z_reduce_kernel<0><<<b.k, 256, 0, st>>>(b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
-                                             b.Z_hi, b.Z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
-                                             b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
-  else if (mode == 1)
-    z_reduce_kernel<1><<<b.k, 256, 0, st>>>(b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
-                                             b.Z_hi, b.Z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
-                                             b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
-  else
-    z_reduce_kernel<2><<<b.k, 256, 0, st>>>(b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
-                                             b.Z_hi, b.Z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
-                                             b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
+  z_reduce_kernel<<<b.k, 256, 0, st>>>(mode, b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
+                                       b.Z_hi, b.Z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
+                                       b.Z_b, b.Z_h, zplane, b.z_scale, wide, b.ctl);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   nl++;
   // 3. V = B^T Z
@@ -2998,25 +2839,20 @@ cudaError_t grouped_gemms_setup(int *c) {
 
 cudaError_t grouped_grids(GroupGrids *gr) {
   cudaError_t e;
-  if ((e = kernel_setup(g_gather_group_kernel<0>, (int)GATHER_GROUP_SMEM, false)) ||
-      (e = kernel_setup(g_gather_group_kernel<1>, (int)GATHER_GROUP_SMEM, false)) ||
-      (e = kernel_setup(g_gather_group_kernel<2>, (int)GATHER_GROUP_SMEM, false)))
-    return e;
   int c = 0;
   if ((e = grouped_gemms_setup<GE_PARTIAL>(&c)) || (e = grouped_gemms_setup<GE_RAW>(&c)) ||
       (e = grouped_gemms_setup<GE_PL1>(&c)) || (e = grouped_gemms_setup<GE_PL0>(&c)))
     return e;
   gr->plan_threads = PLAN_THREADS;
   gr->pairs = c;
-  if ((e = persistent_grid(g_z_reduce_kernel<0>, 256, 0, &gr->col)) ||
+  if ((e = persistent_grid(g_z_reduce_kernel, 256, 0, &gr->col)) ||
       (e = persistent_grid(g_hard_select_kernel, HARD_THREADS, 0, &gr->select_hard)) ||
       (e = kernel_setup(g_soft_select_kernel<false>, SOFT_SMEM, false)) ||
       (e = kernel_setup(g_soft_select_kernel<true>, SOFT_SMEM, false)) ||
       (e = persistent_grid(g_soft_select_kernel<false>, SOFT_THREADS, SOFT_SMEM,
                            &gr->select_soft)) ||
-      (e = persistent_grid(g_gather_kernel<0>, GATHER_THREADS, 0, &gr->gather)) ||
-      (e = persistent_grid(g_gather_group_kernel<0>, GATHER_THREADS, (int)GATHER_GROUP_SMEM,
-                           &gr->gather_group)) ||
+      (e = persistent_grid(g_gather_narrow_kernel, GATHER_THREADS, 0, &gr->gather)) ||
+      (e = persistent_grid(g_gather_tile_kernel, GATHER_THREADS, 0, &gr->gather_tile)) ||
       (e = persistent_grid(g_finalize_kernel, 256, 0, &gr->fin)))
     return e;
   return cudaSuccess;
@@ -3026,20 +2862,14 @@ cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &gr, cudaStr
   cudaError_t e;
   group_plan_kernel<<<1, PLAN_THREADS, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
-  // Z = B V: the sparse gathers (by mode), or the dense path
-  g_gather_group_kernel<0><<<gr.gather_group, GATHER_THREADS, GATHER_GROUP_SMEM, st>>>(g);
-  g_gather_group_kernel<1><<<gr.gather_group, GATHER_THREADS, GATHER_GROUP_SMEM, st>>>(g);
-  g_gather_group_kernel<2><<<gr.gather_group, GATHER_THREADS, GATHER_GROUP_SMEM, st>>>(g);
-  g_gather_kernel<0><<<gr.gather, GATHER_THREADS, 0, st>>>(g);
-  g_gather_kernel<1><<<gr.gather, GATHER_THREADS, 0, st>>>(g);
-  g_gather_kernel<2><<<gr.gather, GATHER_THREADS, 0, st>>>(g);
-  for (int mode = 0; mode < 3; mode++)
-    g_densify_kernel<<<DENSIFY_BLOCKS_PER_SM * num_sms(), DENSIFY_THREADS, 0, st>>>(g, mode);
+  // Z = B V: the sparse gathers, or the dense path
+  g_gather_narrow_kernel<<<gr.gather, GATHER_THREADS, 0, st>>>(g);
+  g_gather_list_kernel<<<gr.col, GATHER_THREADS, 0, st>>>(g);
+  g_gather_tile_kernel<<<gr.gather_tile, GATHER_THREADS, 0, st>>>(g);
+  g_densify_kernel<<<DENSIFY_BLOCKS_PER_SM * num_sms(), DENSIFY_THREADS, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
   if ((e = launch_grouped_gemms<GE_PARTIAL>(g, GL_GEMM1_64, st))) return e;
-  g_z_reduce_kernel<0><<<gr.col, 256, 0, st>>>(g);
-  g_z_reduce_kernel<1><<<gr.col, 256, 0, st>>>(g);
-  g_z_reduce_kernel<2><<<gr.col, 256, 0, st>>>(g);
+  g_z_reduce_kernel<<<gr.col, 256, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
   // V = B^T Z with the penalty fused or the raw output marked for the selects
   if ((e = launch_grouped_gemms<GE_RAW>(g, GL_RAW_64, st)) ||

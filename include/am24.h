@@ -416,7 +416,8 @@ am24_status am24_autotune_clear(void);
 /* Kernel kinds reported by am24_batch_step_timed. */
 typedef enum {
   AM24_KERNEL_GEMM_BV = 0,   /* Z = B V, tensor cores, split-K partial tiles */
-  AM24_KERNEL_Z_REDUCE = 1,  /* split-K sum, sign / norm / normalise of Z */
+  AM24_KERNEL_Z_REDUCE = 1,  /* split-K sum, sign / norm / normalise of Z (sparse steps
+                                with more than 1024 samples: the latter alone) */
   AM24_KERNEL_GEMM_BTZ = 2,  /* V = B^T Z, tensor cores (+ penalty epilogue) */
   AM24_KERNEL_SELECT = 3,    /* top-s select or L1-ball level, normalise (constrained) */
   AM24_KERNEL_FINALIZE = 4,  /* per-start objective, change, logs, batch maximum */
@@ -426,7 +427,10 @@ typedef enum {
                                    phase: FP16, or BF16 with AM24_MIXED_BF16=1) */
   AM24_KERNEL_GEMM_BTZ_BF16 = 7, /* the same kind under its earlier name */
   AM24_KERNEL_SUPPORT = 8,   /* support-stability count and phase switch (MIXED) */
-  AM24_KERNEL_GATHER_BV_GROUP = 9, /* the gather for four starts per block (few non-zeros) */
+  AM24_KERNEL_GATHER_BV_GROUP = 9, /* up to 1024 samples: the gather (one launch for both
+                                      kinds) while no column has over 1024 non-zeros;
+                                      more samples: the listing of the non-zeros before
+                                      AM24_KERNEL_GATHER_BV */
   AM24_KERNEL_SKIPPED = 0x100 /* or-ed into a kind: the launch returned at once */
 } am24_kernel_kind;
 /* One AM step like am24_batch_iterate(h, b, it, 1, NULL), with a CUDA event

@@ -191,21 +191,22 @@ cudaError_t reset_mixed(const BatchDev &d, cudaStream_t st) {
 
 }  // namespace am24host
 
+// The batch's words for newly loaded starts.
+static am24_status reset_loaded(am24_handle h, am24_batch b) {
+  const BatchDev &d = b->d;
+  AM24_CUDA(launch_reset_batch(d.k, d.sel_hint, d.val, d.err, d.max_nnz, d.planes_nnz, d.ctl,
+                               h->stream));
+  if (d.mixed) AM24_CUDA(reset_mixed(d, h->stream));
+  return AM24_OK;
+}
+
 // The starting points staged in b's Vraw (all batch_size columns) become the
-// batch's loadings: values and masks, dense-step gate, no select hints, and
-// ValueCoordinateHolder::reset (c++/src/utils/various.h:33-38).
+// batch's loadings: values and masks, and the words of a new load.
 static am24_status load_from_vraw(am24_handle h, am24_batch b) {
   const MatrixDev &M = b->mat->d;
-  const int k = b->d.k;
-  AM24_CUDA(launch_load_columns(b->d.Vraw, M.ldn, M.n, k, b->d.Vx, M.ldn, b->d.vmask, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b->d.max_nnz, 0xFF, sizeof(uint32_t), h->stream));  // dense starts
-  AM24_CUDA(cudaMemsetAsync(b->d.planes_nnz, 0, sizeof(uint32_t), h->stream));  // stale planes
-  AM24_CUDA(cudaMemsetAsync(b->d.sel_hint, 0, sizeof(float) * k, h->stream));      // no hints
-  AM24_CUDA(cudaMemsetAsync(b->d.val, 0, sizeof(float) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b->d.err, 0, sizeof(float) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b->d.ctl, 0, sizeof(uint32_t) * CTL_WORDS, h->stream));
-  if (b->d.mixed) AM24_CUDA(reset_mixed(b->d, h->stream));
-  return AM24_OK;
+  AM24_CUDA(launch_load_columns(b->d.Vraw, M.ldn, M.n, b->d.k, b->d.Vx, M.ldn, b->d.vmask,
+                                h->stream));
+  return reset_loaded(h, b);
 }
 
 namespace am24host {
@@ -783,7 +784,7 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
       (tf32_1 && ((st = A.get(&d.V_hi, kv)) || (st = A.get(&d.V_lo, kv)))) ||
       ((tf32_1 || tf32_2) && (st = ensure_tf32_planes(h, mat))) ||
       (st = A.get(&d.Vraw, kv)) ||
-      (st = A.get(&d.Z_hi, kz)) || (st = A.get(&d.Z_lo, kz)) ||
+      (st = A.get(&d.Z_hi, kz)) || (!d.fp16_2 && (st = A.get(&d.Z_lo, kz))) ||
       (st = A.get(&d.ws, d.ws_len)) ||
       (st = A.get(&d.fz, k)) || (st = A.get(&d.obj_part, (size_t)k * parts)) ||
       (st = A.get(&d.nnz_part, (size_t)k * parts)) || (st = A.get(&d.nnz, k)) ||
@@ -804,12 +805,11 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
     delete b;
     return st;
   }
-  cudaError_t e = cudaMemsetAsync(d.Vx, 0, sizeof(float) * kv, h->stream);
-  if (!e && d.V_hi) e = cudaMemsetAsync(d.V_hi, 0, sizeof(float) * kv, h->stream);
-  if (!e && d.V_lo) e = cudaMemsetAsync(d.V_lo, 0, sizeof(float) * kv, h->stream);
-  if (!e) e = cudaMemsetAsync(d.Vraw, 0, sizeof(float) * kv, h->stream);
-  if (!e) e = cudaMemsetAsync(d.Z_hi, 0, sizeof(float) * kz, h->stream);
-  if (!e) e = cudaMemsetAsync(d.Z_lo, 0, sizeof(float) * kz, h->stream);
+  // What a step or a read could see before it is written starts zeroed.  The
+  // planes need no initial contents: Vx is defined where vmask is set, every
+  // operand plane is written whole before its product, and nothing past n (m)
+  // entries of a column is used.
+  cudaError_t e = cudaSuccess;
   if (!e) e = cudaMemsetAsync(d.val, 0, sizeof(float) * k, h->stream);
   if (!e) e = cudaMemsetAsync(d.err, 0, sizeof(float) * k, h->stream);
   if (!e) e = cudaMemsetAsync(d.fz, 0, sizeof(float) * k, h->stream);
@@ -820,17 +820,8 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
   if (!e) e = cudaMemsetAsync(d.planes_nnz, 0, sizeof(uint32_t), h->stream);
   if (!e) e = cudaMemsetAsync(d.sel_hint, 0, sizeof(float) * k, h->stream);
   if (!e) e = cudaMemsetAsync(d.ctl, 0, sizeof(uint32_t) * CTL_WORDS, h->stream);
-  if (!e && d.cmask)
-    e = cudaMemsetAsync(d.cmask, 0, sizeof(uint32_t) * k * (M.ldn / 32), h->stream);
-  if (!e && d.Z_b) e = cudaMemsetAsync(d.Z_b, 0, sizeof(uint16_t) * kz, h->stream);
-  if (!e && d.Z_h) e = cudaMemsetAsync(d.Z_h, 0, sizeof(uint16_t) * zh_planes * kz, h->stream);
-  if (!e && d.z_scale) e = cudaMemsetAsync(d.z_scale, 0, sizeof(float) * k, h->stream);
-  if (!e && d.V_h) e = cudaMemsetAsync(d.V_h, 0, sizeof(uint16_t) * 2 * kv, h->stream);
-  if (!e && d.v_scale) e = cudaMemsetAsync(d.v_scale, 0, sizeof(float) * k, h->stream);
   d.row_scale = M.row_scale;
   d.bt_row_scale = M.bt_row_scale;
-  if (!e && d.mixed)
-    e = cudaMemsetAsync(d.vmask_prev, 0, sizeof(uint32_t) * k * (M.ldn / 32), h->stream);
   if (!e && d.mixed) e = reset_mixed(d, h->stream);
   if (!e) e = cudaMemsetAsync(d.iters, 0xFF, sizeof(int) * d.log_capacity, h->stream);
   if (!e) e = cudaMemsetAsync(d.cards, 0xFF, sizeof(int) * d.log_capacity, h->stream);
@@ -1146,9 +1137,10 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
         gidx[j] = shift + j;
         slots[j] = j;
       }
-      // the batch's starts, staged in Vraw by one copy (or generated there)
-      if (s.start_mode == AM24_START_DEVICE_UNIFORM) {
-        AM24_CUDA(launch_uniform_starts(d.Vraw, M.ldn, (int)n, bs, shift, h->stream));
+      // the batch's starts, staged in Vraw by one copy (or generated in place)
+      const bool device = s.start_mode == AM24_START_DEVICE_UNIFORM;
+      if (device) {
+        AM24_CUDA(launch_uniform_starts(d.Vx, M.ldn, (int)n, bs, shift, d.vmask, h->stream));
       } else if (batch == 0 && pre) {  // already on the device
         AM24_CUDA(cudaStreamWaitEvent(h->stream, pre_done, 0));
         AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, pre, sizeof(float) * n,
@@ -1162,8 +1154,7 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
         AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, src, sizeof(float) * n,
                                     sizeof(float) * n, bs, cudaMemcpyHostToDevice, h->stream));
       }
-      AM24_TRY(load_from_vraw(h, b));
-      if (d.mixed) AM24_CUDA(reset_mixed(d, h->stream));
+      AM24_TRY(device ? reset_loaded(h, b) : load_from_vraw(h, b));
       AM24_CUDA(cudaEventRecord(e0, h->stream));
       BatchRun run;
       AM24_TRY(run_batch_steps(h, b, s, (int)shift, &run));

@@ -154,7 +154,7 @@ uint64_t group_problem_bytes(int m, int n, int k, int formulation, bool mixed) {
   const uint64_t parts = (uint64_t)((n + BM - 1) / BM) * 4;
   const uint64_t zh = is_l1_variance(formulation) ? 1 : 2;
   uint64_t b = kv * 4 * 2 + kv * 2 * 2 + words * 4 * (is_constrained(formulation) ? 2 : 1) +
-               kz * (4 + 4 + 2 * zh) +
+               kz * (4 + 2 * zh) +
                (uint64_t)ws_floats(splits, (int)m_tiles1, (int)n_tiles, bn) * 4 +
                (uint64_t)k * (4 * 8 + parts * 8 + (mixed ? 16 : 0)) + 4096;
   return b;
@@ -326,7 +326,7 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
   if ((st = A->get(&P.Vx, kv)) || (st = A->get(&P.vmask, words)) ||
       (st = A->get(&P.Vraw, kv)) || (st = A->get(&P.sel_hint, k)) || (st = A->get(&P.nnz, k)) ||
       (is_constrained(f) && (st = A->get(&P.cmask, words))) ||
-      (st = A->get(&P.Z_hi, kz)) || (st = A->get(&P.Z_lo, kz)) ||
+      (st = A->get(&P.Z_hi, kz)) ||
       (st = A->get(&P.Z_h, zh_planes * kz)) || (st = A->get(&P.z_scale, k)) ||
       (st = A->get(&P.V_h, 2 * kv)) ||
       (st = A->get(&P.v_scale, k)) ||
@@ -339,21 +339,11 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
                  (st = A->get(&P.mask_hash, k)))))
     return st;
   const cudaStream_t hs = h->stream;
-  // every buffer starts zeroed, as a batch's do: a slot's memory may come back
-  // from the pool holding an earlier problem's state
-  AM24_CUDA(cudaMemsetAsync(P.Vx, 0, sizeof(float) * kv, hs));
-  AM24_CUDA(cudaMemsetAsync(P.Vraw, 0, sizeof(float) * kv, hs));
-  AM24_CUDA(cudaMemsetAsync(P.vmask, 0, sizeof(uint32_t) * words, hs));
-  AM24_CUDA(cudaMemsetAsync(P.Z_hi, 0, sizeof(float) * kz, hs));
-  AM24_CUDA(cudaMemsetAsync(P.Z_lo, 0, sizeof(float) * kz, hs));
-  AM24_CUDA(cudaMemsetAsync(P.z_scale, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.v_scale, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.obj_part, 0, sizeof(float) * k * P.parts, hs));
+  // a slot's memory may come back from the pool holding an earlier problem's
+  // state: what a step or a read could see before it is written starts zeroed
+  // (the planes need no contents, as a batch's do not)
   AM24_CUDA(cudaMemsetAsync(P.nnz_part, 0, sizeof(float) * k * P.parts, hs));
   AM24_CUDA(cudaMemsetAsync(P.max_err, 0, sizeof(float), hs));
-  AM24_CUDA(cudaMemsetAsync(P.Z_h, 0, sizeof(uint16_t) * zh_planes * kz, hs));
-  AM24_CUDA(cudaMemsetAsync(P.V_h, 0, sizeof(uint16_t) * 2 * kv, hs));
-  if (P.cmask) AM24_CUDA(cudaMemsetAsync(P.cmask, 0, sizeof(uint32_t) * words, hs));
   AM24_CUDA(cudaMemsetAsync(P.sel_hint, 0, sizeof(float) * k, hs));
   AM24_CUDA(cudaMemsetAsync(P.val, 0, sizeof(float) * k, hs));
   AM24_CUDA(cudaMemsetAsync(P.err, 0, sizeof(float) * k, hs));
@@ -373,7 +363,7 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
   AM24_CUDA(cudaMemcpyAsync(P.ctl, ctl, sizeof ctl, cudaMemcpyHostToDevice, hs));
   // starting points staged in Vraw, then split into values and masks
   if (s.start_mode == AM24_START_DEVICE_UNIFORM) {
-    AM24_CUDA(launch_uniform_starts(P.Vraw, M.ldn, M.n, k, 0, hs));
+    AM24_CUDA(launch_uniform_starts(P.Vx, M.ldn, M.n, k, 0, P.vmask, hs));
   } else {
     std::vector<float> staging;
     const float *src = start_points;
@@ -386,8 +376,8 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
     AM24_CUDA(cudaMemcpy2DAsync(P.Vraw, sizeof(float) * M.ldn, src, sizeof(float) * M.n,
                                 sizeof(float) * M.n, k, cudaMemcpyHostToDevice, hs));
     AM24_CUDA(cudaStreamSynchronize(hs));  // `staging` goes out of scope
+    AM24_CUDA(launch_load_columns(P.Vraw, M.ldn, M.n, k, P.Vx, M.ldn, P.vmask, hs));
   }
-  AM24_CUDA(launch_load_columns(P.Vraw, M.ldn, M.n, k, P.Vx, M.ldn, P.vmask, hs));
   // tensor maps
   GMaps maps;
   std::memset(&maps, 0, sizeof maps);

@@ -168,7 +168,7 @@ __device__ __forceinline__ void for_items(const GroupDev &g, int l, Fn fn, int c
 }
 
 __device__ __forceinline__ ZOut z_out(const GProblem &P, int j) {
-  return z_out(j, P.ldm, P.Z_hi, P.Z_lo, P.Z_b, P.Z_h, P.zplane, P.z_scale, P.fz);
+  return z_out(j, P.ldm, P.Z_hi, nullptr, P.Z_b, P.Z_h, P.zplane, P.z_scale, P.fz);
 }
 
 __global__ void __launch_bounds__(GATHER_THREADS) g_gather_narrow_kernel(GroupDev g) {

@@ -221,7 +221,7 @@ struct GProblem {
   int m_tiles2, n_tiles2;          // V = B^T Z
   int parts;                       // m_tiles2 * 4 penalty partials per start
   // state
-  float *Vx, *Vraw, *sel_hint, *Z_hi, *Z_lo, *fz, *obj_part, *nnz_part, *val, *err, *max_err;
+  float *Vx, *Vraw, *sel_hint, *Z_hi, *fz, *obj_part, *nnz_part, *val, *err, *max_err;
   float *z_scale, *v_scale, *ws;
   uint32_t *vmask, *cmask, *nnz, *ctl, *stable, *phase;
   uint64_t *mask_hash;  // MIXED: per start, a hash of the last step's support
@@ -374,7 +374,9 @@ cudaError_t launch_load_columns(const float *src, int ld_src, int rows, int cols
 // Columns [0, cols) of V (leading dimension ld): device uniform starts for the
 // global start indices first, first + 1, ... (AM24_START_DEVICE_UNIFORM).
 cudaError_t launch_uniform_starts(float *V, int ld, int rows, int cols, uint32_t first,
-                                  cudaStream_t st);
+                                  uint32_t *mask, cudaStream_t st);
+cudaError_t launch_reset_batch(int k, float *sel_hint, float *val, float *err, uint32_t *max_nnz,
+                               uint32_t *planes_nnz, uint32_t *ctl, cudaStream_t st);
 cudaError_t launch_masked_copy(const float *Vx, const uint32_t *mask, int ld, int rows, int cols,
                                float *dst, int ld_dst, cudaStream_t st);
 // ev (optional, >= 17 events): ev[i] is recorded before launch i and
@@ -401,7 +403,7 @@ cudaError_t launch_explained_variance(const MatrixDev &M, const float *x, double
                                       double *out, cudaStream_t st);
 constexpr int EV_CHUNK = 512;  // features per partial sum of the explained variance
 inline size_t ev_partial_len(const MatrixDev &M) {
-  return (size_t)((M.n + EV_CHUNK - 1) / EV_CHUNK) * M.m;
+  return ((size_t)(M.n + EV_CHUNK - 1) / EV_CHUNK + 1) * M.m;  // chunks, then their sum
 }
 int pick_bn(int k);
 size_t ws_floats(int splits, int m_tiles, int n_tiles, int bn);

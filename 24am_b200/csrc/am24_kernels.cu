@@ -430,12 +430,20 @@ __global__ void load_columns_kernel(const float *__restrict__ src, int ld_src, i
   }
 }
 
+// dst = the column's values where its mask is set, zero elsewhere; blockIdx.y
+// walks pieces of COPY_ROWS rows (a single column is most calls' whole work: one
+// block for it took 45 us at 50000 rows).
+constexpr int COPY_ROWS = 2048;
 __global__ void masked_copy_kernel(const float *__restrict__ Vx, const uint32_t *__restrict__ mask,
                                    int ld, int rows, float *__restrict__ dst, int ld_dst) {
   const size_t c = blockIdx.x;
-  for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-    const bool on = (mask[c * (ld >> 5) + (r >> 5)] >> (r & 31)) & 1u;
-    dst[c * ld_dst + r] = on ? Vx[c * ld + r] : 0.f;
+  for (int r0 = blockIdx.y * COPY_ROWS; r0 < rows; r0 += gridDim.y * COPY_ROWS) {
+    const int r1 = min(rows, r0 + COPY_ROWS);
+#pragma unroll 8
+    for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
+      const bool on = (mask[c * (ld >> 5) + (r >> 5)] >> (r & 31)) & 1u;
+      dst[c * ld_dst + r] = on ? Vx[c * ld + r] : 0.f;
+    }
   }
 }
 
@@ -530,7 +538,8 @@ __global__ void __launch_bounds__(DENSIFY_THREADS, DENSIFY_BLOCKS_PER_SM) densif
 // 1: L1 variance               -> z = sgn(y), fz = ||y||_1 (:85-86, :156)
 // 2: L2 variance, penalized    -> z = y * (1/||y||_2)     (:163-164)
 struct ZOut {
-  float *hi, *lo;     // one start's FP32 planes (hi + lo = z), ldm each
+  float *hi, *lo;     // one start's FP32 planes, ldm each: hi + lo = z when lo is
+                      // wanted (the TF32 operands); else hi holds y between passes
   uint16_t *b;        // its BF16 z (null: not wanted)
   uint16_t *h;        // its FP16 z (null: not wanted); second plane at h + plane
   size_t plane;
@@ -539,30 +548,70 @@ struct ZOut {
 __device__ __forceinline__ ZOut z_out(int j, int ldm, float *Z_hi, float *Z_lo, uint16_t *Zb,
                                       uint16_t *Zh, size_t zplane, float *zscale, float *fz) {
   const size_t o = (size_t)j * ldm;
-  return ZOut{Z_hi + o, Z_lo + o, Zb ? Zb + o : nullptr, Zh ? Zh + o : nullptr, zplane,
-              zscale ? zscale + j : nullptr, fz + j};
+  return ZOut{Z_hi + o, Z_lo ? Z_lo + o : nullptr, Zb ? Zb + o : nullptr, Zh ? Zh + o : nullptr,
+              zplane, zscale ? zscale + j : nullptr, fz + j};
 }
-// Sample i's y before the norm is known: its share of the norm into acc, and
-// what can be stored already.  In mode 2 the planes are stored only when `keep`
-// (the second pass reads y back from them).
-__device__ __forceinline__ void z_emit(const ZOut &z, int mode, int i, float y, bool keep,
-                                       double &acc) {
-  if (mode == 1) {
-    acc += (double)fabsf(y);
-    z.hi[i] = sgnf(y);
-    z.lo[i] = 0.f;
-    if (z.b) z.b[i] = bf16_sign(y);
-    if (z.h) z.h[i] = f16_sign(y);
+// C consecutive values of T at p (aligned to them) in one store.
+template <int C, class T>
+__device__ __forceinline__ void store_run(T *p, const T (&v)[C]) {
+  if (C == 1) {
+    *p = v[0];
+  } else if (sizeof(T) == 4) {
+    *reinterpret_cast<uint4 *>(p) = *reinterpret_cast<const uint4 *>(v);
   } else {
-    acc += (double)y * (double)y;
-    if (mode == 0 || keep) split_store(y, z.hi + i, z.lo + i);
-    if (mode == 0 && z.b) z.b[i] = bf16_bits(y);
+    *reinterpret_cast<uint2 *>(p) = *reinterpret_cast<const uint2 *>(v);
   }
+}
+template <int C>
+__device__ __forceinline__ void z_store_split(const ZOut &z, int i, const float (&y)[C]) {
+  alignas(16) float hi[C], lo[C];
+#pragma unroll
+  for (int c = 0; c < C; c++) split_store(y[c], hi + c, lo + c);
+  store_run(z.hi + i, hi);
+  store_run(z.lo + i, lo);
 }
 __device__ __forceinline__ bool z_second_pass(const ZOut &z, int mode) {
   return mode == 2 || (mode == 0 && z.h);
 }
-// Second pass over sample i: mode 2 normalises; both write the FP16 planes of
+// Samples i .. i + C - 1 (C = 1 or 4; beyond m they are zeros of the padding)
+// before the norm is known: their share of it into acc, and what can be stored
+// already.  KEEP: y is stored for a second pass, which reads it back.
+template <int C, bool KEEP>
+__device__ __forceinline__ void z_emit(const ZOut &z, int mode, int i, const float (&y)[C],
+                                       double &acc) {
+  if (mode == 1) {
+    alignas(16) uint16_t b[C], h[C];
+    alignas(16) float sg[C], zero[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      acc += (double)fabsf(y[c]);
+      sg[c] = sgnf(y[c]);
+      zero[c] = 0.f;
+      b[c] = bf16_sign(y[c]);
+      h[c] = f16_sign(y[c]);
+    }
+    if (z.lo) {
+      store_run(z.hi + i, sg);
+      store_run(z.lo + i, zero);
+    }
+    if (z.b) store_run(z.b + i, b);
+    if (z.h) store_run(z.h + i, h);
+  } else {
+    alignas(16) uint16_t b[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) {
+      acc += (double)y[c] * (double)y[c];
+      b[c] = bf16_bits(y[c]);
+    }
+    if (z.lo) {
+      if (mode == 0 || KEEP) z_store_split(z, i, y);
+    } else if (KEEP && C == 1 && z_second_pass(z, mode)) {
+      z.hi[i] = y[0];
+    }
+    if (mode == 0 && z.b) store_run(z.b + i, b);
+  }
+}
+// Second pass over them: mode 2 normalises; both write the FP16 planes of
 // z * 2^s, s from a bound on |z| (||y||_2, or 1 for the normalised z).
 struct ZScale {
   float inv, sc;
@@ -575,13 +624,25 @@ __device__ __forceinline__ ZScale z_scales(int mode, double tot) {
   r.sc = pow2f(r.s);
   return r;
 }
-__device__ __forceinline__ void z_emit2(const ZOut &z, int mode, const ZScale &c, int i, float y) {
-  const float v = mode == 2 ? y * c.inv : y;
-  if (mode == 2) {
-    split_store(v, z.hi + i, z.lo + i);
-    if (z.b) z.b[i] = bf16_bits(v);
+template <int C>
+__device__ __forceinline__ void z_emit2(const ZOut &z, int mode, const ZScale &c, int i,
+                                        const float (&y)[C]) {
+  float v[C];
+  alignas(16) uint16_t b[C], h0[C], h1[C];
+#pragma unroll
+  for (int q = 0; q < C; q++) {
+    v[q] = mode == 2 ? y[q] * c.inv : y[q];
+    b[q] = bf16_bits(v[q]);
+    fp16_split(v[q] * c.sc, h0 + q, h1 + q);
   }
-  if (z.h) fp16_split(v * c.sc, z.h + i, z.h + z.plane + i);
+  if (mode == 2) {
+    if (z.lo) z_store_split(z, i, v);
+    if (z.b) store_run(z.b + i, b);
+  }
+  if (z.h) {
+    store_run(z.h + i, h0);
+    store_run(z.h + z.plane + i, h1);
+  }
 }
 __device__ __forceinline__ void z_close(const ZOut &z, int mode, double tot) {  // one thread
   if (z_second_pass(z, mode) && z.h) *z.scale = pow2f(-z_scales(mode, tot).s);
@@ -603,37 +664,39 @@ __device__ __forceinline__ void z_reduce_body(int mode, const float *__restrict_
       const size_t u = ((size_t)s * m_tiles + mt) * n_tiles + nt;
       y += ws[u * unit_stride + (size_t)c * BM + r];
     }
-    z_emit(z, mode, i, y, true, acc);
+    z_emit<1, true>(z, mode, i, {y}, acc);
   }
   const double tot = block_sum(acc, red);
   if (z_second_pass(z, mode)) {
     const ZScale sc = z_scales(mode, tot);
-    for (int i = threadIdx.x; i < m; i += blockDim.x)
-      z_emit2(z, mode, sc, i, z.hi[i] + z.lo[i]);  // exact: this thread wrote both planes
+    for (int i = threadIdx.x; i < m; i += blockDim.x)  // exact: this thread wrote the planes
+      z_emit2<1>(z, mode, sc, i, {z.lo ? z.hi[i] + z.lo[i] : z.hi[i]});
   }
   if (threadIdx.x == 0) z_close(z, mode, tot);
 }
 
 // Sparse steps of matrices with more than GATHER_NARROW samples: y from the
-// plane gather_tile_body left it in (z.hi).  256 threads, 4 consecutive samples
-// each, 2048 samples per round.
+// plane gather_tile_body left it in (z.hi, zeros in its padding).  256 threads,
+// 4 consecutive samples each (16- and 8-byte stores: 1024 starts of 2000 samples
+// in 7 us, 19 with a store per sample).
 __device__ __forceinline__ void z_finish_body(int mode, int m, const ZOut &z) {
   __shared__ double red[32];
   double acc = 0.0;
   for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x) {
     const float4 y = *reinterpret_cast<const float4 *>(z.hi + i);
-    const float e[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-      if (i + c < m) z_emit(z, mode, i + c, e[c], true, acc);
+    z_emit<4, true>(z, mode, i, {y.x, y.y, y.z, y.w}, acc);
   }
   const double tot = block_sum(acc, red);
   if (z_second_pass(z, mode)) {
     const ZScale sc = z_scales(mode, tot);
-    for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x)
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-        if (i + c < m) z_emit2(z, mode, sc, i + c, z.hi[i + c] + z.lo[i + c]);
+    for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x) {
+      float4 y = *reinterpret_cast<const float4 *>(z.hi + i);
+      if (z.lo) {
+        const float4 l = *reinterpret_cast<const float4 *>(z.lo + i);
+        y = make_float4(y.x + l.x, y.y + l.y, y.z + l.z, y.w + l.w);
+      }
+      z_emit2<4>(z, mode, sc, i, {y.x, y.y, y.z, y.w});
+    }
   }
   if (threadIdx.x == 0) z_close(z, mode, tot);
 }
@@ -824,16 +887,9 @@ __device__ __forceinline__ void gather_narrow_body(int mode, const float *__rest
   }
   const float e[4] = {y.x, y.y, y.z, y.w};
   double acc = 0.0;
-#pragma unroll
-  for (int c = 0; c < 4; c++)
-    if (4 * i4 + c < m) z_emit(z, mode, 4 * i4 + c, e[c], false, acc);
+  if (on) z_emit<4, false>(z, mode, 4 * i4, e, acc);
   const double tot = block_sum(acc, red);
-  if (z_second_pass(z, mode)) {
-    const ZScale sc = z_scales(mode, tot);
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-      if (4 * i4 + c < m) z_emit2(z, mode, sc, 4 * i4 + c, e[c]);
-  }
+  if (on && z_second_pass(z, mode)) z_emit2<4>(z, mode, z_scales(mode, tot), 4 * i4, e);
   if (threadIdx.x == 0) z_close(z, mode, tot);
 }
 __global__ void __launch_bounds__(GATHER_THREADS) gather_narrow_kernel(
@@ -1010,8 +1066,7 @@ __device__ SelResult block_select_src(Src colg, int n, uint32_t rank, uint32_t *
 
 // x_i = f(v_i) for a column in global memory: the non-zero x_i are stored
 // (only they are defined; the bitmask says which) and the column's non-zero
-// bitmask is written.  Entries up to the next multiple of 32 are read; they lie
-// in the column's zero padding.
+// bitmask is written.
 template <class Fn>
 __device__ __forceinline__ void write_column_global(const float *__restrict__ colg, int n,
                                                     float *vx, uint32_t *mask, Fn fn) {
@@ -1019,7 +1074,7 @@ __device__ __forceinline__ void write_column_global(const float *__restrict__ co
   const int n32 = (n + 31) & ~31;
   for (int base = threadIdx.x & ~31; base < n32; base += blockDim.x) {
     const int i = base + lane;
-    const float x = fn(colg[i]);
+    const float x = i < n ? fn(colg[i]) : 0.f;
     if (x != 0.f) vx[i] = x;
     const unsigned nz = __ballot_sync(FULL, x != 0.f);
     if (lane == 0) mask[base >> 5] = nz;
@@ -1222,8 +1277,8 @@ constexpr int HARD_CAND = 2048;  // hinted (key, index) candidates resolved in s
 // flight per thread): the entries with |v| key >= bound (>= 1) go to cand as
 // (key << 32 | ~index), the first `cap` of them in any order; returns how many
 // there are (it may exceed cap) and, BELOW, leaves in counter[1] the largest
-// key below the bound (0 if none).  Entries past n are not taken (the padding
-// read with the last 16 bytes is zero).  The bound leaves a few hundred entries
+// key below the bound (0 if none).  Entries past n (the padding read with the
+// last 16 bytes) are not taken.  The bound leaves a few hundred entries
 // of a column, so a quad of them is tested by its largest key and the taken
 // ones placed by single shared-memory atomics.
 template <bool BELOW>
@@ -1248,12 +1303,12 @@ __device__ uint32_t gather_pairs_above(const float *__restrict__ colg, int n, ui
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const uint32_t k[4] = {abs_key(v[u].x), abs_key(v[u].y), abs_key(v[u].z), abs_key(v[u].w)};
+      const int e0 = 4 * (base + u * (int)blockDim.x);
       if (BELOW) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) below = max(below, k[q] < bound ? k[q] : 0u);
+        for (int q = 0; q < 4; q++) below = max(below, k[q] < bound && e0 + q < n ? k[q] : 0u);
       }
       if (max(max(k[0], k[1]), max(k[2], k[3])) < bound) continue;
-      const int e0 = 4 * (base + u * (int)blockDim.x);
 #pragma unroll
       for (int q = 0; q < 4; q++)
         if (k[q] >= bound && e0 + q < n) {
@@ -2169,42 +2224,85 @@ __device__ void finalize_start(const FinalizeArgs &a, int j, int lane) {
 }
 
 // x = v / ||v|| (c++/src/gpower/sparse_PCA_solver.h:236-237).
-__global__ void finalize_x_kernel(const float *__restrict__ v, int n, float *__restrict__ x) {
+__global__ void __launch_bounds__(1024) finalize_x_kernel(const float *__restrict__ v, int n,
+                                                          float *__restrict__ x) {
   __shared__ double red[32];
+  const int n4 = n >> 2;
+  const float4 *v4 = reinterpret_cast<const float4 *>(v);
+  float4 *x4 = reinterpret_cast<float4 *>(x);
   double ss = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) ss += (double)v[i] * (double)v[i];
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+    const float4 a = v4[i];
+    ss += (double)a.x * a.x + (double)a.y * a.y + (double)a.z * a.z + (double)a.w * a.w;
+  }
+  const int tail = 4 * n4 + threadIdx.x;
+  if (tail < n) ss += (double)v[tail] * (double)v[tail];
   ss = block_sum(ss, red);
   const float inv = 1.0f / (float)sqrt(ss);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) x[i] = v[i] * inv;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < n4; i += blockDim.x) {
+    const float4 a = v4[i];
+    x4[i] = make_float4(a.x * inv, a.y * inv, a.z * inv, a.w * inv);
+  }
+  if (tail < n) x[tail] = v[tail] * inv;
 }
 
 // Partial sums of y_i = sum_c B[i, c] x_c in FP64 over chunks of EV_CHUNK
 // features: partial[chunk * m + i], threads over samples (coalesced reads of
-// B's columns), features with x_c = 0 skipped, a fixed order per chunk.
+// B's columns), features with x_c = 0 skipped, a fixed order per chunk.  The
+// block lists the chunk's non-zeros first, so that their columns' loads do not
+// wait for a test of every feature (2000 x 50000, 16 non-zeros: 3 us, 62 with
+// the test).
 __global__ void __launch_bounds__(256) ev_partial_kernel(const float *__restrict__ Bc, int ldm,
                                                          int m, int n, const float *__restrict__ x,
                                                          double *__restrict__ partial) {
+  __shared__ int list[EV_CHUNK];
+  __shared__ float val[EV_CHUNK];
+  __shared__ int wsum[EV_CHUNK / 32];
+  const int lane = threadIdx.x & 31;
+  const int c0 = blockIdx.y * EV_CHUNK, c1 = min(n, c0 + EV_CHUNK);
+  constexpr int PER = EV_CHUNK / 256;
+  float xc[PER];
+  uint32_t bits[PER];
+#pragma unroll
+  for (int r = 0; r < PER; r++) {
+    const int c = c0 + r * 256 + threadIdx.x;
+    xc[r] = c < c1 ? x[c] : 0.f;
+    bits[r] = __ballot_sync(FULL, xc[r] != 0.f);
+    if (lane == 0) wsum[r * 8 + (threadIdx.x >> 5)] = __popc(bits[r]);
+  }
+  __syncthreads();
+  int total = 0, before[PER];
+#pragma unroll
+  for (int q = 0; q < EV_CHUNK / 32; q++) {
+#pragma unroll
+    for (int r = 0; r < PER; r++)
+      if (q == r * 8 + (int)(threadIdx.x >> 5)) before[r] = total;
+    total += wsum[q];
+  }
+#pragma unroll
+  for (int r = 0; r < PER; r++)
+    if (xc[r] != 0.f) {
+      const int at = before[r] + __popc(bits[r] & ((1u << lane) - 1u));
+      list[at] = c0 + r * 256 + threadIdx.x;
+      val[at] = xc[r];
+    }
+  __syncthreads();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
-  const int c0 = blockIdx.y * EV_CHUNK, c1 = min(n, c0 + EV_CHUNK);
   double acc = 0.0;
-  for (int c = c0; c < c1; c++) {
-    const float xc = x[c];
-    if (xc != 0.f) acc += (double)Bc[(size_t)c * ldm + i] * (double)xc;
-  }
+#pragma unroll 8
+  for (int q = 0; q < total; q++) acc += (double)Bc[(size_t)list[q] * ldm + i] * (double)val[q];
   partial[(size_t)blockIdx.y * m + i] = acc;
 }
 
-// ||y||^2 with y_i the sum of its chunks' partials (in chunk order).
-__global__ void ev_sum_kernel(const double *__restrict__ partial, int chunks, int m,
-                              double *__restrict__ out) {
+// ||y||^2 (one block).
+__global__ void __launch_bounds__(1024) ev_norm_kernel(const double *__restrict__ y, int m,
+                                                       double *__restrict__ out) {
   __shared__ double red[32];
   double acc = 0.0;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    double y = 0.0;
-    for (int c = 0; c < chunks; c++) y += partial[(size_t)c * m + i];
-    acc += y * y;
-  }
+  for (int i = threadIdx.x; i < m; i += blockDim.x) acc += y[i] * y[i];
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) *out = acc;
 }
@@ -2241,6 +2339,7 @@ __global__ void rowsum_kernel(const double *__restrict__ partial, int chunks, in
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   double acc = 0.0;
+#pragma unroll 8
   for (int c = 0; c < chunks; c++) acc += partial[(size_t)c * m + i];
   y[i] = acc;
 }
@@ -2455,36 +2554,96 @@ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   return x ^ (x >> 31);
 }
 
-// Column c: U[-1, 1) from the top 24 bits of splitmix64((first + c) << 32 | i)
-// for row i < rows, then scaled to unit 2-norm.
-__global__ void __launch_bounds__(256) uniform_starts_kernel(float *__restrict__ V, int ld,
-                                                             int rows, uint32_t first) {
+// Column c of the loadings: U[-1, 1) from the top 24 bits of splitmix64((first +
+// c) << 32 | i) for row i < rows, scaled to unit 2-norm, zero up to ld, and its
+// non-zero mask.  u = t 2^-23 with t a 24-bit integer, so the squares add up
+// exactly in integers.  Persistent at two blocks per SM: the second pass, which
+// scales, finds the column in L2.  Bound by the mixer's integer instructions:
+// 1024 columns of 50000 take 108 us (310 with 256-thread blocks and a pass of
+// load_columns_kernel for the values and masks).
+constexpr int STARTS_THREADS = 1024;
+__global__ void __launch_bounds__(STARTS_THREADS, 2) uniform_starts_kernel(
+    float *__restrict__ V, int ld, int rows, int cols, uint32_t first,
+    uint32_t *__restrict__ mask) {
   __shared__ double red[32];
-  const size_t c = blockIdx.x;
-  float *v = V + c * ld;
-  const uint64_t key = (uint64_t)(first + (uint32_t)c) << 32;
-  double ss = 0.0;
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) {
-    const float u = (float)(splitmix64(key | (uint32_t)i) >> 40) * (2.0f / 16777216.0f) - 1.0f;
-    v[i] = u;
-    ss += (double)u * (double)u;
+  for (int c = blockIdx.x; c < cols; c += gridDim.x) {
+    float *v = V + (size_t)c * ld;
+    const uint64_t key = (uint64_t)(first + (uint32_t)c) << 32;
+    double ss = 0.0;
+    uint64_t part = 0;
+    int run = 0;  // squares in `part`: each at most 2^46
+    float4 *v4 = reinterpret_cast<float4 *>(v);
+    for (int q = threadIdx.x; q < (ld >> 2); q += STARTS_THREADS) {
+      float u[4];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const int i = 4 * q + e;
+        int t = (int)(uint32_t)(splitmix64(key | (uint32_t)i) >> 40) - (1 << 23);
+        if (i >= rows) t = 0;
+        u[e] = (float)t * (1.0f / 8388608.0f);
+        part += (uint64_t)((int64_t)t * t);
+      }
+      v4[q] = make_float4(u[0], u[1], u[2], u[3]);
+      if ((run += 4) == 1 << 17) {
+        ss += (double)part;
+        part = 0;
+        run = 0;
+      }
+    }
+    ss = block_sum((ss + (double)part) * (1.0 / 70368744177664.0), red);
+    const float inv = (float)(1.0 / sqrt(ss));
+    for (int q = threadIdx.x; q < (ld >> 2); q += STARTS_THREADS) {
+      float4 x = v4[q];
+      x = make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv);
+      v4[q] = x;
+      uint32_t nz = (x.x != 0.f) | (x.y != 0.f) << 1 | (x.z != 0.f) << 2 | (x.w != 0.f) << 3;
+      // eight lanes hold a word (ld is a multiple of 32, so they are all here)
+      nz <<= 4 * (threadIdx.x & 7);
+      const uint32_t eight = 0xFFu << (threadIdx.x & 24);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) nz |= __shfl_xor_sync(eight, nz, o);
+      if ((threadIdx.x & 7) == 0) mask[(size_t)c * (ld >> 5) + (q >> 3)] = nz;
+    }
   }
-  ss = block_sum(ss, red);
-  const float inv = (float)(1.0 / sqrt(ss));
-  for (int i = threadIdx.x; i < rows; i += blockDim.x) v[i] *= inv;
 }
 
 cudaError_t launch_uniform_starts(float *V, int ld, int rows, int cols, uint32_t first,
-                                  cudaStream_t st) {
+                                  uint32_t *mask, cudaStream_t st) {
   if (cols <= 0) return cudaSuccess;
-  uniform_starts_kernel<<<cols, 256, 0, st>>>(V, ld, rows, first);
+  uniform_starts_kernel<<<std::min(cols, 2 * num_sms()), STARTS_THREADS, 0, st>>>(
+      V, ld, rows, cols, first, mask);
+  return cudaGetLastError();
+}
+
+// ValueCoordinateHolder::reset (c++/src/utils/various.h:33-38) and a batch's
+// other words for newly loaded starts: no hints, a dense first step, no planes,
+// the run-ahead words cleared.
+__global__ void reset_batch_kernel(int k, float *sel_hint, float *val, float *err,
+                                   uint32_t *max_nnz, uint32_t *planes_nnz, uint32_t *ctl) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < k) {
+    sel_hint[j] = 0.f;
+    val[j] = 0.f;
+    err[j] = 0.f;
+  }
+  if (j < CTL_WORDS) ctl[j] = 0u;
+  if (j == 0) {
+    *max_nnz = 0xFFFFFFFFu;
+    if (planes_nnz) *planes_nnz = 0u;
+  }
+}
+cudaError_t launch_reset_batch(int k, float *sel_hint, float *val, float *err, uint32_t *max_nnz,
+                               uint32_t *planes_nnz, uint32_t *ctl, cudaStream_t st) {
+  reset_batch_kernel<<<(std::max(k, (int)CTL_WORDS) + 255) / 256, 256, 0, st>>>(
+      k, sel_hint, val, err, max_nnz, planes_nnz, ctl);
   return cudaGetLastError();
 }
 
 cudaError_t launch_masked_copy(const float *Vx, const uint32_t *mask, int ld, int rows, int cols,
                                float *dst, int ld_dst, cudaStream_t st) {
   if (cols <= 0) return cudaSuccess;
-  masked_copy_kernel<<<cols, 256, 0, st>>>(Vx, mask, ld, rows, dst, ld_dst);
+  const int pieces = std::min(65535, (rows + COPY_ROWS - 1) / COPY_ROWS);
+  masked_copy_kernel<<<dim3(cols, pieces), 256, 0, st>>>(Vx, mask, ld, rows, dst, ld_dst);
   return cudaGetLastError();
 }
 
@@ -2520,9 +2679,9 @@ cudaError_t launch_explained_variance(const MatrixDev &M, const float *x, double
   const int chunks = (M.n + EV_CHUNK - 1) / EV_CHUNK;
   ev_partial_kernel<<<dim3((M.m + 255) / 256, chunks), 256, 0, st>>>(M.Bc, M.ldm, M.m, M.n, x,
                                                                      partial);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  ev_sum_kernel<<<1, 1024, 0, st>>>(partial, chunks, M.m, out);
+  double *y = partial + (size_t)chunks * M.m;
+  rowsum_kernel<<<(M.m + 127) / 128, 128, 0, st>>>(partial, chunks, M.m, y);
+  ev_norm_kernel<<<1, 1024, 0, st>>>(y, M.m, out);
   return cudaGetLastError();
 }
 
@@ -2583,6 +2742,7 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   g1.gate_max = 0xFFFFFFFFu;
   const int mode = is_l1_variance(f) ? 1 : (is_constrained(f) ? 0 : 2);
   const size_t zplane = (size_t)b.k * M.ldm;  // second FP16 plane of Z
+  float *z_lo = b.fp16_2 ? nullptr : b.Z_lo;  // FP16 operands read no TF32 planes
   // 1a. sparse V (every column <= sparse_cap non-zeros last step): gather
   const bool wide = gather_is_wide(M.m);
   if ((e = mark(9)) != cudaSuccess) return e;
@@ -2598,7 +2758,7 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
     nl++;
   } else {
     gather_narrow_kernel<<<b.k, GATHER_THREADS, 0, st>>>(
-        mode, M.Bc, M.ldm, M.m, M.ldn, b.Vx, b.vmask, b.Z_hi, b.Z_lo, b.fz, b.max_nnz,
+        mode, M.Bc, M.ldm, M.m, M.ldn, b.Vx, b.vmask, b.Z_hi, z_lo, b.fz, b.max_nnz,
         b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
     nl++;
     if (ev) {  // one launch serves both kinds: am24_batch_step_timed names it by the counts
@@ -2635,7 +2795,7 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   const int splits1 = b.fp16_1 ? b.splits1p : b.splits1;
   if ((e = mark(1)) != cudaSuccess) return e;
   z_reduce_kernel<<<b.k, 256, 0, st>>>(mode, b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
-                                       b.Z_hi, b.Z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
+                                       b.Z_hi, z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
                                        b.Z_b, b.Z_h, zplane, b.z_scale, wide, b.ctl);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   nl++;

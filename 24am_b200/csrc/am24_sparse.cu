@@ -302,10 +302,8 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   if (S.long_cols.segs) AM24_TRY(A.get(&b.part_cols, (size_t)S.long_cols.segs * b.kp));
   if (S.long_rows.segs) AM24_TRY(A.get(&b.part_rows, (size_t)S.long_rows.segs * b.kp));
   if (S.comps) AM24_TRY(A.get(&b.defl_a, (size_t)k * SP_DEFL_MAX));
-  // every buffer starts defined: pool memory can hold an earlier call's state
-  AM24_CUDA(cudaMemsetAsync(b.vmask, 0, sizeof(uint32_t) * (size_t)k * (b.ldn / 32), h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.Vx, 0, sizeof(float) * (size_t)k * b.ldn, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.Vraw, 0, sizeof(float) * (size_t)k * b.ldn, h->stream));
+  // what a step could see before it is written starts defined: pool memory can
+  // hold an earlier call's state
   AM24_CUDA(cudaMemsetAsync(b.fz, 0, sizeof(float) * k, h->stream));
   AM24_CUDA(cudaMemsetAsync(b.obj_part, 0, sizeof(float) * k, h->stream));
   AM24_CUDA(cudaMemsetAsync(b.nnz_part, 0, sizeof(float) * k, h->stream));
@@ -344,7 +342,7 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
     // the batch's starts, staged in Vraw (or generated there), then split
     // into values and masks; ValueCoordinateHolder::reset
     if (s.start_mode == AM24_START_DEVICE_UNIFORM) {
-      AM24_CUDA(launch_uniform_starts(b.Vraw, b.ldn, (int)n, k, shift, h->stream));
+      AM24_CUDA(launch_uniform_starts(b.Vx, b.ldn, (int)n, k, shift, b.vmask, h->stream));
     } else {
       const float *src = start_points + (size_t)shift * n;
       if (s.start_mode != AM24_START_INJECTED) {
@@ -353,13 +351,10 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
       }
       AM24_CUDA(cudaMemcpy2DAsync(b.Vraw, sizeof(float) * b.ldn, src, sizeof(float) * n,
                                   sizeof(float) * n, k, cudaMemcpyHostToDevice, h->stream));
+      AM24_CUDA(launch_load_columns(b.Vraw, b.ldn, (int)n, k, b.Vx, b.ldn, b.vmask, h->stream));
     }
-    AM24_CUDA(launch_load_columns(b.Vraw, b.ldn, (int)n, k, b.Vx, b.ldn, b.vmask, h->stream));
-    AM24_CUDA(cudaMemsetAsync(b.sel_hint, 0, sizeof(float) * k, h->stream));
-    AM24_CUDA(cudaMemsetAsync(b.val, 0, sizeof(float) * k, h->stream));
-    AM24_CUDA(cudaMemsetAsync(b.err, 0, sizeof(float) * k, h->stream));
-    AM24_CUDA(cudaMemsetAsync(b.ctl, 0, sizeof(uint32_t) * CTL_WORDS, h->stream));
-    AM24_CUDA(cudaMemsetAsync(b.max_nnz, 0xFF, sizeof(uint32_t), h->stream));  // dense starts
+    AM24_CUDA(launch_reset_batch(k, b.sel_hint, b.val, b.err, b.max_nnz, nullptr, b.ctl,
+                                 h->stream));
     AM24_CUDA(cudaEventRecord(e0, h->stream));
     // the batch loop: finalize sets the stop word after the step the
     // reference's loop ends on; the host reads it after each step

@@ -303,9 +303,8 @@ am24_status run_batch_steps(am24_handle h, am24_batch b, const am24_settings &s,
   for (int it = 0; it < s.max_iter; it++) {
     StepParams p = step_params(s, it, shift);
     p.stop_check = 1;
+    p.host_stop = &h->flags[it % AHEAD];
     AM24_CUDA(launch_am_step(b->mat->d, b->d, b->tm, p, h->stream, &b->launches));
-    AM24_CUDA(cudaMemcpyAsync(&h->flags[it % AHEAD], d.ctl + CTL_STOP, sizeof(uint32_t),
-                              cudaMemcpyDeviceToHost, h->stream));
     AM24_CUDA(cudaEventRecord(h->run_ev[it % AHEAD], h->stream));
     const int probe = it - (AHEAD - 1);  // the oldest step still unread
     if (probe >= 0) {
@@ -878,8 +877,8 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
   }
   // a gather over V's non-zeros beats the dense product while they are few
   d.sparse_cap = (uint32_t)std::min(4096, M.n / 32);
-  b->launches = (is_constrained(settings->formulation) ? 7 : 6) +
-                (gather_is_wide(M.m) ? 1 : 0) + (d.mixed ? 2 : 0);
+  b->launches = 6 + (gather_is_wide(M.m) ? 1 : 0) +
+                (d.mixed ? (is_constrained(settings->formulation) ? 3 : 2) : 0);
   *out = b;
   return AM24_OK;
 }

@@ -210,16 +210,16 @@ __global__ void __launch_bounds__(256) g_z_reduce_kernel(GroupDev g) {
 
 __global__ void __launch_bounds__(HARD_THREADS) g_hard_select_kernel(GroupDev g) {
   for_items(g, GL_SEL_HARD, [](const GProblem &P, int j) {
-    hard_select_body(P.Vraw, P.ldn, P.n, P.constraint, P.Vx, P.nnz, P.status, P.vmask,
-                     P.sel_hint, P.ctl + CTL_STOP, P.cmask, j);
+    hard_select_body(P.Vraw, P.ldn, P.n, P.constraint, P.Vx, P.nnz, P.vmask,
+                     P.sel_hint, P.cmask, j);
   });
 }
 
 template <bool EXACT>
 __global__ void __launch_bounds__(SOFT_THREADS, 4) g_soft_select_kernel(GroupDev g) {
   for_items(g, EXACT ? GL_SEL_EXACT : GL_SEL_SCAN, [](const GProblem &P, int j) {
-    soft_select_body<EXACT>(P.Vraw, P.ldn, P.n, P.constraint, P.Vx, P.nnz, P.status, P.vmask,
-                            P.sel_hint, P.ctl + CTL_STOP, P.cmask, j);
+    soft_select_body<EXACT>(P.Vraw, P.ldn, P.n, P.constraint, P.Vx, P.nnz, P.vmask,
+                            P.sel_hint, P.cmask, j);
   });
 }
 
@@ -287,7 +287,8 @@ __global__ void __launch_bounds__(256) g_finalize_kernel(GroupDev g) {
     a.val = P.val;
     a.err = P.err;
     a.max_err = P.max_err;
-    a.max_nnz = P.ctl + GCTL_NEXT;
+    a.next_nnz = P.ctl + GCTL_NEXT;
+    a.max_nnz = a.planes_nnz = a.host_stop = nullptr;  // the plan hands the count on
     a.iters = nullptr;
     a.cards = nullptr;
     a.ctl = P.ctl;

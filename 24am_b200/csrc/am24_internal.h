@@ -127,6 +127,7 @@ struct StepParams {
   int log_shift;      // batch shift of the per-start logs
   unsigned long long timeout_ns;
   int stop_check = 0;  // the step sets the stop word when the batch loop would end
+  uint32_t *host_stop = nullptr;  // pinned host word the step writes the stop word to
 };
 
 // The sparse Z = B V of matrices with few samples is one launch, which
@@ -143,6 +144,7 @@ enum : int {
   CTL_LOW_STEPS = 2,  // ... of them in the BF16 phase (MIXED)
   CTL_MAX_ERR = 3,    // the last executed step's largest change (float bits)
   CTL_BLOCKS = 4,     // finalize's block counter (scratch)
+  CTL_NEXT_NNZ = 5,   // the running step's largest non-zero count
   CTL_WORDS = 8
 };
 

@@ -456,6 +456,7 @@ __global__ void densify_kernel(const float *__restrict__ Vx, const uint32_t *__r
                                float *__restrict__ V_lo, const uint32_t *gate,
                                const uint32_t *planes, uint32_t gate_max,
                                const uint32_t *stop) {
+  pdl_enter();
   if (*stop || *gate <= gate_max || *planes > gate_max) return;
   const size_t c = blockIdx.x;
   for (int r = threadIdx.x; r < ld; r += blockDim.x) {
@@ -526,6 +527,7 @@ __global__ void __launch_bounds__(DENSIFY_THREADS, DENSIFY_BLOCKS_PER_SM) densif
     const float *__restrict__ Vx, const uint32_t *__restrict__ mask, int ld, int rows,
     uint16_t *__restrict__ Vh, size_t plane, float *__restrict__ v_scale, const uint32_t *gate,
     uint32_t gate_max, const uint32_t *stop, int k) {
+  pdl_enter();
   for (int c = blockIdx.x; c < k; c += gridDim.x) {
     densify_fp16_body(Vx, mask, ld, rows, Vh, plane, v_scale, gate, gate_max, stop, c);
     __syncthreads();  // red[] is reused by the next column
@@ -713,6 +715,7 @@ __global__ void __launch_bounds__(256) z_reduce_kernel(int mode, const float *__
                                                        uint16_t *__restrict__ Zh, size_t zplane,
                                                        float *__restrict__ zscale, bool wide,
                                                        const uint32_t *stop) {
+  pdl_enter();
   if (*stop) return;
   const bool dense = *gate > gate_max;
   if (!dense && !wide) return;  // gather_narrow_kernel produced Z this step
@@ -747,6 +750,7 @@ __global__ void __launch_bounds__(256) support_kernel(const uint32_t *__restrict
                                                       uint32_t *stable, uint32_t *phase,
                                                       uint32_t k_stable, uint32_t need,
                                                       const uint32_t *stop) {
+  pdl_enter();
   if (*stop) return;
   const int j = blockIdx.x;
   const uint32_t *a = vmask + (size_t)j * words, *b = prev + (size_t)j * words;
@@ -896,8 +900,12 @@ __global__ void __launch_bounds__(GATHER_THREADS) gather_narrow_kernel(
     int mode, const float *__restrict__ Bc, int ldm, int m, int ldn, const float *__restrict__ Vx,
     const uint32_t *__restrict__ vmask, float *__restrict__ Z_hi, float *__restrict__ Z_lo,
     float *__restrict__ fz, const uint32_t *gate, uint32_t gate_max, uint16_t *__restrict__ Zb,
-    uint16_t *__restrict__ Zh, size_t zplane, float *__restrict__ zscale, const uint32_t *stop) {
-  if (*stop || *gate > gate_max) return;  // dense V: gemm1 + z_reduce
+    uint16_t *__restrict__ Zh, size_t zplane, float *__restrict__ zscale, float *max_err,
+    const uint32_t *stop) {
+  pdl_enter();
+  if (*stop) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *max_err = 0.f;  // the step begins here
+  if (*gate > gate_max) return;  // dense V: gemm1 + z_reduce
   gather_narrow_body(mode, Bc, ldm, m, ldn, Vx, vmask,
                      z_out(blockIdx.x, ldm, Z_hi, Z_lo, Zb, Zh, zplane, zscale, fz), blockIdx.x);
 }
@@ -920,8 +928,11 @@ __device__ __forceinline__ void gather_list_body(int ldn, const float *__restric
 }
 __global__ void __launch_bounds__(GATHER_THREADS) gather_list_kernel(
     int ldn, const float *__restrict__ Vx, const uint32_t *__restrict__ vmask, const uint32_t *gate,
-    uint32_t gate_max, int2 *__restrict__ lists, const uint32_t *stop) {
-  if (*stop || *gate > gate_max) return;
+    uint32_t gate_max, int2 *__restrict__ lists, float *max_err, const uint32_t *stop) {
+  pdl_enter();
+  if (*stop) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *max_err = 0.f;  // the step begins here
+  if (*gate > gate_max) return;
   gather_list_body(ldn, Vx, vmask, gate_max, lists, blockIdx.x);
 }
 
@@ -965,6 +976,7 @@ __device__ __forceinline__ void gather_tile_body(const float *__restrict__ Bc, i
 __global__ void __launch_bounds__(GATHER_THREADS) gather_tile_kernel(
     const float *__restrict__ Bc, int ldm, int ldn, int k, const int2 *__restrict__ lists,
     float *__restrict__ Z_hi, const uint32_t *gate, uint32_t gate_max, const uint32_t *stop) {
+  pdl_enter();
   if (*stop || *gate > gate_max) return;
   gather_tile_body(Bc, ldm, ldn, k, lists, Z_hi, blockIdx.x);
 }
@@ -1269,6 +1281,116 @@ __device__ uint32_t pairs_from_mask(const uint32_t *__restrict__ mk, int words,
   return total;
 }
 
+// ------------------------------------------------------------ end of a step
+// Per start: objective f, relative change |f - f0| / f0
+// (c++/src/utils/termination_criteria.h:30-36), the storeIterationsForAllPoints
+// logs (c++/src/gpower/gpower_commons.h:120-130), and the batch maximum that
+// ignores NaN changes (:132-133).  Runs at the end of the select kernels, or as
+// finalize_kernel where a step has no select (the penalties) or another pass
+// after it (MIXED).
+struct FinalizeArgs {
+  int k, formulation, parts, it, store_all, log_shift, log_capacity;
+  double tolerance;
+  const float *fz;
+  const float *obj_part, *nnz_part;
+  const uint32_t *nnz_sel;
+  float *val, *err, *max_err;
+  uint32_t *next_nnz;    // the step's largest non-zero count is formed here ...
+  uint32_t *max_nnz;     // ... and becomes the next step's gate as the step closes
+  uint32_t *planes_nnz;  // takes the closing step's own gate (null: not wanted)
+  int *iters, *cards;
+  // run-ahead control (StepCtl words); stop_check: this step may stop the batch
+  uint32_t *ctl;
+  uint32_t *host_stop;    // pinned host word that takes the stop word (or null)
+  const uint32_t *phase;  // MIXED: phase[3] is the phase the step ran in; else null
+  const int *status;
+  int stop_check;
+};
+
+// Whether the batch had stopped before this step (tells the host so).
+__device__ __forceinline__ bool step_stopped(const FinalizeArgs &a) {
+  if (!a.ctl[CTL_STOP]) return false;
+  if (a.host_stop && blockIdx.x == 0 && threadIdx.x == 0)
+    *reinterpret_cast<volatile uint32_t *>(a.host_stop) = 1u;
+  return true;
+}
+
+// One start's objective f and non-zero count (one thread).  The batch maximum
+// is an atomicMax on the bit pattern of the (non-negative, non-NaN) changes,
+// zeroed as the step begins -- max is order-independent, so the result is
+// deterministic.
+__device__ void finalize_value(const FinalizeArgs &a, int j, float f, uint32_t nz) {
+  atomicMax(a.next_nnz, nz);
+  const float f0 = a.val[j];
+  const float e = fabsf(f - f0) / f0;
+  a.err[j] = e;
+  a.val[j] = f;
+  // the reference's `if (max < e) max = e`: NaN never wins
+  if (e > 0.f) atomicMax(reinterpret_cast<unsigned int *>(a.max_err), __float_as_uint(e));
+  if (a.store_all) {
+    // the penalized thresholding calls log into slot j of every batch
+    // (gpower_commons.h:170,173 leave the batch shift at 0)
+    const int slot = a.formulation <= 3 ? a.log_shift + j : j;
+    if (slot < a.log_capacity) {
+      const bool done = a.it > 0 && (double)e < a.tolerance;
+      if (done && a.iters[slot] == -1) {
+        a.iters[slot] = a.it;
+        a.cards[slot] = (int)nz;
+      } else if (!done && a.iters[slot] != -1) {
+        a.iters[slot] = -1;
+      }
+    }
+  }
+}
+
+// One start, by a warp (lane 0 writes): the constraints' values as they stand,
+// the penalties' from the epilogue's partials.
+__device__ void finalize_start(const FinalizeArgs &a, int j, int lane) {
+  float f;
+  uint32_t nz;
+  if (a.formulation <= 3) {
+    f = a.fz[j];
+    nz = a.nnz_sel[j];
+  } else {
+    // fixed order: lane-strided partial sums, then a butterfly
+    double acc = 0.0, c = 0.0;
+    for (int q = lane; q < a.parts; q += 32) {
+      acc += (double)a.obj_part[(size_t)j * a.parts + q];
+      c += (double)a.nnz_part[(size_t)j * a.parts + q];
+    }
+    acc = warp_sum(acc);
+    c = warp_sum(c);
+    f = a.formulation >= 6 ? (float)sqrt(acc) : (float)acc;
+    nz = (uint32_t)c;
+  }
+  if (lane == 0) finalize_value(a, j, f, nz);
+}
+
+// Called by one thread of every block once its starts are done.  The last block
+// closes the step for the run-ahead driver: it counts the step (and, MIXED,
+// whether it ran in the BF16 phase), keeps the batch's largest change, hands the
+// non-zero count to the next step, and sets the stop word when the reference's
+// batch loop would end here (it > 0, a refinement step, max change < tolerance)
+// or a device-side wait gave up.
+__device__ void close_step(const FinalizeArgs &a) {
+  __threadfence();
+  if (atomicAdd(&a.ctl[CTL_BLOCKS], 1u) != gridDim.x - 1) return;
+  __threadfence();
+  const float me = *reinterpret_cast<volatile float *>(a.max_err);
+  const bool refined = a.phase == nullptr || a.phase[3] != 0u;
+  a.ctl[CTL_STEPS] += 1u;
+  if (!refined) a.ctl[CTL_LOW_STEPS] += 1u;
+  a.ctl[CTL_MAX_ERR] = __float_as_uint(me);
+  if (a.planes_nnz) *a.planes_nnz = *a.max_nnz;
+  *a.max_nnz = atomicExch(a.next_nnz, 0u);
+  const bool stop =
+      (a.stop_check && a.it > 0 && refined && (double)me < a.tolerance) ||
+      *reinterpret_cast<const volatile int *>(a.status) != 0;
+  if (stop) a.ctl[CTL_STOP] = 1u;
+  if (a.host_stop) *reinterpret_cast<volatile uint32_t *>(a.host_stop) = stop ? 1u : 0u;
+  a.ctl[CTL_BLOCKS] = 0u;
+}
+
 // ------------------------------------------------------------ L0 constraint
 constexpr int HARD_THREADS = 256;
 constexpr int HARD_CAND = 2048;  // hinted (key, index) candidates resolved in shared memory
@@ -1433,9 +1555,8 @@ __device__ uint32_t gather_keys_above(const float *__restrict__ colg, int n, uin
 // came up short streamed the column twice).
 __device__ __forceinline__ void hard_select_body(
     const float *__restrict__ Vraw, int ldv, int n, unsigned s, float *__restrict__ Vx,
-    uint32_t *__restrict__ nnz_out, int *status, uint32_t *__restrict__ vmask,
-    float *__restrict__ hints, const uint32_t *stop, const uint32_t *__restrict__ cmask, int j) {
-  if (*stop) return;
+    uint32_t *__restrict__ nnz_out, uint32_t *__restrict__ vmask, float *__restrict__ hints,
+    const uint32_t *__restrict__ cmask, int j) {
   // also 2 * HARD_CAND keys for (b), and the sample, read 16 bytes at a time
   __shared__ __align__(16) uint64_t cand[HARD_CAND];
   __shared__ uint32_t hist[2048];
@@ -1550,11 +1671,18 @@ __device__ __forceinline__ void hard_select_body(
     nnz_out[j] = (uint32_t)cnt;
   }
 }
+// `finish`: the step ends here (FinalizeArgs), one start per block.
 __global__ void __launch_bounds__(HARD_THREADS) hard_select_kernel(
     const float *__restrict__ Vraw, int ldv, int n, unsigned s, float *__restrict__ Vx,
-    uint32_t *__restrict__ nnz_out, int *status, uint32_t *__restrict__ vmask,
-    float *__restrict__ hints, const uint32_t *stop, const uint32_t *__restrict__ cmask) {
-  hard_select_body(Vraw, ldv, n, s, Vx, nnz_out, status, vmask, hints, stop, cmask, blockIdx.x);
+    uint32_t *__restrict__ nnz_out, uint32_t *__restrict__ vmask, float *__restrict__ hints,
+    const uint32_t *__restrict__ cmask, FinalizeArgs a, bool finish) {
+  pdl_enter();
+  if (step_stopped(a)) return;
+  hard_select_body(Vraw, ldv, n, s, Vx, nnz_out, vmask, hints, cmask, blockIdx.x);
+  if (finish && threadIdx.x == 0) {
+    finalize_value(a, blockIdx.x, a.fz[blockIdx.x], nnz_out[blockIdx.x]);
+    close_step(a);
+  }
 }
 
 // ------------------------------------------------------------ L1 constraint
@@ -1849,9 +1977,8 @@ __device__ __noinline__ uint32_t exact_walk(Src src, uint32_t len, uint32_t n, d
 template <bool EXACT>
 __device__ __forceinline__ void soft_select_body(
     const float *__restrict__ Vraw, int ldv, int n, unsigned s, float *__restrict__ Vx,
-    uint32_t *__restrict__ nnz_out, int *status, uint32_t *__restrict__ vmask,
-    float *__restrict__ hints, const uint32_t *stop, const uint32_t *__restrict__ cmask, int j) {
-  if (*stop) return;
+    uint32_t *__restrict__ nnz_out, uint32_t *__restrict__ vmask, float *__restrict__ hints,
+    const uint32_t *__restrict__ cmask, int j) {
   // dynamic shared memory (SOFT_SMEM bytes): the hinted (key, index)
   // candidates, a chunk of sorted values and its prefix sums; the histogram
   // of the slower paths reuses the candidates' space (those paths run only
@@ -2118,109 +2245,27 @@ __device__ __forceinline__ void soft_select_body(
 template <bool EXACT>
 __global__ void __launch_bounds__(SOFT_THREADS, 4) soft_select_kernel(
     const float *__restrict__ Vraw, int ldv, int n, unsigned s, float *__restrict__ Vx,
-    uint32_t *__restrict__ nnz_out, int *status, uint32_t *__restrict__ vmask,
-    float *__restrict__ hints, const uint32_t *stop, const uint32_t *__restrict__ cmask) {
-  soft_select_body<EXACT>(Vraw, ldv, n, s, Vx, nnz_out, status, vmask, hints, stop, cmask,
-                          blockIdx.x);
+    uint32_t *__restrict__ nnz_out, uint32_t *__restrict__ vmask, float *__restrict__ hints,
+    const uint32_t *__restrict__ cmask, FinalizeArgs a, bool finish) {
+  pdl_enter();
+  if (step_stopped(a)) return;
+  soft_select_body<EXACT>(Vraw, ldv, n, s, Vx, nnz_out, vmask, hints, cmask, blockIdx.x);
+  if (finish && threadIdx.x == 0) {
+    finalize_value(a, blockIdx.x, a.fz[blockIdx.x], nnz_out[blockIdx.x]);
+    close_step(a);
+  }
 }
 
 // ------------------------------------------------------------ finalize
-// Per start: objective f, relative change |f - f0| / f0
-// (c++/src/utils/termination_criteria.h:30-36), the storeIterationsForAllPoints
-// logs (c++/src/gpower/gpower_commons.h:120-130), and the batch maximum that
-// ignores NaN changes (:132-133).  One block.
-struct FinalizeArgs {
-  int k, formulation, parts, it, store_all, log_shift, log_capacity;
-  double tolerance;
-  const float *fz;
-  const float *obj_part, *nnz_part;
-  const uint32_t *nnz_sel;
-  float *val, *err, *max_err;
-  uint32_t *max_nnz;
-  int *iters, *cards;
-  // run-ahead control (StepCtl words); stop_check: this step may stop the batch
-  uint32_t *ctl;
-  const uint32_t *phase;  // MIXED: phase[3] is the phase the step ran in; else null
-  const int *status;
-  int stop_check;
-};
-
-// One warp per start; the batch maximum is an atomicMax on the bit pattern
-// of the (non-negative, non-NaN) changes, zeroed before the step -- max is
-// order-independent, so the result is deterministic.
-__device__ void finalize_start(const FinalizeArgs &a, int j, int lane);
-
-// The last block to finish also closes the step for the run-ahead driver: it
-// counts the step (and, MIXED, whether it ran in the BF16 phase), keeps the
-// batch's largest change, and sets the stop word when the reference's batch
-// loop would end here (it > 0, a refinement step, max change < tolerance) or
-// a device-side wait gave up.
+// Penalized and MIXED steps: one warp per start, after the step's other passes.
 __global__ void __launch_bounds__(256) finalize_kernel(FinalizeArgs a) {
-  if (a.ctl[CTL_STOP]) return;
+  pdl_enter();
+  if (step_stopped(a)) return;
   const int lane = threadIdx.x & 31;
   const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (j < a.k) finalize_start(a, j, lane);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(&a.ctl[CTL_BLOCKS], 1u) == gridDim.x - 1) {
-      __threadfence();
-      const float me = *reinterpret_cast<volatile float *>(a.max_err);
-      const bool refined = a.phase == nullptr || a.phase[3] != 0u;
-      a.ctl[CTL_STEPS] += 1u;
-      if (!refined) a.ctl[CTL_LOW_STEPS] += 1u;
-      a.ctl[CTL_MAX_ERR] = __float_as_uint(me);
-      if ((a.stop_check && a.it > 0 && refined && (double)me < a.tolerance) ||
-          *reinterpret_cast<const volatile int *>(a.status) != 0)
-        a.ctl[CTL_STOP] = 1u;
-      a.ctl[CTL_BLOCKS] = 0u;
-    }
-  }
-}
-
-// One start's objective, change and logs (one warp; lane 0 writes).
-__device__ void finalize_start(const FinalizeArgs &a, int j, int lane) {
-  const bool cons = a.formulation <= 3;
-  const bool l1pen = a.formulation >= 6;
-  float f;
-  uint32_t nz;
-  if (cons) {
-    f = a.fz[j];
-    nz = a.nnz_sel[j];
-  } else {
-    // fixed order: lane-strided partial sums, then a butterfly
-    double acc = 0.0, c = 0.0;
-    for (int q = lane; q < a.parts; q += 32) {
-      acc += (double)a.obj_part[(size_t)j * a.parts + q];
-      c += (double)a.nnz_part[(size_t)j * a.parts + q];
-    }
-    acc = warp_sum(acc);
-    c = warp_sum(c);
-    f = l1pen ? (float)sqrt(acc) : (float)acc;
-    nz = (uint32_t)c;
-  }
-  if (lane != 0) return;
-  atomicMax(a.max_nnz, nz);
-  const float f0 = a.val[j];
-  const float e = fabsf(f - f0) / f0;
-  a.err[j] = e;
-  a.val[j] = f;
-  // the reference's `if (max < e) max = e`: NaN never wins
-  if (e > 0.f) atomicMax(reinterpret_cast<unsigned int *>(a.max_err), __float_as_uint(e));
-  if (a.store_all) {
-    // the penalized thresholding calls log into slot j of every batch
-    // (gpower_commons.h:170,173 leave the batch shift at 0)
-    const int slot = cons ? a.log_shift + j : j;
-    if (slot < a.log_capacity) {
-      const bool done = a.it > 0 && (double)e < a.tolerance;
-      if (done && a.iters[slot] == -1) {
-        a.iters[slot] = a.it;
-        a.cards[slot] = (int)nz;
-      } else if (!done && a.iters[slot] != -1) {
-        a.iters[slot] = -1;
-      }
-    }
-  }
+  if (threadIdx.x == 0) close_step(a);
 }
 
 // x = v / ||v|| (c++/src/gpower/sparse_PCA_solver.h:236-237).
@@ -2405,6 +2450,28 @@ cudaError_t kernel_setup(K kern, int smem, bool pair, int *clusters = nullptr) {
   return it->second.err;
 }
 
+// Launches a kernel of a step so that it may start while the one before it
+// still runs (programmatic stream serialization): every step kernel begins with
+// pdl_enter(), which waits for that one to complete, so only launch latency and
+// set-up overlap.  A small batch's step is a chain of short kernels: 20 steps of 64
+// starts of 96 x 640 took 1323 us with 2 us and a memset or copy between kernels,
+// 849 with this and none.
+template <class... P, class... A>
+cudaError_t launch_step(void (*kern)(P...), int grid, int threads, int smem, cudaStream_t st,
+                        A &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+
 template <int BN, int BKT, int ST, class Epi>
 cudaError_t run_gemm(const CUtensorMap &a_hi, const CUtensorMap &a_lo, const CUtensorMap &b_hi,
                      const CUtensorMap &b_lo, const GemmShape &sh, const Epi &epi,
@@ -2414,8 +2481,7 @@ cudaError_t run_gemm(const CUtensorMap &a_hi, const CUtensorMap &a_lo, const CUt
   const cudaError_t e = kernel_setup(kern, L::TOTAL, false);
   if (e != cudaSuccess) return e;
   const int grid = sh.num_units < num_sms() ? sh.num_units : num_sms();
-  kern<<<grid, GEMM_THREADS, L::TOTAL, st>>>(a_hi, a_lo, b_hi, b_lo, sh, epi);
-  return cudaGetLastError();
+  return launch_step(kern, grid, GEMM_THREADS, L::TOTAL, st, a_hi, a_lo, b_hi, b_lo, sh, epi);
 }
 
 // Stages per (N tile, K slab) fill ~192 KB of shared memory.
@@ -2434,8 +2500,7 @@ cudaError_t run_gemm_pair(const CUtensorMap &m0, const CUtensorMap &m1, const CU
   s2.splits = (s2.kb_total + s2.kb_per_split - 1) / s2.kb_per_split;
   s2.num_units = s2.splits * ((sh.m_tiles + 1) / 2) * sh.n_tiles;
   const int pairs = s2.num_units < clusters ? s2.num_units : clusters;
-  kern<<<2 * pairs, GEMM_THREADS, L::TOTAL, st>>>(m0, m1, m2, m3, s2, epi);
-  return cudaGetLastError();
+  return launch_step(kern, 2 * pairs, GEMM_THREADS, L::TOTAL, st, m0, m1, m2, m3, s2, epi);
 }
 
 template <class Epi>
@@ -2708,6 +2773,21 @@ cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double
   return cudaGetLastError();
 }
 
+// The select of a constrained form (the L1 ball in p's mode); see the kernels.
+static cudaError_t launch_select(int f, const StepParams &p, int k, const float *Vraw, int ldn,
+                                 int n, float *Vx, uint32_t *nnz, uint32_t *vmask, float *hints,
+                                 const uint32_t *cmask, const FinalizeArgs &fa, bool finish,
+                                 cudaStream_t st) {
+  if (!is_l1_constrained(f))
+    return launch_step(hard_select_kernel, k, HARD_THREADS, 0, st, Vraw, ldn, n, p.constraint, Vx,
+                       nnz, vmask, hints, cmask, fa, finish);
+  auto kern = p.l1_mode == 0 ? soft_select_kernel<false> : soft_select_kernel<true>;
+  const cudaError_t e = kernel_setup(kern, SOFT_SMEM, false);
+  if (e != cudaSuccess) return e;
+  return launch_step(kern, k, SOFT_THREADS, SOFT_SMEM, st, Vraw, ldn, n, p.constraint, Vx, nnz,
+                     vmask, hints, cmask, fa, finish);
+}
+
 cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm,
                            const StepParams &p, cudaStream_t st, int *launches, cudaEvent_t *ev,
                            int *kinds) {
@@ -2718,7 +2798,6 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
     if (kinds) kinds[nl] = kind;
     return ev ? cudaEventRecord(ev[nl], st) : cudaSuccess;
   };
-  if ((e = cudaMemsetAsync(b.max_err, 0, sizeof(float), st)) != cudaSuccess) return e;
   if (b.mixed &&  // the support this step starts from, for the stability count
       (e = cudaMemcpyAsync(b.vmask_prev, b.vmask, sizeof(uint32_t) * (size_t)b.k * (M.ldn / 32),
                            cudaMemcpyDeviceToDevice, st)) != cudaSuccess)
@@ -2749,34 +2828,37 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   if (wide) {
     // the lists take the dense planes' place (not read on sparse steps)
     int2 *lists = reinterpret_cast<int2 *>(b.fp16_1 ? (void *)b.V_h : (void *)b.V_hi);
-    gather_list_kernel<<<b.k, GATHER_THREADS, 0, st>>>(M.ldn, b.Vx, b.vmask, b.max_nnz,
-                                                       b.sparse_cap, lists, b.ctl);
+    if ((e = launch_step(gather_list_kernel, b.k, GATHER_THREADS, 0, st, M.ldn, b.Vx, b.vmask,
+                         b.max_nnz, b.sparse_cap, lists, b.max_err, b.ctl)) != cudaSuccess)
+      return e;
     nl++;
     if ((e = mark(5)) != cudaSuccess) return e;
-    gather_tile_kernel<<<gather_tiles(M.ldm) * gather_groups(b.k), GATHER_THREADS, 0, st>>>(
-        M.Bc, M.ldm, M.ldn, b.k, lists, b.Z_hi, b.max_nnz, b.sparse_cap, b.ctl);
+    if ((e = launch_step(gather_tile_kernel, gather_tiles(M.ldm) * gather_groups(b.k),
+                         GATHER_THREADS, 0, st, M.Bc, M.ldm, M.ldn, b.k, lists, b.Z_hi,
+                         b.max_nnz, b.sparse_cap, b.ctl)) != cudaSuccess)
+      return e;
     nl++;
   } else {
-    gather_narrow_kernel<<<b.k, GATHER_THREADS, 0, st>>>(
-        mode, M.Bc, M.ldm, M.m, M.ldn, b.Vx, b.vmask, b.Z_hi, z_lo, b.fz, b.max_nnz,
-        b.sparse_cap, b.Z_b, b.Z_h, zplane, b.z_scale, b.ctl);
+    if ((e = launch_step(gather_narrow_kernel, b.k, GATHER_THREADS, 0, st, mode, M.Bc, M.ldm, M.m,
+                         M.ldn, b.Vx, b.vmask, b.Z_hi, z_lo, b.fz, b.max_nnz, b.sparse_cap, b.Z_b,
+                         b.Z_h, zplane, b.z_scale, b.max_err, b.ctl)) != cudaSuccess)
+      return e;
     nl++;
     if (ev) {  // one launch serves both kinds: am24_batch_step_timed names it by the counts
       if ((e = mark(5)) != cudaSuccess) return e;
       nl++;
     }
   }
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   // 1b. dense V: TF32 hi/lo planes, tensor-core Z = B V (split-K partials) ...
   if ((e = mark(6)) != cudaSuccess) return e;
   if (b.fp16_1)
-    densify_fp16_kernel<<<std::min(b.k, DENSIFY_BLOCKS_PER_SM * num_sms()), DENSIFY_THREADS, 0,
-                          st>>>(b.Vx, b.vmask, M.ldn, M.n, b.V_h, (size_t)b.k * M.ldn, b.v_scale,
-                                b.max_nnz, b.sparse_cap, b.ctl, b.k);
+    e = launch_step(densify_fp16_kernel, std::min(b.k, DENSIFY_BLOCKS_PER_SM * num_sms()),
+                    DENSIFY_THREADS, 0, st, b.Vx, b.vmask, M.ldn, M.n, b.V_h, (size_t)b.k * M.ldn,
+                    b.v_scale, b.max_nnz, b.sparse_cap, b.ctl, b.k);
   else
-    densify_kernel<<<b.k, 256, 0, st>>>(b.Vx, b.vmask, M.ldn, M.n, b.V_hi, b.V_lo, b.max_nnz,
-                                        b.planes_nnz, b.sparse_cap, b.ctl);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_step(densify_kernel, b.k, 256, 0, st, b.Vx, b.vmask, M.ldn, M.n, b.V_hi, b.V_lo,
+                    b.max_nnz, b.planes_nnz, b.sparse_cap, b.ctl);
+  if (e != cudaSuccess) return e;
   nl++;
   EpiPartial ep{b.ws, b.bn1, b.m_tiles1, b.n_tiles1};
   if ((e = mark(0)) != cudaSuccess) return e;
@@ -2794,10 +2876,10 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   // 2. ... then reduce + sign / normalise
   const int splits1 = b.fp16_1 ? b.splits1p : b.splits1;
   if ((e = mark(1)) != cudaSuccess) return e;
-  z_reduce_kernel<<<b.k, 256, 0, st>>>(mode, b.ws, splits1, b.m_tiles1, b.n_tiles1, b.bn1, M.m,
-                                       b.Z_hi, z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
-                                       b.Z_b, b.Z_h, zplane, b.z_scale, wide, b.ctl);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  if ((e = launch_step(z_reduce_kernel, b.k, 256, 0, st, mode, b.ws, splits1, b.m_tiles1,
+                       b.n_tiles1, b.bn1, M.m, b.Z_hi, z_lo, M.ldm, b.fz, b.max_nnz, b.sparse_cap,
+                       b.Z_b, b.Z_h, zplane, b.z_scale, wide, b.ctl)) != cudaSuccess)
+    return e;
   nl++;
   // 3. V = B^T Z
   GemmShape g2;
@@ -2869,42 +2951,6 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
     e = gemm2(pe);
   }
   if (e != cudaSuccess) return e;
-  // 4. constrained: selection / projection + normalisation
-  if (is_constrained(f)) {
-    if ((e = mark(3)) != cudaSuccess) return e;
-    if (!is_l1_constrained(f)) {
-      hard_select_kernel<<<b.k, HARD_THREADS, 0, st>>>(b.Vraw, M.ldn, M.n, p.constraint, b.Vx,
-                                                        b.nnz, b.status, b.vmask, b.sel_hint,
-                                                        b.ctl, b.cmask);
-      e = cudaGetLastError();
-    } else {
-      if (p.l1_mode == 0) {
-        if ((e = kernel_setup(soft_select_kernel<false>, SOFT_SMEM, false)) != cudaSuccess)
-          return e;
-        soft_select_kernel<false><<<b.k, SOFT_THREADS, SOFT_SMEM, st>>>(
-            b.Vraw, M.ldn, M.n, p.constraint, b.Vx, b.nnz, b.status, b.vmask, b.sel_hint, b.ctl,
-            b.cmask);
-      } else {
-        if ((e = kernel_setup(soft_select_kernel<true>, SOFT_SMEM, false)) != cudaSuccess)
-          return e;
-        soft_select_kernel<true><<<b.k, SOFT_THREADS, SOFT_SMEM, st>>>(
-            b.Vraw, M.ldn, M.n, p.constraint, b.Vx, b.nnz, b.status, b.vmask, b.sel_hint, b.ctl,
-            b.cmask);
-      }
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) return e;
-    nl++;
-  }
-  // 4b. MIXED: support stability and the phase switch
-  if (b.mixed) {
-    if ((e = mark(8)) != cudaSuccess) return e;
-    support_kernel<<<b.k, 256, 0, st>>>(b.vmask, b.vmask_prev, M.ldn / 32, b.stable, b.phase,
-                                        b.k_stable, b.need_stable, b.ctl);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    nl++;
-  }
-  // 5. finalize
   FinalizeArgs fa;
   fa.k = b.k;
   fa.formulation = f;
@@ -2923,23 +2969,39 @@ cudaError_t launch_am_step(const MatrixDev &M, BatchDev &b, const TensorMaps &tm
   fa.max_err = b.max_err;
   fa.iters = b.iters;
   fa.cards = b.cards;
+  fa.next_nnz = b.ctl + CTL_NEXT_NNZ;
   fa.max_nnz = b.max_nnz;
+  // penalized forms: the count this step's epilogue saw (whether it wrote the
+  // dense planes), for the next step's densify gate
+  fa.planes_nnz = !is_constrained(f) && !b.fp16_1 ? b.planes_nnz : nullptr;
   fa.ctl = b.ctl;
+  fa.host_stop = p.host_stop;
   fa.phase = b.mixed ? b.phase : nullptr;
   fa.status = b.status;
   fa.stop_check = p.stop_check;
-  // Z = B V of this step has read max_nnz; finalize sets it for the next step
-  // penalized forms: the count this step's epilogue saw (whether it wrote the
-  // dense planes), for the next step's densify gate
-  if (!is_constrained(f) && !b.fp16_1 &&
-      (e = cudaMemcpyAsync(b.planes_nnz, b.max_nnz, sizeof(uint32_t), cudaMemcpyDeviceToDevice,
-                           st)) != cudaSuccess)
-    return e;
-  if ((e = cudaMemsetAsync(b.max_nnz, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-  if ((e = mark(4)) != cudaSuccess) return e;
-  finalize_kernel<<<(b.k + 7) / 8, 256, 0, st>>>(fa);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  nl++;
+  // 4. constrained: selection / projection + normalisation, and the step's end
+  const bool finish = is_constrained(f) && !b.mixed;
+  if (is_constrained(f)) {
+    if ((e = mark(3)) != cudaSuccess) return e;
+    if ((e = launch_select(f, p, b.k, b.Vraw, M.ldn, M.n, b.Vx, b.nnz, b.vmask, b.sel_hint, b.cmask,
+                           fa, finish, st)) != cudaSuccess)
+      return e;
+    nl++;
+  }
+  // 4b. MIXED: support stability and the phase switch
+  if (b.mixed) {
+    if ((e = mark(8)) != cudaSuccess) return e;
+    if ((e = launch_step(support_kernel, b.k, 256, 0, st, b.vmask, b.vmask_prev, M.ldn / 32,
+                         b.stable, b.phase, b.k_stable, b.need_stable, b.ctl)) != cudaSuccess)
+      return e;
+    nl++;
+  }
+  // 5. finalize
+  if (!finish) {
+    if ((e = mark(4)) != cudaSuccess) return e;
+    if ((e = launch_step(finalize_kernel, (b.k + 7) / 8, 256, 0, st, fa)) != cudaSuccess) return e;
+    nl++;
+  }
   if (ev && (e = cudaEventRecord(ev[nl], st)) != cudaSuccess) return e;
   if (launches) *launches = nl;
   return cudaSuccess;
@@ -3082,10 +3144,8 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
   cudaError_t e;
   const int f = p.formulation;
   const bool centred = S.means || S.row_means;
-  if ((e = cudaMemsetAsync(b.max_err, 0, sizeof(float), st))) return e;
   // 1. Z = (B - 1 mu^T - r 1^T) V: CSR rows against V transposed
   // the centring's sums, and the entries a scatter of the supports would touch
-  if ((e = cudaMemsetAsync(b.work, 0, sizeof(unsigned long long), st))) return e;
   sp_vstats_kernel<<<b.k, SP_THREADS, 0, st>>>(b.Vx, b.vmask, b.ldn, S.n, S.means,
                                                centred ? b.sum_v : nullptr, b.dot_mu, S.col_ptr,
                                                b.work, b.ctl);
@@ -3100,7 +3160,7 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
   sp_zgate_kernel<<<1, 1, 0, st>>>(
       b.max_nnz, (uint32_t)SP_SCATTER_CAP, b.work,
       S.comps > 0 ? -1.0 : SP_SCATTER_PER_STEP * (double)S.nnz * (double)(b.kp / 32), b.zgate,
-      b.ctl);
+      b.max_err, b.ctl);
   sp_transpose_v_kernel<<<dim3((S.n + SP_TILE - 1) / SP_TILE, (b.kp + SP_WIDE - 1) / SP_WIDE),
                           SP_THREADS, 0, st>>>(b.Vx, b.vmask, b.ldn, S.n, b.k, b.Vt, b.kp,
                                                b.xmask, b.ctl, b.zgate, 1u, S.defl, S.comps,
@@ -3125,33 +3185,6 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
                                                     b.ctl);
   if ((e = cudaGetLastError())) return e;
   // 4. thresholds: the dense path's selects (own candidate gather), or the penalties
-  if (is_constrained(f)) {
-    if (!is_l1_constrained(f)) {
-      hard_select_kernel<<<b.k, HARD_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, p.constraint, b.Vx,
-                                                        b.nnz, b.status, b.vmask, b.sel_hint,
-                                                        b.ctl, nullptr);
-    } else if (p.l1_mode == 0) {
-      if ((e = kernel_setup(soft_select_kernel<false>, SOFT_SMEM, false))) return e;
-      soft_select_kernel<false><<<b.k, SOFT_THREADS, SOFT_SMEM, st>>>(
-          b.Vraw, b.ldn, S.n, p.constraint, b.Vx, b.nnz, b.status, b.vmask, b.sel_hint, b.ctl,
-          nullptr);
-    } else {
-      if ((e = kernel_setup(soft_select_kernel<true>, SOFT_SMEM, false))) return e;
-      soft_select_kernel<true><<<b.k, SOFT_THREADS, SOFT_SMEM, st>>>(
-          b.Vraw, b.ldn, S.n, p.constraint, b.Vx, b.nnz, b.status, b.vmask, b.sel_hint, b.ctl,
-          nullptr);
-    }
-  } else if (is_l1_penalized(f)) {
-    sp_penalty_kernel<true><<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, (float)p.penalty,
-                                                        b.Vx, b.vmask, b.obj_part, b.nnz_part,
-                                                        b.ctl);
-  } else {
-    sp_penalty_kernel<false><<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, (float)p.penalty,
-                                                         b.Vx, b.vmask, b.obj_part, b.nnz_part,
-                                                         b.ctl);
-  }
-  if ((e = cudaGetLastError())) return e;
-  // 5. objective, change, logs and the batch loop's termination test
   FinalizeArgs fa;
   fa.k = b.k;
   fa.formulation = f;
@@ -3170,12 +3203,28 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
   fa.max_err = b.max_err;
   fa.iters = b.iters;
   fa.cards = b.cards;
+  fa.next_nnz = b.ctl + CTL_NEXT_NNZ;
   fa.max_nnz = b.max_nnz;
+  fa.planes_nnz = nullptr;
   fa.ctl = b.ctl;
+  fa.host_stop = p.host_stop;
   fa.phase = nullptr;
   fa.status = b.status;
   fa.stop_check = p.stop_check;
-  if ((e = cudaMemsetAsync(b.max_nnz, 0, sizeof(uint32_t), st))) return e;
+  if (is_constrained(f)) {
+    return launch_select(f, p, b.k, b.Vraw, b.ldn, S.n, b.Vx, b.nnz, b.vmask, b.sel_hint, nullptr,
+                         fa, true, st);
+  } else if (is_l1_penalized(f)) {
+    sp_penalty_kernel<true><<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, (float)p.penalty,
+                                                        b.Vx, b.vmask, b.obj_part, b.nnz_part,
+                                                        b.ctl);
+  } else {
+    sp_penalty_kernel<false><<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, (float)p.penalty,
+                                                         b.Vx, b.vmask, b.obj_part, b.nnz_part,
+                                                         b.ctl);
+  }
+  if ((e = cudaGetLastError())) return e;
+  // 5. objective, change, logs and the batch loop's termination test
   finalize_kernel<<<(b.k + 7) / 8, 256, 0, st>>>(fa);
   return cudaGetLastError();
 }

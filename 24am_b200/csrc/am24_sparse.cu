@@ -304,6 +304,7 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   if (S.comps) AM24_TRY(A.get(&b.defl_a, (size_t)k * SP_DEFL_MAX));
   // what a step could see before it is written starts defined: pool memory can
   // hold an earlier call's state
+  AM24_CUDA(cudaMemsetAsync(b.work, 0, sizeof(unsigned long long), h->stream));
   AM24_CUDA(cudaMemsetAsync(b.fz, 0, sizeof(float) * k, h->stream));
   AM24_CUDA(cudaMemsetAsync(b.obj_part, 0, sizeof(float) * k, h->stream));
   AM24_CUDA(cudaMemsetAsync(b.nnz_part, 0, sizeof(float) * k, h->stream));
@@ -356,16 +357,21 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
     AM24_CUDA(launch_reset_batch(k, b.sel_hint, b.val, b.err, b.max_nnz, nullptr, b.ctl,
                                  h->stream));
     AM24_CUDA(cudaEventRecord(e0, h->stream));
-    // the batch loop: finalize sets the stop word after the step the
-    // reference's loop ends on; the host reads it after each step
+    // the batch loop: the step's end sets the stop word after the step the
+    // reference's loop ends on; the host looks at it AHEAD steps behind, and the
+    // steps queued past it return at once
+    constexpr int AHEAD = am24_handle_s::AHEAD;
     for (int it = 0; it < s.max_iter; it++) {
       StepParams p = step_params(s, it, (int)shift);
       p.stop_check = 1;
+      p.host_stop = &h->flags[it % AHEAD];
       AM24_CUDA(launch_sparse_step(S, b, p, h->stream));
-      AM24_CUDA(cudaMemcpyAsync(&h->flags[0], b.ctl + CTL_STOP, sizeof(uint32_t),
-                                cudaMemcpyDeviceToHost, h->stream));
-      AM24_CUDA(cudaStreamSynchronize(h->stream));
-      if (h->flags[0]) break;
+      AM24_CUDA(cudaEventRecord(h->run_ev[it % AHEAD], h->stream));
+      const int probe = it - (AHEAD - 1);
+      if (probe >= 0) {
+        AM24_CUDA(cudaEventSynchronize(h->run_ev[probe % AHEAD]));
+        if (h->flags[probe % AHEAD]) break;
+      }
     }
     AM24_CUDA(cudaEventRecord(e1, h->stream));
     uint32_t c[CTL_WORDS];

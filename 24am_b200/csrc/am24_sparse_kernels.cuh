@@ -399,10 +399,12 @@ __global__ void __launch_bounds__(SP_THREADS) sp_vstats_kernel(
 // 4.9 against 1.4.
 constexpr double SP_SCATTER_PER_STEP = 0.25;
 __global__ void sp_zgate_kernel(const uint32_t *max_nnz, uint32_t cap,
-                                const unsigned long long *work, double csr_steps,
-                                uint32_t *zgate, const uint32_t *stop) {
+                                unsigned long long *work, double csr_steps, uint32_t *zgate,
+                                float *max_err, const uint32_t *stop) {
   if (*stop) return;
   *zgate = (*max_nnz <= cap && (double)*work < csr_steps) ? 0u : 1u;
+  *work = 0ull;  // for the next step's count
+  *max_err = 0.f;
 }
 
 // Per start j (one block), on z = Zs[j] after the centred product:

@@ -248,6 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  pdl_enter();
   if ((shape.stop && *shape.stop) ||
       (shape.gate && (*shape.gate < shape.gate_min || *shape.gate > shape.gate_max)))
     return;  // uniform over the grid

@@ -171,6 +171,16 @@ __device__ __forceinline__ uint64_t sdesc_kmajor(uint32_t smem_addr, uint32_t sb
   return d;
 }
 
+// ---------------------------------------------------------------- launches
+// First statement of a kernel launched with programmatic stream serialization:
+// waits until the kernel before it in the stream has completed and its writes
+// are visible, then lets the next one be set up.  Every thread of every such
+// kernel passes here before it returns, so completion carries along the chain.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---------------------------------------------------------------- clusters
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -364,21 +364,19 @@ void host_starts(const am24_settings &s, unsigned n, const float *start_points,
   }
 }
 
+// `cols` starting points (n x cols host floats, one after another) become the
+// loadings of the batch's starts slots[0..cols): one copy into Vraw (raw GEMM
+// output, free between steps) and one kernel.  slots_dev: room for cols ints.
 am24_status upload_columns(am24_handle h, am24_batch b, const float *host, int cols,
-                           const int *slots) {
+                           const int *slots, int *slots_dev) {
   const MatrixDev &M = b->mat->d;
-  // stage through Vraw (raw GEMM output, free between steps), then split
-  for (int c = 0; c < cols; c++) {
-    AM24_CUDA(cudaMemcpyAsync(b->d.Vraw + (size_t)slots[c] * M.ldn, host + (size_t)c * M.n,
-                              sizeof(float) * M.n, cudaMemcpyHostToDevice, h->stream));
-    AM24_CUDA(launch_load_columns(b->d.Vraw + (size_t)slots[c] * M.ldn, M.ldn, M.n, 1,
-                                  b->d.Vx + (size_t)slots[c] * M.ldn, M.ldn,
-                                  b->d.vmask + (size_t)slots[c] * (M.ldn / 32), h->stream));
-    AM24_CUDA(cudaMemsetAsync(b->d.sel_hint + slots[c], 0, sizeof(float), h->stream));
-  }
-  // new starts are dense: the next Z = B V runs on the tensor cores
-  AM24_CUDA(cudaMemsetAsync(b->d.max_nnz, 0xFF, sizeof(uint32_t), h->stream));
-  AM24_CUDA(cudaMemsetAsync(b->d.planes_nnz, 0, sizeof(uint32_t), h->stream));  // stale planes
+  const BatchDev &d = b->d;
+  AM24_CUDA(cudaMemcpyAsync(slots_dev, slots, sizeof(int) * cols, cudaMemcpyHostToDevice,
+                            h->stream));
+  AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, host, sizeof(float) * M.n,
+                              sizeof(float) * M.n, cols, cudaMemcpyHostToDevice, h->stream));
+  AM24_CUDA(launch_load_slots(d.Vraw, M.ldn, M.n, cols, slots_dev, d.Vx, M.ldn, d.vmask, d.sel_hint,
+                              d.val, d.max_nnz, d.planes_nnz, h->stream));
   return AM24_OK;
 }
 
@@ -787,7 +785,7 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
       (st = A.get(&d.ws, d.ws_len)) ||
       (st = A.get(&d.fz, k)) || (st = A.get(&d.obj_part, (size_t)k * parts)) ||
       (st = A.get(&d.nnz_part, (size_t)k * parts)) || (st = A.get(&d.nnz, k)) ||
-      (st = A.get(&d.val, k)) || (st = A.get(&d.err, k)) || (st = A.get(&d.max_err, 1)) ||
+      (st = A.get(&d.val, 2 * (size_t)k)) || (st = A.get(&d.max_err, 1)) ||
       (st = A.get(&d.iters, d.log_capacity)) || (st = A.get(&d.cards, d.log_capacity)) ||
       (st = A.get(&d.status, 1)) || (st = A.get(&d.vmask, (size_t)k * (M.ldn / 32))) ||
       (st = A.get(&d.max_nnz, 1)) || (st = A.get(&d.planes_nnz, 1)) ||
@@ -804,6 +802,7 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
     delete b;
     return st;
   }
+  d.err = d.val + k;  // one copy reads both
   // What a step or a read could see before it is written starts zeroed.  The
   // planes need no initial contents: Vx is defined where vmask is set, every
   // operand plane is written whole before its product, and nothing past n (m)
@@ -1195,9 +1194,20 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
       gidx[j] = j;
       slots[j] = j;
     }
-    host_starts(s, n, start_points, gidx.data(), bs, staging);
-    AM24_TRY(upload_columns(h, b, staging.data(), bs, slots.data()));
-    AM24_CUDA(cudaMemsetAsync(d.val, 0, sizeof(float) * bs, h->stream));
+    int *slots_dev = nullptr;
+    AM24_TRY(local.get(&slots_dev, bs));
+    // starts are handed out in order of their global index, so the next `cols`
+    // of them lie one after another in the caller's matrix
+    auto refill = [&](int cols) -> am24_status {
+      const float *src = start_points ? start_points + (size_t)gidx[0] * n : nullptr;
+      if (s.start_mode != AM24_START_INJECTED) {
+        host_starts(s, n, start_points, gidx.data(), cols, staging);
+        src = staging.data();
+      }
+      return upload_columns(h, b, src, cols, slots.data(), slots_dev);
+    };
+    AM24_TRY(refill(bs));
+    std::vector<float> val_err(2 * (size_t)bs);
     unsigned generated = (unsigned)bs;
     bool go = true;
     // MIXED: one BF16 phase for the whole run (starts refilled after the switch
@@ -1209,17 +1219,19 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
       total_it++;
       const bool refined = phase != 0;
       low_its += refined ? 0 : 1;
-      const StepParams p = step_params(s, 0, 0);
+      StepParams p = step_params(s, 0, 0);
+      p.host_stop = h->flags;
       AM24_CUDA(launch_am_step(M, b->d, b->tm, p, h->stream, &b->launches));
-      AM24_CUDA(cudaMemcpyAsync(err.data(), d.err, sizeof(float) * bs, cudaMemcpyDeviceToHost,
-                                h->stream));
-      AM24_CUDA(cudaMemcpyAsync(val.data(), d.val, sizeof(float) * bs, cudaMemcpyDeviceToHost,
-                                h->stream));
+      AM24_CUDA(cudaMemcpyAsync(val_err.data(), d.val, sizeof(float) * 2 * bs,
+                                cudaMemcpyDeviceToHost, h->stream));  // val, then err
       if (d.mixed)
         AM24_CUDA(cudaMemcpyAsync(&phase, d.phase, sizeof phase, cudaMemcpyDeviceToHost,
                                   h->stream));
       AM24_CUDA(cudaStreamSynchronize(h->stream));
-      AM24_TRY(check_device_status(b));
+      // without a stop_check only a wait that gave up sets the stop word
+      if (h->flags[0]) AM24_TRY(check_device_status(b));
+      std::copy(val_err.begin(), val_err.begin() + bs, val.begin());
+      std::copy(val_err.begin() + bs, val_err.end(), err.begin());
       start_its += (uint64_t)bs;
       go = false;
       int nref = 0;
@@ -1245,10 +1257,7 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
         }
       }
       if (nref > 0) {
-        host_starts(s, n, start_points, gidx.data(), nref, staging);
-        AM24_TRY(upload_columns(h, b, staging.data(), nref, slots.data()));
-        for (int r = 0; r < nref; r++)
-          AM24_CUDA(cudaMemsetAsync(d.val + slots[r], 0, sizeof(float), h->stream));
+        AM24_TRY(refill(nref));
       }
     }
     AM24_CUDA(cudaEventRecord(e1, h->stream));

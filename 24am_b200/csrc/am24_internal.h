@@ -377,6 +377,11 @@ cudaError_t launch_load_columns(const float *src, int ld_src, int rows, int cols
 // global start indices first, first + 1, ... (AM24_START_DEVICE_UNIFORM).
 cudaError_t launch_uniform_starts(float *V, int ld, int rows, int cols, uint32_t first,
                                   uint32_t *mask, cudaStream_t st);
+// Column c of src becomes column slots[c] of dst with its mask, no hint, objective
+// 0; the next step is dense.
+cudaError_t launch_load_slots(const float *src, int ld_src, int rows, int cols, const int *slots,
+                              float *dst, int ld_dst, uint32_t *mask, float *sel_hint, float *val,
+                              uint32_t *max_nnz, uint32_t *planes_nnz, cudaStream_t st);
 cudaError_t launch_reset_batch(int k, float *sel_hint, float *val, float *err, uint32_t *max_nnz,
                                uint32_t *planes_nnz, uint32_t *ctl, cudaStream_t st);
 cudaError_t launch_masked_copy(const float *Vx, const uint32_t *mask, int ld, int rows, int cols,

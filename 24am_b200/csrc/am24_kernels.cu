@@ -414,19 +414,42 @@ __global__ void prep_transpose_kernel(const float *__restrict__ B, int ldB, int 
   }
 }
 
-// One block per column: dst = src (rows entries, zero up to ld_dst) and the
-// column's non-zero bitmask (ld_dst / 32 words).
+// dst = src (rows entries, zero up to ld_dst) and the column's non-zero bitmask
+// (ld_dst / 32 words); whole warps.
+__device__ __forceinline__ void load_column(const float *__restrict__ src, int rows,
+                                            float *__restrict__ dst, int ld_dst,
+                                            uint32_t *__restrict__ mask) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 4
+  for (int base = threadIdx.x & ~31; base < ld_dst; base += blockDim.x) {
+    const int r = base + lane;
+    const float v = (r < rows) ? src[r] : 0.f;
+    dst[r] = v;
+    const unsigned nz = __ballot_sync(FULL, v != 0.f);
+    if (lane == 0) mask[base >> 5] = nz;
+  }
+}
+// One block per column.
 __global__ void load_columns_kernel(const float *__restrict__ src, int ld_src, int rows,
                                     float *__restrict__ dst, int ld_dst,
                                     uint32_t *__restrict__ mask) {
   const size_t c = blockIdx.x;
-  const int lane = threadIdx.x & 31;
-  for (int base = threadIdx.x & ~31; base < ld_dst; base += blockDim.x) {
-    const int r = base + lane;
-    const float v = (r < rows) ? src[c * ld_src + r] : 0.f;
-    dst[c * ld_dst + r] = v;
-    const unsigned nz = __ballot_sync(FULL, v != 0.f);
-    if (lane == 0) mask[c * (ld_dst >> 5) + (base >> 5)] = nz;
+  load_column(src + c * ld_src, rows, dst + c * ld_dst, ld_dst, mask + c * (ld_dst >> 5));
+}
+// Column c into column slots[c], a start that begins anew (launch_load_slots).
+__global__ void load_slots_kernel(const float *__restrict__ src, int ld_src, int rows,
+                                  const int *__restrict__ slots, float *__restrict__ dst,
+                                  int ld_dst, uint32_t *__restrict__ mask, float *sel_hint,
+                                  float *val, uint32_t *max_nnz, uint32_t *planes_nnz) {
+  const size_t c = blockIdx.x, to = slots[c];
+  load_column(src + c * ld_src, rows, dst + to * ld_dst, ld_dst, mask + to * (ld_dst >> 5));
+  if (threadIdx.x == 0) {
+    sel_hint[to] = 0.f;
+    val[to] = 0.f;
+    if (c == 0) {
+      *max_nnz = 0xFFFFFFFFu;
+      *planes_nnz = 0u;
+    }
   }
 }
 
@@ -2607,6 +2630,15 @@ cudaError_t launch_load_columns(const float *src, int ld_src, int rows, int cols
                                 int ld_dst, uint32_t *mask, cudaStream_t st) {
   if (cols <= 0) return cudaSuccess;
   load_columns_kernel<<<cols, 256, 0, st>>>(src, ld_src, rows, dst, ld_dst, mask);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_load_slots(const float *src, int ld_src, int rows, int cols, const int *slots,
+                              float *dst, int ld_dst, uint32_t *mask, float *sel_hint, float *val,
+                              uint32_t *max_nnz, uint32_t *planes_nnz, cudaStream_t st) {
+  if (cols <= 0) return cudaSuccess;
+  load_slots_kernel<<<cols, 1024, 0, st>>>(src, ld_src, rows, slots, dst, ld_dst, mask, sel_hint,
+                                           val, max_nnz, planes_nnz);
   return cudaGetLastError();
 }
 

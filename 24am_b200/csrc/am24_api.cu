@@ -123,54 +123,29 @@ am24_status ensure_tf32_planes(am24_handle h, am24_matrix mat) {
   return AM24_OK;
 }
 
-// The matrix's two scaled FP16 planes of B and their row scales (made once, on
-// first use).
+// The matrix's scaled FP16 planes, two of B and two of B^T, with their row scales
+// (made once, on first use, in one allocation).
 am24_status ensure_fp16_planes(am24_handle h, am24_matrix mat) {
   MatrixDev &M = mat->d;
   if (M.Bc_h2) return AM24_OK;
-  const size_t plane = (size_t)M.n * M.ldm;
-  uint16_t *p = nullptr;
-  float *rs = nullptr;
-  AM24_TRY(mat->mem.get(&p, 2 * plane));
-  AM24_TRY(mat->mem.get(&rs, (size_t)M.n));
-  if (M.ldm > M.m)  // the pad rows of both planes (2n columns)
-    AM24_CUDA(cudaMemset2DAsync(p + M.m, sizeof(uint16_t) * M.ldm, 0,
-                                sizeof(uint16_t) * (M.ldm - M.m), 2 * (size_t)M.n, h->stream));
-  M.Bc_h2 = p;
-  M.row_scale = rs;
-  cudaError_t e = launch_prep_fp16x2(M, h->stream);
+  auto pad = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+  const size_t c_bytes = pad(2 * sizeof(uint16_t) * (size_t)M.n * M.ldm);
+  const size_t t_bytes = pad(2 * sizeof(uint16_t) * (size_t)M.m * M.ldn);
+  const size_t n_bytes = pad(sizeof(float) * M.n), m_bytes = pad(sizeof(float) * M.m);
+  char *p = nullptr;
+  AM24_TRY(mat->mem.get(&p, c_bytes + t_bytes + n_bytes + m_bytes +
+                                sizeof(uint32_t) * ((size_t)M.n + M.m)));
+  M.Bc_h2 = reinterpret_cast<uint16_t *>(p);
+  M.Bt_h2 = reinterpret_cast<uint16_t *>(p + c_bytes);
+  M.row_scale = reinterpret_cast<float *>(p + c_bytes + t_bytes);
+  M.bt_row_scale = reinterpret_cast<float *>(p + c_bytes + t_bytes + n_bytes);
+  M.fp16_keys = reinterpret_cast<uint32_t *>(p + c_bytes + t_bytes + n_bytes + m_bytes);
+  cudaError_t e = launch_prep_fp16(M, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
-    M.Bc_h2 = nullptr;
-    M.row_scale = nullptr;
+    M.Bc_h2 = M.Bt_h2 = nullptr;
+    M.row_scale = M.bt_row_scale = nullptr;
     return fail(AM24_ERR_CUDA, std::string("FP16 planes: ") + cudaGetErrorString(e));
-  }
-  return AM24_OK;
-}
-
-// The matrix's two scaled FP16 planes of B^T and their row scales (made once,
-// on first use).
-am24_status ensure_bt_fp16_planes(am24_handle h, am24_matrix mat) {
-  MatrixDev &M = mat->d;
-  if (M.Bt_h2) return AM24_OK;
-  const size_t plane = (size_t)M.m * M.ldn;
-  uint16_t *p = nullptr;
-  float *rs = nullptr;
-  uint32_t *key = nullptr;
-  AM24_TRY(mat->mem.get(&p, 2 * plane));
-  AM24_TRY(mat->mem.get(&rs, (size_t)M.m));
-  AM24_TRY(mat->mem.get(&key, (size_t)M.m));
-  if (M.ldn > M.n)  // the pad columns of both planes (2m rows)
-    AM24_CUDA(cudaMemset2DAsync(p + M.n, sizeof(uint16_t) * M.ldn, 0,
-                                sizeof(uint16_t) * (M.ldn - M.n), 2 * (size_t)M.m, h->stream));
-  M.Bt_h2 = p;
-  M.bt_row_scale = rs;
-  cudaError_t e = launch_prep_bt_fp16x2(M, key, h->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-  if (e != cudaSuccess) {
-    M.Bt_h2 = nullptr;
-    M.bt_row_scale = nullptr;
-    return fail(AM24_ERR_CUDA, std::string("FP16 planes of B^T: ") + cudaGetErrorString(e));
   }
   return AM24_OK;
 }
@@ -568,17 +543,30 @@ static am24_status create_matrix(am24_handle h, const float *B, int32_t ldB, uin
     delete mat;
     return st;
   }
-  // one 2-D copy straight into Bc's layout (host or device source), pad rows
-  // zeroed; the other layouts are made from Bc when a batch first needs them
+  // one copy straight into Bc's layout, pad rows zeroed: a kernel for a source in
+  // this device's own memory, a 2-D copy otherwise (host, or another device's
+  // memory, which a kernel may not reach); the other layouts are made from Bc when
+  // a batch first needs them
   cudaError_t e = cudaSuccess;
-  if (M.ldm > (int)m)
-    e = cudaMemset2DAsync(M.Bc + m, sizeof(float) * M.ldm, 0, sizeof(float) * (M.ldm - m), n,
-                          h->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpy2DAsync(M.Bc, sizeof(float) * M.ldm, B, sizeof(float) * (size_t)ldB,
-                          sizeof(float) * m, n,
-                          on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
-                          h->stream);
+  bool own = false;
+  if (on_device) {
+    cudaPointerAttributes at;
+    own = cudaPointerGetAttributes(&at, B) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+          at.device == h->device;
+    if (!own) cudaGetLastError();
+  }
+  if (own) {
+    e = launch_copy_matrix(M, B, ldB, h->stream);
+  } else {
+    if (M.ldm > (int)m)
+      e = cudaMemset2DAsync(M.Bc + m, sizeof(float) * M.ldm, 0, sizeof(float) * (M.ldm - m), n,
+                            h->stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpy2DAsync(M.Bc, sizeof(float) * M.ldm, B, sizeof(float) * (size_t)ldB,
+                            sizeof(float) * m, n,
+                            on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                            h->stream);
+  }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
     delete mat;
@@ -666,14 +654,11 @@ am24_status am24_matrix_deflate(am24_handle h, am24_matrix mat, const float *x,
   AM24_CUDA(cudaMemcpyAsync(xd, x, sizeof(float) * M.n,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                             h->stream));
-  AM24_CUDA(launch_deflate(M, xd, partial, y, h->stream));
+  int *bad = nullptr;
+  AM24_TRY(local.get(&bad, 1));
+  AM24_CUDA(launch_deflate(M, xd, partial, y, bad, h->stream));
   // every layout made so far is rebuilt from the new B, in place
-  if (M.Bc_h2) AM24_CUDA(launch_prep_fp16x2(M, h->stream));
-  if (M.Bt_h2) {
-    uint32_t *key = nullptr;
-    AM24_TRY(local.get(&key, (size_t)M.m));
-    AM24_CUDA(launch_prep_bt_fp16x2(M, key, h->stream));
-  }
+  if (M.Bc_h2) AM24_CUDA(launch_prep_fp16(M, h->stream));
   if (M.Bc_hi) AM24_CUDA(launch_prep_tf32_planes(M, h->stream));
   if (M.Bc_b3) AM24_CUDA(launch_prep_bf16x3(M, h->stream));
   AM24_CUDA(cudaStreamSynchronize(h->stream));
@@ -796,7 +781,7 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
       (d.fp16_2 && ((st = A.get(&d.Z_h, zh_planes * kz)) || (st = A.get(&d.z_scale, k)) ||
                     (st = ensure_fp16_planes(h, mat)))) ||
       (d.fp16_1 && ((st = A.get(&d.V_h, 2 * kv)) || (st = A.get(&d.v_scale, k)) ||
-                    (st = ensure_bt_fp16_planes(h, mat)))) ||
+                    (st = ensure_fp16_planes(h, mat)))) ||
       (d.mixed && ((st = A.get(&d.vmask_prev, (size_t)k * (M.ldn / 32))) ||
                    (st = A.get(&d.stable, k)) || (st = A.get(&d.phase, 4))))) {
     delete b;

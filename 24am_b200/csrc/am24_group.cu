@@ -278,7 +278,6 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
   const bool mixed = s.precision == AM24_PRECISION_MIXED;
   const int f = s.formulation;
   AM24_TRY(ensure_fp16_planes(h, mat));
-  AM24_TRY(ensure_bt_fp16_planes(h, mat));
 
   GroupSlot &sl = g->slots[slot];
   GProblem P{};

@@ -126,7 +126,6 @@ am24_status make_map_bf16(am24_handle h, CUtensorMap *map, const uint16_t *base,
 am24_status ensure_bf16_planes(am24_handle h, am24_matrix mat, int planes);
 am24_status ensure_tf32_planes(am24_handle h, am24_matrix mat);
 am24_status ensure_fp16_planes(am24_handle h, am24_matrix mat);
-am24_status ensure_bt_fp16_planes(am24_handle h, am24_matrix mat);
 void choose_splits(int tiles, int kb_total, int sms, int *splits, int *kbps);
 am24_status validate_settings(const am24_settings *s);
 // The phase word a MIXED batch or problem starts in (lead_iterations > 0: the FP32 lead-in).

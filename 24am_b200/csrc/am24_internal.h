@@ -47,6 +47,7 @@ struct MatrixDev {
   // scaled per sample (plane p at Bt_h2 + p * m * ldn), bt_row_scale[i] = 2^-s_i.
   uint16_t *Bt_h2;
   float *bt_row_scale;
+  uint32_t *fp16_keys;  // n + m words: the rows' largest |x| (scratch of launch_prep_fp16)
 };
 
 // Per-batch device state for k starting points.
@@ -364,10 +365,11 @@ bool gather_is_wide(int m);
 cudaError_t launch_prep_tf32_planes(MatrixDev &M, cudaStream_t st);
 // Fills M.Bc_b3 from M.Bc (its M.bf16_planes planes).
 cudaError_t launch_prep_bf16x3(const MatrixDev &M, cudaStream_t st);
-// Fills M.Bc_h2 and M.row_scale from M.Bc.
-cudaError_t launch_prep_fp16x2(const MatrixDev &M, cudaStream_t st);
-// Fills M.Bt_h2 and M.bt_row_scale from M.Bc; key: m words of scratch.
-cudaError_t launch_prep_bt_fp16x2(const MatrixDev &M, uint32_t *key, cudaStream_t st);
+// Fills both pairs of FP16 operand planes and their scales from M.Bc
+// (M.fp16_keys: scratch of n + m words).
+cudaError_t launch_prep_fp16(const MatrixDev &M, cudaStream_t st);
+// M.Bc from B in this device's memory (leading dimension ldB), pad rows zeroed.
+cudaError_t launch_copy_matrix(const MatrixDev &M, const float *B, int ldB, cudaStream_t st);
 // Loadings of `cols` columns from src (rows entries each) into dst and their
 // non-zero masks (mask + c * (ld_dst / 32) per column).
 cudaError_t launch_load_columns(const float *src, int ld_src, int rows, int cols, float *dst,
@@ -403,7 +405,7 @@ cudaError_t launch_csc_to_dense(MatrixDev &M, const float *vals, const int32_t *
                                const float *row_means, cudaStream_t st);
 // B <- B (I - x x^T) on M.Bc (device x; partial: ev_partial_len(M) doubles of
 // scratch, y: m doubles).  The other layouts are not touched.
-cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double *y,
+cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double *y, int *bad,
                            cudaStream_t st);
 // ||B x||^2 in FP64 into *out; partial: ev_partial_len(M) doubles of scratch.
 cudaError_t launch_explained_variance(const MatrixDev &M, const float *x, double *partial,

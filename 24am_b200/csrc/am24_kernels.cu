@@ -330,68 +330,116 @@ __global__ void prep_bf16x3_kernel(const float *__restrict__ Bc, int ldm, int m,
   }
 }
 
-// Two FP16 planes of each feature of B with a power-of-two scale per feature:
-// x * 2^s = h0 + h1 (fp16_split), s from the feature's largest |x| so that it
-// lands in [2^14, 2^15); row_scale[c] = 2^-s undoes it in the GEMM epilogue.
-__global__ void __launch_bounds__(256) prep_fp16x2_kernel(const float *__restrict__ Bc, int ldm,
-                                                          int m, size_t plane,
-                                                          uint16_t *__restrict__ out,
-                                                          float *__restrict__ row_scale) {
-  __shared__ uint32_t red[8];
-  const size_t c = blockIdx.x;
-  uint32_t mx = 0;
-  for (int r = threadIdx.x; r < m; r += blockDim.x) mx = max(mx, abs_key(Bc[c * ldm + r]));
-  mx = __reduce_max_sync(FULL, mx);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
-  __syncthreads();
-  mx = 0;
-#pragma unroll
-  for (int w = 0; w < 8; w++) mx = max(mx, red[w]);
-  const int s = fp16_shift(__uint_as_float(mx));
-  const float sc = pow2f(s);
-  if (threadIdx.x == 0) row_scale[c] = pow2f(-s);
-  for (int r = threadIdx.x; r < m; r += blockDim.x) {
-    const size_t o = c * ldm + r;
-    fp16_split(Bc[o] * sc, out + o, out + plane + o);
-  }
-}
-
-// Per sample i, the largest |B[i, c]| over the features as a key, for the
-// FP16 planes of B^T: blocks of SAMPLE_MAX_CHUNK features, threads over samples
-// (coalesced reads of B's columns), atomicMax into key[i] (zeroed before).
-constexpr int SAMPLE_MAX_CHUNK = 64;
-__global__ void __launch_bounds__(256) sample_max_kernel(const float *__restrict__ Bc, int ldm,
-                                                         int m, int n, uint32_t *__restrict__ key) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= m) return;
-  const int c0 = blockIdx.y * SAMPLE_MAX_CHUNK, c1 = min(n, c0 + SAMPLE_MAX_CHUNK);
-  uint32_t mx = 0;
-  for (int c = c0; c < c1; c++) mx = max(mx, abs_key(Bc[(size_t)c * ldm + i]));
-  atomicMax(key + i, mx);
-}
-
-// As prep_fp16x2_kernel for the rows of B^T: out[i * ldn + c] (second plane at
-// out + plane) split from B[i, c] * 2^s_i, s_i from key[i]; row_scale[i] = 2^-s_i.
-// 32 x 32 tiles through shared memory; columns [n, ldn) are left as they are.
-__global__ void prep_bt_fp16x2_kernel(const float *__restrict__ Bc, int ldm, int m, int n,
-                                      const uint32_t *__restrict__ key, int ldn, size_t plane,
-                                      uint16_t *__restrict__ out, float *__restrict__ row_scale) {
-  __shared__ float tile[32][33];
-  const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;  // features, samples
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const int c = c0 + y, r = r0 + threadIdx.x;
-    tile[y][threadIdx.x] = (c < n && r < m) ? Bc[(size_t)c * ldm + r] : 0.f;
-  }
-  __syncthreads();
-  for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-    const int r = r0 + y, c = c0 + threadIdx.x;
-    if (r >= m) continue;
-    const int s = fp16_shift(__uint_as_float(key[r]));
-    if (c < n) {
-      const size_t o = (size_t)r * ldn + c;
-      fp16_split(tile[threadIdx.x][y] * pow2f(s), out + o, out + plane + o);
+// B (column-major, leading dimension ldB) into Bc's layout, pad rows zeroed;
+// 16 bytes at a time where the source allows it (`vec`).
+__global__ void __launch_bounds__(256) copy_matrix_kernel(const float *__restrict__ B, int ldB,
+                                                          int m, bool vec, float *__restrict__ Bc,
+                                                          int ldm) {
+  const float *src = B + (size_t)blockIdx.x * ldB;
+  float *dst = Bc + (size_t)blockIdx.x * ldm;
+  for (int q = threadIdx.x; q < (ldm >> 2); q += blockDim.x) {
+    const int r = 4 * q;
+    float4 v;
+    if (vec && r + 3 < m) {
+      v = __ldg(reinterpret_cast<const float4 *>(src) + q);
+    } else {
+      v.x = r < m ? src[r] : 0.f;
+      v.y = r + 1 < m ? src[r + 1] : 0.f;
+      v.z = r + 2 < m ? src[r + 2] : 0.f;
+      v.w = r + 3 < m ? src[r + 3] : 0.f;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) row_scale[r] = pow2f(-s);
+    reinterpret_cast<float4 *>(dst)[q] = v;
+  }
+}
+
+// The largest |B[i, c]| as keys, per feature (row_key) and per sample (key),
+// both zeroed before: blocks of 1024 samples x MAX_CHUNK features, four samples
+// per thread.
+constexpr int MAX_CHUNK = 64;
+__global__ void __launch_bounds__(256) matrix_max_kernel(const float *__restrict__ Bc, int ldm,
+                                                         int m, int n,
+                                                         uint32_t *__restrict__ row_key,
+                                                         uint32_t *__restrict__ key) {
+  __shared__ uint32_t fmax[8][MAX_CHUNK];  // per warp
+  const int warp = threadIdx.x >> 5;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool on = q < (ldm >> 2);
+  const size_t ld4 = (size_t)ldm >> 2;
+  const int c0 = blockIdx.y * MAX_CHUNK, cn = min(n - c0, MAX_CHUNK);
+  const float4 *B4 = reinterpret_cast<const float4 *>(Bc) + (size_t)c0 * ld4 + (on ? q : 0);
+  uint32_t mx[4] = {0u, 0u, 0u, 0u};
+#pragma unroll 8
+  for (int c = 0; c < cn; c++) {
+    const float4 v = __ldg(B4 + c * ld4);  // off threads repeat the first quad
+    const uint32_t k[4] = {abs_key(v.x), abs_key(v.y), abs_key(v.z), abs_key(v.w)};
+#pragma unroll
+    for (int e = 0; e < 4; e++) mx[e] = max(mx[e], k[e]);
+    const uint32_t f = __reduce_max_sync(FULL, max(max(k[0], k[1]), max(k[2], k[3])));
+    if ((threadIdx.x & 31) == 0) fmax[warp][c] = f;
+  }
+  if (on)
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (4 * q + e < m) atomicMax(key + 4 * q + e, mx[e]);
+  __syncthreads();
+  if (threadIdx.x < cn) {
+    uint32_t f = 0;
+#pragma unroll
+    for (int w = 0; w < 8; w++) f = max(f, fmax[w][threadIdx.x]);
+    atomicMax(row_key + c0 + threadIdx.x, f);
+  }
+}
+
+// The FP16 operand planes of B (rows = features) and of B^T (rows = samples),
+// each row with its power-of-two scale from its largest |x|:
+// x * 2^s = h0 + h1 (fp16_split), second plane at + plane; scale[row] = 2^-s
+// undoes it in the GEMM epilogue.  64 x 64 tiles through shared memory, B read
+// once for both, 8-byte stores.  HBM bound: 1000 x 20000 in 40 us (240 MB), with
+// matrix_max_kernel 66; a pass per orientation and one for the samples' maxima
+// took 180.
+__global__ void __launch_bounds__(256) split_matrix_kernel(
+    const float *__restrict__ Bc, int ldm, int m, int n, int ldn,
+    const uint32_t *__restrict__ row_key, const uint32_t *__restrict__ key,
+    uint16_t *__restrict__ Ch, size_t cplane, float *__restrict__ row_scale,
+    uint16_t *__restrict__ Th, size_t tplane, float *__restrict__ bt_row_scale) {
+  __shared__ float tile[64][65];
+  const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;  // features, samples
+  const int q = threadIdx.x & 15, row = threadIdx.x >> 4;
+  auto put = [](const float (&v)[4], float sc, uint16_t *out, size_t plane) {
+    uint16_t a[4], b[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) fp16_split(v[e] * sc, &a[e], &b[e]);
+    *reinterpret_cast<uint2 *>(out) =
+        make_uint2(a[0] | ((uint32_t)a[1] << 16), a[2] | ((uint32_t)a[3] << 16));
+    *reinterpret_cast<uint2 *>(out + plane) =
+        make_uint2(b[0] | ((uint32_t)b[1] << 16), b[2] | ((uint32_t)b[3] << 16));
+  };
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int f = row + 16 * i, c = c0 + f, r = r0 + 4 * q;
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (c < n && r < ldm) {  // rows in [m, ldm) are zeros
+      const float4 x = __ldg(reinterpret_cast<const float4 *>(Bc + (size_t)c * ldm + r));
+      v[0] = x.x;
+      v[1] = x.y;
+      v[2] = x.z;
+      v[3] = x.w;
+      const int s = fp16_shift(__uint_as_float(row_key[c]));
+      put(v, pow2f(s), Ch + (size_t)c * ldm + r, cplane);
+      if (r == 0) row_scale[c] = pow2f(-s);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++) tile[f][4 * q + e] = v[e];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int t = row + 16 * i, r = r0 + t, c = c0 + 4 * q;
+    if (r >= m || c >= ldn) continue;  // columns in [n, ldn) take zeros
+    const float v[4] = {tile[4 * q][t], tile[4 * q + 1][t], tile[4 * q + 2][t], tile[4 * q + 3][t]};
+    const int s = fp16_shift(__uint_as_float(key[r]));
+    put(v, pow2f(s), Th + (size_t)r * ldn + c, tplane);
+    if (c == 0) bt_row_scale[r] = pow2f(-s);
   }
 }
 
@@ -2402,22 +2450,29 @@ __global__ void center_kernel(float *__restrict__ Bc, int ldm, int m,
 }
 
 // y_i = the sum of its chunks' partials (in chunk order), FP64.
+// *bad (may be null) is set when some y_i is not finite.
 __global__ void rowsum_kernel(const double *__restrict__ partial, int chunks, int m,
-                              double *__restrict__ y) {
+                              double *__restrict__ y, int *bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   double acc = 0.0;
 #pragma unroll 8
   for (int c = 0; c < chunks; c++) acc += partial[(size_t)c * m + i];
   y[i] = acc;
+  if (bad && !isfinite(acc)) *bad = 1;
 }
 
 // Deflation B <- B (I - x x^T) = B - y x^T with y = B x: every entry in FP64,
-// rounded to FP32 once.  One block per feature, threads over samples.
+// rounded to FP32 once.  One block per feature, threads over samples.  Features
+// with x_c = 0 keep their values (unless y is not finite: 0 y_i is NaN then), and
+// a sparse component leaves most of them: 1000 x 20000 in 13 us, 52 with every
+// feature rewritten.
 __global__ void deflate_kernel(float *__restrict__ Bc, int ldm, int m,
-                               const double *__restrict__ y, const float *__restrict__ x) {
+                               const double *__restrict__ y, const float *__restrict__ x,
+                               const int *__restrict__ bad) {
   const size_t c = blockIdx.x;
   const double xc = (double)x[c];
+  if (xc == 0.0 && !*bad) return;
   for (int i = threadIdx.x; i < m; i += blockDim.x) {
     const size_t o = c * ldm + i;
     Bc[o] = (float)((double)Bc[o] - y[i] * xc);
@@ -2599,20 +2654,22 @@ cudaError_t launch_prep_bf16x3(const MatrixDev &M, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t launch_prep_fp16x2(const MatrixDev &M, cudaStream_t st) {
-  prep_fp16x2_kernel<<<M.n, 256, 0, st>>>(M.Bc, M.ldm, M.m, (size_t)M.n * M.ldm, M.Bc_h2,
-                                          M.row_scale);
+cudaError_t launch_copy_matrix(const MatrixDev &M, const float *B, int ldB, cudaStream_t st) {
+  const bool vec = ldB % 4 == 0 && reinterpret_cast<uintptr_t>(B) % 16 == 0;
+  copy_matrix_kernel<<<M.n, 256, 0, st>>>(B, ldB, M.m, vec, M.Bc, M.ldm);
   return cudaGetLastError();
 }
 
-cudaError_t launch_prep_bt_fp16x2(const MatrixDev &M, uint32_t *key, cudaStream_t st) {
-  cudaError_t e = cudaMemsetAsync(key, 0, sizeof(uint32_t) * M.m, st);
+cudaError_t launch_prep_fp16(const MatrixDev &M, cudaStream_t st) {
+  uint32_t *row_key = M.fp16_keys, *key = M.fp16_keys + M.n;
+  cudaError_t e = cudaMemsetAsync(M.fp16_keys, 0, sizeof(uint32_t) * ((size_t)M.n + M.m), st);
   if (e != cudaSuccess) return e;
-  sample_max_kernel<<<dim3((M.m + 255) / 256, (M.n + SAMPLE_MAX_CHUNK - 1) / SAMPLE_MAX_CHUNK),
-                      256, 0, st>>>(M.Bc, M.ldm, M.m, M.n, key);
+  matrix_max_kernel<<<dim3((M.ldm / 4 + 255) / 256, (M.n + MAX_CHUNK - 1) / MAX_CHUNK), 256, 0,
+                      st>>>(M.Bc, M.ldm, M.m, M.n, row_key, key);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  prep_bt_fp16x2_kernel<<<dim3((M.n + 31) / 32, (M.m + 31) / 32), dim3(32, 8), 0, st>>>(
-      M.Bc, M.ldm, M.m, M.n, key, M.ldn, (size_t)M.m * M.ldn, M.Bt_h2, M.bt_row_scale);
+  split_matrix_kernel<<<dim3((M.n + 63) / 64, (M.ldm + 63) / 64), 256, 0, st>>>(
+      M.Bc, M.ldm, M.m, M.n, M.ldn, row_key, key, M.Bc_h2, (size_t)M.n * M.ldm, M.row_scale,
+      M.Bt_h2, (size_t)M.m * M.ldn, M.bt_row_scale);
   return cudaGetLastError();
 }
 
@@ -2777,7 +2834,7 @@ cudaError_t launch_explained_variance(const MatrixDev &M, const float *x, double
   ev_partial_kernel<<<dim3((M.m + 255) / 256, chunks), 256, 0, st>>>(M.Bc, M.ldm, M.m, M.n, x,
                                                                      partial);
   double *y = partial + (size_t)chunks * M.m;
-  rowsum_kernel<<<(M.m + 127) / 128, 128, 0, st>>>(partial, chunks, M.m, y);
+  rowsum_kernel<<<(M.m + 127) / 128, 128, 0, st>>>(partial, chunks, M.m, y, nullptr);
   ev_norm_kernel<<<1, 1024, 0, st>>>(y, M.m, out);
   return cudaGetLastError();
 }
@@ -2792,16 +2849,17 @@ cudaError_t launch_csc_to_dense(MatrixDev &M, const float *vals, const int32_t *
   return cudaGetLastError();
 }
 
-cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double *y,
+cudaError_t launch_deflate(MatrixDev &M, const float *x, double *partial, double *y, int *bad,
                            cudaStream_t st) {
   const int chunks = (M.n + EV_CHUNK - 1) / EV_CHUNK;
   ev_partial_kernel<<<dim3((M.m + 255) / 256, chunks), 256, 0, st>>>(M.Bc, M.ldm, M.m, M.n, x,
                                                                      partial);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  rowsum_kernel<<<(M.m + 255) / 256, 256, 0, st>>>(partial, chunks, M.m, y);
+  if ((e = cudaMemsetAsync(bad, 0, sizeof(int), st)) != cudaSuccess) return e;
+  rowsum_kernel<<<(M.m + 255) / 256, 256, 0, st>>>(partial, chunks, M.m, y, bad);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  deflate_kernel<<<M.n, 256, 0, st>>>(M.Bc, M.ldm, M.m, y, x);
+  deflate_kernel<<<M.n, 256, 0, st>>>(M.Bc, M.ldm, M.m, y, x, bad);
   return cudaGetLastError();
 }
 

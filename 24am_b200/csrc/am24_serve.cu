@@ -276,7 +276,6 @@ am24_status am24_server_add_matrix_f32(am24_server s, const float *B, int32_t ld
     std::lock_guard<std::mutex> lk(s->upload_mu);
     st = am24_matrix_create_f32(s->upload_h, B, ldB, m, n, on_device, &mat);
     if (st == AM24_OK) st = ensure_fp16_planes(s->upload_h, mat);
-    if (st == AM24_OK) st = ensure_bt_fp16_planes(s->upload_h, mat);
     if (st != AM24_OK && mat) {
       const std::string err = g_last_error;
       am24_matrix_destroy(s->upload_h, mat);

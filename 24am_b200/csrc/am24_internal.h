@@ -270,6 +270,7 @@ struct GroupDev {
   int *pref;  // [GL_COUNT][cap + 1]: exclusive prefix of their items
   uint32_t *done;  // per slot after each step: 0 free, 1 iterating, 2 stopped
   const int *order;  // [cap]: the slots in the order the plan lists them (widest first)
+  int *active;       // [cap]: this step's active slots in that order (plan scratch)
   unsigned long long timeout_ns;
 };
 
@@ -279,7 +280,13 @@ struct GroupGrids {
   int plan_threads, col, select_hard, select_soft, gather, gather_tile, fin, pairs;
 };
 cudaError_t grouped_grids(GroupGrids *g);
-cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &grids, cudaStream_t st);
+// The streams and events of a step's branches.
+struct GroupStreams {
+  cudaStream_t side[3] = {};
+  cudaEvent_t ev[7] = {};
+};
+cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &grids, const GroupStreams &q,
+                                cudaStream_t st);
 // Sets the WHILE condition of a captured loop: 1 while some problem is live and
 // unstopped, the plan's loop count is below its cap and no wait gave up.
 cudaError_t launch_grouped_condition(const GroupDev &g, unsigned long long handle,

@@ -3123,17 +3123,17 @@ cudaError_t launch_grouped_gemm(const GroupDev &g, int list, cudaStream_t st) {
   const cudaError_t e = grouped_gemm_setup<BN, EPI>(&clusters);
   if (e != cudaSuccess) return e;
   gemm_pair_grouped_kernel<BN, EPI>
-      <<<2 * clusters, GEMM_THREADS, GPairSmem<BN>::TOTAL, st>>>(g, list);
+      <<<2 * clusters, PairEpi<BN>::THREADS, GPairSmem<BN>::TOTAL, st>>>(g, list);
   return cudaGetLastError();
 }
 
-// The three N tiles of one epilogue, lists l64, l64 + 1, l64 + 2.
+// The three N tiles of one epilogue, lists l64, l64 + 1, l64 + 2; the widest first.
 template <int EPI>
 cudaError_t launch_grouped_gemms(const GroupDev &g, int l64, cudaStream_t st) {
   cudaError_t e;
-  if ((e = launch_grouped_gemm<64, EPI>(g, l64, st)) ||
+  if ((e = launch_grouped_gemm<256, EPI>(g, l64 + 2, st)) ||
       (e = launch_grouped_gemm<128, EPI>(g, l64 + 1, st)) ||
-      (e = launch_grouped_gemm<256, EPI>(g, l64 + 2, st)))
+      (e = launch_grouped_gemm<64, EPI>(g, l64, st)))
     return e;
   return cudaSuccess;
 }
@@ -3170,27 +3170,44 @@ cudaError_t grouped_grids(GroupGrids *gr) {
   return cudaSuccess;
 }
 
-cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &gr, cudaStream_t st) {
+// The parts of a step that do not depend on one another run as branches (side
+// streams of the capture): the sparse gathers beside the dense product, the three
+// epilogues of V = B^T Z beside each other, the selects beside the penalties'
+// products.  Every one is persistent and ends with a tail of its last units, which
+// the next branch's blocks fill: HOLD_BRANCH
+cudaError_t launch_grouped_step(const GroupDev &g, const GroupGrids &gr, const GroupStreams &q,
+                                cudaStream_t st) {
   cudaError_t e;
+  auto after = [&](cudaStream_t to, int ev, cudaStream_t from) -> cudaError_t {
+    const cudaError_t r = cudaEventRecord(q.ev[ev], from);
+    return r ? r : cudaStreamWaitEvent(to, q.ev[ev], 0);
+  };
   group_plan_kernel<<<1, PLAN_THREADS, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
-  // Z = B V: the sparse gathers, or the dense path
-  g_gather_narrow_kernel<<<gr.gather, GATHER_THREADS, 0, st>>>(g);
-  g_gather_list_kernel<<<gr.col, GATHER_THREADS, 0, st>>>(g);
-  g_gather_tile_kernel<<<gr.gather_tile, GATHER_THREADS, 0, st>>>(g);
+  // Z = B V: the sparse gathers, and the dense path
+  if ((e = after(q.side[0], 0, st))) return e;
+  g_gather_list_kernel<<<gr.col, GATHER_THREADS, 0, q.side[0]>>>(g);
+  g_gather_tile_kernel<<<gr.gather_tile, GATHER_THREADS, 0, q.side[0]>>>(g);
+  g_gather_narrow_kernel<<<gr.gather, GATHER_THREADS, 0, q.side[0]>>>(g);
   g_densify_kernel<<<DENSIFY_BLOCKS_PER_SM * num_sms(), DENSIFY_THREADS, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
   if ((e = launch_grouped_gemms<GE_PARTIAL>(g, GL_GEMM1_64, st))) return e;
+  if ((e = after(st, 1, q.side[0]))) return e;
   g_z_reduce_kernel<<<gr.col, 256, 0, st>>>(g);
   if ((e = cudaGetLastError())) return e;
-  // V = B^T Z with the penalty fused or the raw output marked for the selects
-  if ((e = launch_grouped_gemms<GE_RAW>(g, GL_RAW_64, st)) ||
-      (e = launch_grouped_gemms<GE_PL1>(g, GL_PL1_64, st)) ||
-      (e = launch_grouped_gemms<GE_PL0>(g, GL_PL0_64, st)))
+  // V = B^T Z with the raw output marked for the selects or the penalty fused
+  if ((e = after(q.side[0], 2, st)) || (e = cudaStreamWaitEvent(q.side[1], q.ev[2], 0)) ||
+      (e = launch_grouped_gemms<GE_RAW>(g, GL_RAW_64, st)) ||
+      (e = launch_grouped_gemms<GE_PL0>(g, GL_PL0_64, q.side[0])) ||
+      (e = launch_grouped_gemms<GE_PL1>(g, GL_PL1_64, q.side[1])) ||
+      (e = after(q.side[2], 3, st)))
     return e;
-  g_hard_select_kernel<<<gr.select_hard, HARD_THREADS, 0, st>>>(g);
   g_soft_select_kernel<false><<<gr.select_soft, SOFT_THREADS, SOFT_SMEM, st>>>(g);
   g_soft_select_kernel<true><<<gr.select_soft, SOFT_THREADS, SOFT_SMEM, st>>>(g);
+  g_hard_select_kernel<<<gr.select_hard, HARD_THREADS, 0, q.side[2]>>>(g);
+  if ((e = cudaGetLastError()) || (e = after(st, 4, q.side[0])) || (e = after(st, 5, q.side[1])) ||
+      (e = after(st, 6, q.side[2])))
+    return e;
   g_support_kernel<<<gr.col, 256, 0, st>>>(g);
   g_finalize_kernel<<<gr.fin, 256, 0, st>>>(g);
   return cudaGetLastError();

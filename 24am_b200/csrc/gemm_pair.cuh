@@ -30,7 +30,7 @@
 // MMA accumulations in both schemes) and the epilogue warps add it into
 // round-to-nearest FP32 registers.
 //
-// Roles are the one-CTA kernel's (warp 0 TMA, warp 1 MMA, warps 2..9
+// Roles are the one-CTA kernel's (warp 0 TMA, warp 1 MMA, the other warps
 // accumulate + epilogue), with the MMA warp active in the leader only.
 // Barriers sit at the same shared-memory offsets in both CTAs:
 //   full[s]   used in the leader: armed there with both CTAs' bytes; the TMA
@@ -216,10 +216,24 @@ struct PairSmem {
   static constexpr int TOTAL = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
 };
 
-constexpr int PAIR_EPI_WARPS = 2 * (GEMM_EPI_THREADS / 32);  // tempty arrivals per phase
+// The epilogue warps of a pair kernel: four per 32-lane quarter of tensor memory
+// (two for the narrowest tile), each with BN / PARTS columns of its 32 rows.  With
+// two per quarter the epilogue's instructions ran one per 7.5 cycles and warp, two
+// warps a scheduler.  With four, and tensor memory read 16 columns at a time (112
+// registers a thread in place of 168): 202 x 33654, 1005 starts 122 -> 100 us a
+// launch with the L1 penalty, 90 -> 62 with raw output; 2000 x 50000, 1024 starts
+// 430 -> 405.
+template <int BN>
+struct PairEpi {
+  static constexpr int PARTS = BN >= 128 ? 4 : 2;
+  static constexpr int COLS = BN / PARTS;
+  static constexpr int WARPS = 4 * PARTS;
+  static constexpr int THREADS = 64 + 32 * WARPS;
+  static constexpr int ARRIVALS = 2 * WARPS;  // of both CTAs, per tempty phase
+};
 
 template <class S, int BN, int STAGES, int PROMO, class Epi>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairEpi<BN>::THREADS, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap tm0,
                      const __grid_constant__ CUtensorMap tm1,
                      const __grid_constant__ CUtensorMap tm2,
@@ -263,7 +277,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
     for (int a = 0; a < 2; a++) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], PAIR_EPI_WARPS);
+      mbar_init(&tempty[a], PairEpi<BN>::ARRIVALS);
     }
     mbar_init(drain, 1);
     *abort = 0;
@@ -395,9 +409,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
   } else {
     // ------------------------------------------------------------ accumulate + epilogue (both)
-    constexpr int HALF = BN / 2;
+    constexpr int COLS = PairEpi<BN>::COLS;
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
+    const int part = (warp - 2) >> 2;
     const int row = q * 32 + lane;
     Epi ep = epi;  // per-launch state the epilogue reads once
     ep.setup();
@@ -408,18 +422,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       const Unit t = decode_pair_unit(shape, u, rank);
       // per-column data of this unit, one value per lane and 32 columns,
       // loaded before the drain so that their latency hides behind it
-      ep.unit_begin(t, lane, half * HALF);
-      float cs[HALF / 32];
+      ep.unit_begin(t, lane, part * COLS);
+      float cs[COLS / 32];
 #pragma unroll
-      for (int c = 0; c < HALF / 32; c++)
+      for (int c = 0; c < COLS / 32; c++)
         cs[c] = shape.col_scale ? __ldg(shape.col_scale +
-                                        min(t.nt * BN + half * HALF + c * 32 + lane, shape.N - 1))
+                                        min(t.nt * BN + part * COLS + c * 32 + lane, shape.N - 1))
                                 : 1.f;
       const float rs =
           shape.row_scale ? __ldg(shape.row_scale + min(t.m0 + row, shape.M - 1)) : 1.f;
-      float sum[HALF];
+      float sum[COLS];
 #pragma unroll
-      for (int i = 0; i < HALF; i++) sum[i] = 0.f;
+      for (int i = 0; i < COLS; i++) sum[i] = 0.f;
       for (int c0 = t.kb0; c0 < t.kb1; c0 += PROMO) {
         if (__any_sync(0xffffffffu, *abort != 0) ||
             !warp_wait(&tfull[acc], acc_phase, abort, shape.status, DEV_ERR_TIMEOUT_EPILOGUE,
@@ -429,14 +443,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
         }
         tc_fence_after();
 #pragma unroll
-        for (int c = 0; c < HALF / 32; c++) {
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                                 static_cast<uint32_t>(acc * BN + half * HALF + c * 32),
+        for (int c = 0; c < COLS / 16; c++) {  // 16 at a time: few registers beside the sums
+          uint32_t r[16];
+          tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                                 static_cast<uint32_t>(acc * BN + part * COLS + c * 16),
                              r);
           tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < 32; j++) sum[c * 32 + j] += __uint_as_float(r[j]);
+          for (int j = 0; j < 16; j++) sum[c * 16 + j] += __uint_as_float(r[j]);
         }
         tc_fence_before();
         __syncwarp();
@@ -449,15 +463,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
       if (!ok) break;
       if (shape.row_scale) {  // exact: powers of two
 #pragma unroll
-        for (int i = 0; i < HALF; i++) sum[i] *= rs;
+        for (int i = 0; i < COLS; i++) sum[i] *= rs;
       }
       if (shape.col_scale) {
 #pragma unroll
-        for (int i = 0; i < HALF; i++) sum[i] *= __shfl_sync(0xffffffffu, cs[i >> 5], i & 31);
+        for (int i = 0; i < COLS; i++) sum[i] *= __shfl_sync(0xffffffffu, cs[i >> 5], i & 31);
       }
 #pragma unroll
-      for (int c = 0; c < HALF / 32; c++)
-        ep.chunk(t, q, lane, row, half * HALF + c * 32,
+      for (int c = 0; c < COLS / 32; c++)
+        ep.chunk(t, q, lane, row, part * COLS + c * 32,
                   *reinterpret_cast<float(*)[32]>(sum + c * 32));
     }
   }

@@ -4,7 +4,7 @@
 // The pipeline is gemm_pair_kernel's (gemm_pair.cuh): a cluster of two CTAs
 // computes a 256 x BN tile with tcgen05.mma.cta_group::2, warp 0 loads K slabs
 // with cp.async.bulk.tensor (no multicast), warp 1 of the leader issues the
-// MMAs into one of two TMEM buffers, warps 2..9 of both CTAs drain them into
+// MMAs into one of two TMEM buffers, the other warps of both CTAs drain them into
 // round-to-nearest FP32 sums.  What changes is where a work unit comes from:
 // the launch walks the units of one list of the step's plan (GPlan), whose
 // problems and exclusive unit prefix the plan kernel wrote; unit u belongs to
@@ -120,35 +120,35 @@ __device__ __forceinline__ bool grouped_drain(Epi &ep, const Unit &t, int promo,
                                               uint64_t *tempty, volatile int *abort, int *status,
                                               unsigned long long tmo, int &acc,
                                               uint32_t &acc_phase, int warp, int lane) {
-  constexpr int HALF = BN / 2;
+  constexpr int COLS = PairEpi<BN>::COLS;
   const int q = warp & 3;
-  const int half = (warp - 2) >> 2;
+  const int part = (warp - 2) >> 2;
   const int row = q * 32 + lane;
   ep.setup();
-  ep.unit_begin(t, lane, half * HALF);
-  float cs[HALF / 32];
+  ep.unit_begin(t, lane, part * COLS);
+  float cs[COLS / 32];
 #pragma unroll
-  for (int c = 0; c < HALF / 32; c++)
-    cs[c] = col_scale ? __ldg(col_scale + min(t.nt * BN + half * HALF + c * 32 + lane, N - 1))
+  for (int c = 0; c < COLS / 32; c++)
+    cs[c] = col_scale ? __ldg(col_scale + min(t.nt * BN + part * COLS + c * 32 + lane, N - 1))
                       : 1.f;
   const float rs = row_scale ? __ldg(row_scale + min(t.m0 + row, M - 1)) : 1.f;
-  float sum[HALF];
+  float sum[COLS];
 #pragma unroll
-  for (int i = 0; i < HALF; i++) sum[i] = 0.f;
+  for (int i = 0; i < COLS; i++) sum[i] = 0.f;
   for (int c0 = t.kb0; c0 < t.kb1; c0 += promo) {
     if (__any_sync(0xffffffffu, *abort != 0) ||
         !warp_wait(&tfull[acc], acc_phase, abort, status, DEV_ERR_TIMEOUT_EPILOGUE, tmo))
       return false;
     tc_fence_after();
 #pragma unroll
-    for (int c = 0; c < HALF / 32; c++) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
-                             static_cast<uint32_t>(acc * BN + half * HALF + c * 32),
+    for (int c = 0; c < COLS / 16; c++) {  // 16 at a time: few registers beside the sums
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(tmem_base + (static_cast<uint32_t>(q * 32) << 16) +
+                             static_cast<uint32_t>(acc * BN + part * COLS + c * 16),
                          r);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; j++) sum[c * 32 + j] += __uint_as_float(r[j]);
+      for (int j = 0; j < 16; j++) sum[c * 16 + j] += __uint_as_float(r[j]);
     }
     tc_fence_before();
     __syncwarp();
@@ -160,15 +160,15 @@ __device__ __forceinline__ bool grouped_drain(Epi &ep, const Unit &t, int promo,
   }
   if (row_scale) {
 #pragma unroll
-    for (int i = 0; i < HALF; i++) sum[i] *= rs;
+    for (int i = 0; i < COLS; i++) sum[i] *= rs;
   }
   if (col_scale) {
 #pragma unroll
-    for (int i = 0; i < HALF; i++) sum[i] *= __shfl_sync(0xffffffffu, cs[i >> 5], i & 31);
+    for (int i = 0; i < COLS; i++) sum[i] *= __shfl_sync(0xffffffffu, cs[i >> 5], i & 31);
   }
 #pragma unroll
-  for (int c = 0; c < HALF / 32; c++)
-    ep.chunk(t, q, lane, row, half * HALF + c * 32, *reinterpret_cast<float(*)[32]>(sum + c * 32));
+  for (int c = 0; c < COLS / 32; c++)
+    ep.chunk(t, q, lane, row, part * COLS + c * 32, *reinterpret_cast<float(*)[32]>(sum + c * 32));
   return true;
 }
 
@@ -177,7 +177,7 @@ __device__ __forceinline__ bool grouped_drain(Epi &ep, const Unit &t, int promo,
 // formulations all take epilogue EPI (one epilogue per launch keeps the drain's
 // registers those of the one-problem kernel).
 template <int BN, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairEpi<BN>::THREADS, 1)
     gemm_pair_grouped_kernel(const GroupDev g, int list) {
   constexpr bool Z1 = EPI == GE_PARTIAL;
   using L = GPairSmem<BN>;
@@ -216,7 +216,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GEMM_THREADS, 1)
     }
     for (int a = 0; a < 2; a++) {
       mbar_init(&tfull[a], 1);
-      mbar_init(&tempty[a], PAIR_EPI_WARPS);
+      mbar_init(&tempty[a], PairEpi<BN>::ARRIVALS);
     }
     mbar_init(drain, 1);
     *abort = 0;

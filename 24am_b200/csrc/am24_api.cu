@@ -35,6 +35,16 @@ namespace am24host {
 thread_local std::string g_last_error;
 }  // namespace am24host
 
+// Whether p lies in memory of the handle's own device, which its kernels can read.
+static bool own_memory(am24_handle h, const void *p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == h->device;
+}
+
 namespace am24host {
 
 // K-major FP32 operand [rows][ld], loaded as bk x box_rows tiles; the swizzle
@@ -175,12 +185,11 @@ static am24_status reset_loaded(am24_handle h, am24_batch b) {
   return AM24_OK;
 }
 
-// The starting points staged in b's Vraw (all batch_size columns) become the
+// Starting points in device memory (n x batch_size, one after another) become the
 // batch's loadings: values and masks, and the words of a new load.
-static am24_status load_from_vraw(am24_handle h, am24_batch b) {
+static am24_status load_from(am24_handle h, am24_batch b, const float *src) {
   const MatrixDev &M = b->mat->d;
-  AM24_CUDA(launch_load_columns(b->d.Vraw, M.ldn, M.n, b->d.k, b->d.Vx, M.ldn, b->d.vmask,
-                                h->stream));
+  AM24_CUDA(launch_load_columns(src, M.n, M.n, b->d.k, b->d.Vx, M.ldn, b->d.vmask, h->stream));
   return reset_loaded(h, b);
 }
 
@@ -348,9 +357,9 @@ am24_status upload_columns(am24_handle h, am24_batch b, const float *host, int c
   const BatchDev &d = b->d;
   AM24_CUDA(cudaMemcpyAsync(slots_dev, slots, sizeof(int) * cols, cudaMemcpyHostToDevice,
                             h->stream));
-  AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, host, sizeof(float) * M.n,
-                              sizeof(float) * M.n, cols, cudaMemcpyHostToDevice, h->stream));
-  AM24_CUDA(launch_load_slots(d.Vraw, M.ldn, M.n, cols, slots_dev, d.Vx, M.ldn, d.vmask, d.sel_hint,
+  AM24_CUDA(cudaMemcpyAsync(d.Vraw, host, sizeof(float) * (size_t)M.n * cols,
+                            cudaMemcpyHostToDevice, h->stream));
+  AM24_CUDA(launch_load_slots(d.Vraw, M.n, M.n, cols, slots_dev, d.Vx, M.ldn, d.vmask, d.sel_hint,
                               d.val, d.max_nnz, d.planes_nnz, h->stream));
   return AM24_OK;
 }
@@ -548,13 +557,7 @@ static am24_status create_matrix(am24_handle h, const float *B, int32_t ldB, uin
   // memory, which a kernel may not reach); the other layouts are made from Bc when
   // a batch first needs them
   cudaError_t e = cudaSuccess;
-  bool own = false;
-  if (on_device) {
-    cudaPointerAttributes at;
-    own = cudaPointerGetAttributes(&at, B) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
-          at.device == h->device;
-    if (!own) cudaGetLastError();
-  }
+  const bool own = on_device && own_memory(h, B);
   if (own) {
     e = launch_copy_matrix(M, B, ldB, h->stream);
   } else {
@@ -881,14 +884,13 @@ am24_status am24_batch_load(am24_handle h, am24_batch b, const float *V, int32_t
   if (!h || !b || !V) return fail(AM24_ERR_INVALID_ARG, "NULL argument");
   const MatrixDev &M = b->mat->d;
   const int k = b->d.k;
-  if (on_device) {
-    AM24_CUDA(cudaMemcpy2DAsync(b->d.Vraw, sizeof(float) * M.ldn, V, sizeof(float) * M.n,
-                                sizeof(float) * M.n, k, cudaMemcpyDeviceToDevice, h->stream));
-  } else {
-    AM24_CUDA(cudaMemcpy2DAsync(b->d.Vraw, sizeof(float) * M.ldn, V, sizeof(float) * M.n,
-                                sizeof(float) * M.n, k, cudaMemcpyHostToDevice, h->stream));
-  }
-  return load_from_vraw(h, b);
+  // read in place where a kernel can (this device's own memory), else staged in
+  // Vraw by one contiguous copy
+  if (on_device && own_memory(h, V)) return load_from(h, b, V);
+  AM24_CUDA(cudaMemcpyAsync(b->d.Vraw, V, sizeof(float) * (size_t)M.n * k,
+                            on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                            h->stream));
+  return load_from(h, b, b->d.Vraw);
 }
 
 am24_status am24_batch_iterate(am24_handle h, am24_batch b, int32_t it0, int32_t iterations,
@@ -913,10 +915,9 @@ am24_status am24_batch_read(am24_handle h, am24_batch b, float *V, float *val, f
   const MatrixDev &M = b->mat->d;
   const int k = b->d.k;
   if (V) {
-    AM24_CUDA(launch_masked_copy(b->d.Vx, b->d.vmask, M.ldn, M.n, k, b->d.Vraw, M.ldn,
-                                 h->stream));
-    AM24_CUDA(cudaMemcpy2DAsync(V, sizeof(float) * M.n, b->d.Vraw, sizeof(float) * M.ldn,
-                                sizeof(float) * M.n, k, cudaMemcpyDeviceToHost, h->stream));
+    AM24_CUDA(launch_masked_copy(b->d.Vx, b->d.vmask, M.ldn, M.n, k, b->d.Vraw, M.n, h->stream));
+    AM24_CUDA(cudaMemcpyAsync(V, b->d.Vraw, sizeof(float) * (size_t)M.n * k,
+                              cudaMemcpyDeviceToHost, h->stream));
   }
   if (val)
     AM24_CUDA(cudaMemcpyAsync(val, b->d.val, sizeof(float) * k, cudaMemcpyDeviceToHost, h->stream));
@@ -1120,24 +1121,24 @@ am24_status am24_solve_resident_f32(am24_handle h, am24_matrix mat, float *x,
         gidx[j] = shift + j;
         slots[j] = j;
       }
-      // the batch's starts, staged in Vraw by one copy (or generated in place)
+      // the batch's starts, staged by one copy (or generated in place)
       const bool device = s.start_mode == AM24_START_DEVICE_UNIFORM;
+      const float *staged = d.Vraw;
       if (device) {
         AM24_CUDA(launch_uniform_starts(d.Vx, M.ldn, (int)n, bs, shift, d.vmask, h->stream));
       } else if (batch == 0 && pre) {  // already on the device
         AM24_CUDA(cudaStreamWaitEvent(h->stream, pre_done, 0));
-        AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, pre, sizeof(float) * n,
-                                    sizeof(float) * n, bs, cudaMemcpyDeviceToDevice, h->stream));
+        staged = pre;
       } else {
         const float *src = start_points + (size_t)shift * n;  // injected: read in place
         if (s.start_mode != AM24_START_INJECTED) {
           host_starts(s, n, start_points, gidx.data(), bs, staging);
           src = staging.data();
         }
-        AM24_CUDA(cudaMemcpy2DAsync(d.Vraw, sizeof(float) * M.ldn, src, sizeof(float) * n,
-                                    sizeof(float) * n, bs, cudaMemcpyHostToDevice, h->stream));
+        AM24_CUDA(cudaMemcpyAsync(d.Vraw, src, sizeof(float) * (size_t)n * bs,
+                                  cudaMemcpyHostToDevice, h->stream));
       }
-      AM24_TRY(device ? reset_loaded(h, b) : load_from_vraw(h, b));
+      AM24_TRY(device ? reset_loaded(h, b) : load_from(h, b, staged));
       AM24_CUDA(cudaEventRecord(e0, h->stream));
       BatchRun run;
       AM24_TRY(run_batch_steps(h, b, s, (int)shift, &run));

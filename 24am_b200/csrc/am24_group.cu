@@ -382,10 +382,10 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
       host_starts(s, (unsigned)M.n, start_points, gidx.data(), k, staging);
       src = staging.data();
     }
-    AM24_CUDA(cudaMemcpy2DAsync(P.Vraw, sizeof(float) * M.ldn, src, sizeof(float) * M.n,
-                                sizeof(float) * M.n, k, cudaMemcpyHostToDevice, hs));
+    AM24_CUDA(cudaMemcpyAsync(P.Vraw, src, sizeof(float) * (size_t)M.n * k,
+                              cudaMemcpyHostToDevice, hs));
     AM24_CUDA(cudaStreamSynchronize(hs));  // `staging` goes out of scope
-    AM24_CUDA(launch_load_columns(P.Vraw, M.ldn, M.n, k, P.Vx, M.ldn, P.vmask, hs));
+    AM24_CUDA(launch_load_columns(P.Vraw, M.n, M.n, k, P.Vx, M.ldn, P.vmask, hs));
   }
   // tensor maps
   GMaps maps;
@@ -486,9 +486,9 @@ am24_status am24_group_read(am24_group g, uint32_t problem, float *V, float *val
   AM24_CUDA(cudaSetDevice(g->h->device));
   const int k = P.k;
   if (V) {
-    AM24_CUDA(launch_masked_copy(P.Vx, P.vmask, P.ldn, P.n, k, P.Vraw, P.ldn, hs));
-    AM24_CUDA(cudaMemcpy2DAsync(V, sizeof(float) * P.n, P.Vraw, sizeof(float) * P.ldn,
-                                sizeof(float) * P.n, k, cudaMemcpyDeviceToHost, hs));
+    AM24_CUDA(launch_masked_copy(P.Vx, P.vmask, P.ldn, P.n, k, P.Vraw, P.n, hs));
+    AM24_CUDA(cudaMemcpyAsync(V, P.Vraw, sizeof(float) * (size_t)P.n * k, cudaMemcpyDeviceToHost,
+                              hs));
   }
   if (val) AM24_CUDA(cudaMemcpyAsync(val, P.val, sizeof(float) * k, cudaMemcpyDeviceToHost, hs));
   if (err) AM24_CUDA(cudaMemcpyAsync(err, P.err, sizeof(float) * k, cudaMemcpyDeviceToHost, hs));

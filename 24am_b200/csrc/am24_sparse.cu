@@ -350,9 +350,9 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
         host_starts(s, n, start_points, gidx.data(), k, staging);
         src = staging.data();
       }
-      AM24_CUDA(cudaMemcpy2DAsync(b.Vraw, sizeof(float) * b.ldn, src, sizeof(float) * n,
-                                  sizeof(float) * n, k, cudaMemcpyHostToDevice, h->stream));
-      AM24_CUDA(launch_load_columns(b.Vraw, b.ldn, (int)n, k, b.Vx, b.ldn, b.vmask, h->stream));
+      AM24_CUDA(cudaMemcpyAsync(b.Vraw, src, sizeof(float) * (size_t)n * k,
+                                cudaMemcpyHostToDevice, h->stream));
+      AM24_CUDA(launch_load_columns(b.Vraw, (int)n, (int)n, k, b.Vx, b.ldn, b.vmask, h->stream));
     }
     AM24_CUDA(launch_reset_batch(k, b.sel_hint, b.val, b.err, b.max_nnz, nullptr, b.ctl,
                                  h->stream));

@@ -340,13 +340,15 @@ struct SparseBatchDev {
   float *Vraw = nullptr;     // k x ldn raw V = B^T Z (and the staging of loads)
   float *Vt = nullptr;       // n x kp
   uint32_t *xmask = nullptr; // per tile of starts, a bit per row of Vt: not zero in the tile
-  float *Zs = nullptr;       // k x ldm
+  float *Zs = nullptr;       // k x ldm (the scatter's)
   float *Zt = nullptr;       // m x kp
   float *fz = nullptr, *val = nullptr, *err = nullptr, *max_err = nullptr;
   float *sel_hint = nullptr, *obj_part = nullptr, *nnz_part = nullptr;
   uint32_t *nnz = nullptr, *max_nnz = nullptr;
   uint32_t *ctl = nullptr;  // CTL_WORDS
   double *sum_v = nullptr, *dot_mu = nullptr, *zsum = nullptr, *zdot = nullptr;  // per start
+  double *zpart = nullptr;   // 3 x sparse_zblocks(m, kp) x kp partial sums of the pass over Z
+  float *zinv = nullptr;     // kp: 1 / ||z|| (penalized L2 variance)
   float *part_cols = nullptr, *part_rows = nullptr;  // segments x kp partial sums
   unsigned long long *work = nullptr;  // matrix entries in the supports' columns (this step)
   uint32_t *zgate = nullptr;           // this step's Z = B V path: 0 scatter, 1 CSR product
@@ -366,6 +368,8 @@ cudaError_t launch_sparse_ev(const SparseDev &S, const float *x, double *scratch
                              cudaStream_t st);
 inline size_t sparse_ev_scratch(const SparseDev &S) { return (size_t)(S.m + 255) / 256 + 2; }
 int num_sms();
+// Blocks per tile of starts of the sparse step's pass over Z.
+int sparse_zblocks(int m, int kp);
 // Whether the sparse Z = B V of m samples is the listed, tiled form.
 bool gather_is_wide(int m);
 // Fills M's TF32 planes (Bc_hi/lo, Bt_hi/lo) from M.Bc.

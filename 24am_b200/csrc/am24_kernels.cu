@@ -3256,7 +3256,7 @@ namespace {
 // and the segments of the long ones, the combine kernel for the long ones' sums.
 // gate (may be null): the launches do their work only when *gate >= gate_min.
 // xmask (may be null): the rows of X that are not zero, per tile of starts.
-template <bool SKIP>
+template <bool SKIP, bool ROWS>
 void sparse_product(const int32_t *ptr, const int32_t *idx, const float *val, int ncols,
                     const SparseLong &L, const float *X, float *part, const SparseBatchDev &b,
                     float *out, int ld_out, const float *cvec, const double *a, const double *bv,
@@ -3264,16 +3264,25 @@ void sparse_product(const int32_t *ptr, const int32_t *idx, const float *val, in
                     cudaStream_t st) {
   const int tiles = (b.kp + SP_WIDE - 1) / SP_WIDE;
   const int seg_blocks = L.count ? (L.segs + SP_OUTER - 1) / SP_OUTER : 0;
-  sp_spmm_kernel<SKIP>
+  sp_spmm_kernel<SKIP, ROWS>
       <<<dim3(seg_blocks + (ncols + SP_OUTER - 1) / SP_OUTER, tiles), SP_THREADS, 0, st>>>(
           ptr, idx, val, ncols, X, b.kp, b.k, out, ld_out, cvec, a, bv, b.ctl, gate, gate_min,
           xmask, b.ldn / 32, L.seg_e0, L.seg_e1, L.segs, seg_blocks, part);
   if (L.count == 0) return;
-  sp_spmm_long_kernel<<<dim3(L.count, b.kp / SP_TILE), SP_TILE, 0, st>>>(
+  sp_spmm_long_kernel<ROWS><<<dim3(L.count, b.kp / SP_TILE), SP_TILE, 0, st>>>(
       L.outer, L.seg_first, part, b.kp, b.k, out, ld_out, cvec, a, bv, b.ctl, gate, gate_min);
 }
 
 }  // namespace
+
+// Blocks a tile of starts for the pass over Z: over all tiles as many as run at once
+// (three a multiprocessor), each warp with at least four rows.
+int sparse_zblocks(int m, int kp) {
+  const int tiles = (kp + SP_WIDE - 1) / SP_WIDE;
+  const int most = std::max(1, 3 * num_sms() / tiles);
+  const int per = 4 * SP_THREADS / 32;
+  return std::max(1, std::min(most, (m + per - 1) / per));
+}
 
 cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, const StepParams &p,
                                cudaStream_t st) {
@@ -3301,21 +3310,39 @@ cudaError_t launch_sparse_step(const SparseDev &S, const SparseBatchDev &b, cons
                           SP_THREADS, 0, st>>>(b.Vx, b.vmask, b.ldn, S.n, b.k, b.Vt, b.kp,
                                                b.xmask, b.ctl, b.zgate, 1u, S.defl, S.comps,
                                                b.defl_a);
-  sparse_product<true>(S.row_ptr, S.col_ind, S.rvals, S.m, S.long_rows, b.Vt, b.part_rows, b,
-                       b.Zs, b.ldm, S.row_means, S.row_means ? b.sum_v : nullptr,
-                       S.means ? b.dot_mu : nullptr, b.zgate, 1u, b.xmask, st);
+  sparse_product<true, true>(S.row_ptr, S.col_ind, S.rvals, S.m, S.long_rows, b.Vt, b.part_rows,
+                             b, b.Zt, b.kp, S.row_means, S.row_means ? b.sum_v : nullptr,
+                             S.means ? b.dot_mu : nullptr, b.zgate, 1u, b.xmask, st);
   sp_scatter_z_kernel<<<b.k, SP_THREADS, 0, st>>>(
       S.col_ptr, S.row_ind, S.cvals, b.Vx, b.vmask, b.ldn, b.Zs, b.ldm, S.m, S.row_means,
       S.row_means ? b.sum_v : nullptr, S.means ? b.dot_mu : nullptr, b.zgate, 0u, b.ctl);
+  // eight blocks a multiprocessor, so that a step without the scatter passes quickly
+  const int zt_blocks = std::max(1, 8 * num_sms() / (b.kp / SP_TILE));
+  sp_transpose_z_kernel<<<dim3(std::min((S.m + SP_TILE - 1) / SP_TILE, zt_blocks),
+                               b.kp / SP_TILE),
+                          SP_THREADS, 0, st>>>(b.Zs, b.ldm, S.m, b.k, b.Zt, b.kp, b.zgate, b.ctl);
   // 2. the formulation's sign / norm of z, and the sums V's correction needs
-  sp_zreduce_kernel<<<b.k, SP_THREADS, 0, st>>>(b.Zs, b.ldm, S.m, f, b.fz, S.row_means,
-                                                centred ? b.zsum : nullptr, b.zdot, b.ctl);
-  sp_transpose_z_kernel<<<dim3((S.m + SP_TILE - 1) / SP_TILE, b.kp / SP_TILE), SP_THREADS, 0,
-                          st>>>(b.Zs, b.ldm, S.m, b.k, b.Zt, b.kp, b.ctl);
+  const dim3 zp(sparse_zblocks(S.m, b.kp), (b.kp + SP_WIDE - 1) / SP_WIDE);
+  const int rows = (S.m + zp.x - 1) / zp.x;
+  const bool l1var = f & 1, norm = f <= 3 || !l1var, twice = f > 3 && !l1var;
+  sp_zpass_kernel<<<zp, SP_THREADS, 0, st>>>(b.Zt, b.kp, S.m, rows, f, nullptr, centred,
+                                             S.row_means, b.zpart, b.ctl);
+  if (norm || centred)
+    sp_zsum_kernel<<<b.kp / 32, SP_THREADS, 0, st>>>(b.zpart, zp.x, b.kp, b.k, f, norm,
+                                                     centred && !twice, b.fz, b.zinv, b.zsum,
+                                                     b.zdot, b.ctl);
+  if (twice) {
+    sp_zpass_kernel<<<zp, SP_THREADS, 0, st>>>(b.Zt, b.kp, S.m, rows, f, b.zinv, centred,
+                                               S.row_means, b.zpart, b.ctl);
+    if (centred)
+      sp_zsum_kernel<<<b.kp / 32, SP_THREADS, 0, st>>>(b.zpart, zp.x, b.kp, b.k, f, false, true,
+                                                       b.fz, b.zinv, b.zsum, b.zdot, b.ctl);
+  }
   // 3. V = (B - 1 mu^T - r 1^T)^T Z: CSC columns against Z transposed
-  sparse_product<false>(S.col_ptr, S.row_ind, S.cvals, S.n, S.long_cols, b.Zt, b.part_cols, b,
-                        b.Vraw, b.ldn, S.means, S.means ? b.zsum : nullptr,
-                        S.row_means ? b.zdot : nullptr, nullptr, 0, nullptr, st);
+  sparse_product<false, false>(S.col_ptr, S.row_ind, S.cvals, S.n, S.long_cols, b.Zt,
+                               b.part_cols, b, b.Vraw, b.ldn, S.means,
+                               S.means ? b.zsum : nullptr, S.row_means ? b.zdot : nullptr,
+                               nullptr, 0, nullptr, st);
   if (S.comps > 0)
     sp_defl_vraw_kernel<<<b.k, SP_THREADS, 0, st>>>(b.Vraw, b.ldn, S.n, S.defl, S.comps, S.gram,
                                                     b.ctl);

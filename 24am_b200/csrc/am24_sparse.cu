@@ -293,6 +293,8 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   AM24_TRY(A.get(&b.dot_mu, k));
   AM24_TRY(A.get(&b.zsum, k));
   AM24_TRY(A.get(&b.zdot, k));
+  AM24_TRY(A.get(&b.zpart, 3 * (size_t)sparse_zblocks(S.m, b.kp) * b.kp));
+  AM24_TRY(A.get(&b.zinv, b.kp));
   AM24_TRY(A.get(&b.status, 1));
   AM24_TRY(A.get(&b.iters, b.log_capacity));
   AM24_TRY(A.get(&b.cards, b.log_capacity));

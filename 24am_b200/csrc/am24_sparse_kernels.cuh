@@ -116,6 +116,8 @@ __device__ __forceinline__ float sp_correct(float acc, int c, int j, const float
 
 // out[j][c] (j < k, c < ncols) = sum_e val[e] X[idx[e] * kp + j]
 //                                - (cvec ? cvec[c] * a[j] : 0) - (b ? b[j] : 0)
+// with out start-major (ROWS: row-major, out[c][j] for j < kp, zero past k: Z in the
+// layout that B^T Z reads).
 // One warp per outer entry, SP_VEC starts per lane: every entry reads one row
 // segment of X, 512 bytes.  Each sum runs over the outer entry's entries in
 // storage order with FP32 FMAs (deterministic); the correction is applied in
@@ -126,7 +128,7 @@ __device__ __forceinline__ float sp_correct(float acc, int c, int j, const float
 // (17.6 TB/s for B^T Z of 6 M entries, 512 starts: 0.69 ms; with one start per
 // lane the instructions did: 2.8 ms), and where rows are left out the scan of the
 // entries (0.34 ms once supports are sparse; 2.0 ms when every row was read).
-template <bool SKIP>
+template <bool SKIP, bool ROWS>
 __global__ void __launch_bounds__(SP_THREADS) sp_spmm_kernel(
     const int32_t *__restrict__ ptr, const int32_t *__restrict__ idx,
     const float *__restrict__ val, int ncols, const float *__restrict__ X, int kp, int k,
@@ -136,8 +138,6 @@ __global__ void __launch_bounds__(SP_THREADS) sp_spmm_kernel(
     const int32_t *__restrict__ seg_e0, const int32_t *__restrict__ seg_e1, int segs,
     int seg_blocks, float *__restrict__ part) {
   if (*stop || (gate && *gate < gate_min)) return;
-  __shared__ float tile[SP_WIDE][SP_OUTER + 1];
-  __shared__ int skip[SP_OUTER];
   __shared__ int2 queues[SKIP ? SP_OUTER : 1][64];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j0 = blockIdx.y * SP_WIDE, j = j0 + SP_VEC * lane;
@@ -162,17 +162,27 @@ __global__ void __launch_bounds__(SP_THREADS) sp_spmm_kernel(
       sp_dot<SKIP>(idx, val, X, kp, jl, e0, e1, xm, queue, acc);
     }
   }
-  const float y[SP_VEC] = {acc.x, acc.y, acc.z, acc.w};
+  float y[SP_VEC] = {acc.x, acc.y, acc.z, acc.w};
+  if constexpr (ROWS) {
+    if (!own || j >= kp) return;
 #pragma unroll
-  for (int i = 0; i < SP_VEC; i++)
-    tile[SP_VEC * lane + i][warp] =
-        own && j + i < k ? sp_correct(y[i], c, j + i, cvec, a, b) : 0.f;
-  if (lane == 0) skip[warp] = !own;
-  __syncthreads();
-  const int cw = threadIdx.x % SP_OUTER;  // a start's row of the tile: one 32-byte sector
-  if (c0 + cw >= ncols || skip[cw]) return;
-  for (int r = threadIdx.x / SP_OUTER; r < SP_WIDE; r += SP_THREADS / SP_OUTER)
-    if (j0 + r < k) out[(size_t)(j0 + r) * ld_out + c0 + cw] = tile[r][cw];
+    for (int i = 0; i < SP_VEC; i++)
+      y[i] = j + i < k ? sp_correct(y[i], c, j + i, cvec, a, b) : 0.f;
+    *reinterpret_cast<float4 *>(out + (size_t)c * ld_out + j) = make_float4(y[0], y[1], y[2], y[3]);
+  } else {
+    __shared__ float tile[SP_WIDE][SP_OUTER + 1];
+    __shared__ int skip[SP_OUTER];
+#pragma unroll
+    for (int i = 0; i < SP_VEC; i++)
+      tile[SP_VEC * lane + i][warp] =
+          own && j + i < k ? sp_correct(y[i], c, j + i, cvec, a, b) : 0.f;
+    if (lane == 0) skip[warp] = !own;
+    __syncthreads();
+    const int cw = threadIdx.x % SP_OUTER;  // a start's row of the tile: one 32-byte sector
+    if (c0 + cw >= ncols || skip[cw]) return;
+    for (int r = threadIdx.x / SP_OUTER; r < SP_WIDE; r += SP_THREADS / SP_OUTER)
+      if (j0 + r < k) out[(size_t)(j0 + r) * ld_out + c0 + cw] = tile[r][cw];
+  }
 }
 
 // Z = (B - centring) V once V is sparse (when sp_zgate_kernel chose this path:
@@ -250,7 +260,9 @@ __global__ void __launch_bounds__(SP_THREADS) sp_scatter_z_kernel(
   }
 }
 
-// Long outer entries: per (entry, start) the segments' sums in segment order, then the centring, into out[j][c].
+// Long outer entries: per (entry, start) the segments' sums in segment order, then the centring, into
+// out[j][c] (ROWS: out[c][j], zero past k).
+template <bool ROWS>
 __global__ void __launch_bounds__(SP_TILE) sp_spmm_long_kernel(
     const int32_t *__restrict__ outer, const int32_t *__restrict__ seg_first,
     const float *__restrict__ part, int kp, int k, float *__restrict__ out, int ld_out,
@@ -259,11 +271,12 @@ __global__ void __launch_bounds__(SP_TILE) sp_spmm_long_kernel(
   if (*stop || (gate && *gate < gate_min)) return;
   const int x = blockIdx.x;
   const int j = blockIdx.y * SP_TILE + threadIdx.x;
-  if (j >= k) return;
+  if (j >= (ROWS ? kp : k)) return;
   const int c = outer[x];
   float acc = 0.f;
   for (int s = seg_first[x]; s < seg_first[x + 1]; s++) acc += part[(size_t)s * kp + j];
-  out[(size_t)j * ld_out + c] = sp_correct(acc, c, j, cvec, a, b);
+  if (j < k) acc = sp_correct(acc, c, j, cvec, a, b);
+  out[ROWS ? (size_t)c * ld_out + j : (size_t)j * ld_out + c] = j < k ? acc : 0.f;
 }
 
 // Vt[q][j] = V's column j at row q (zero where its mask bit is clear), for
@@ -316,23 +329,26 @@ __global__ void __launch_bounds__(SP_THREADS) sp_transpose_v_kernel(
   if (threadIdx.x == 0) xmask[(size_t)blockIdx.y * words + blockIdx.x] = any;
 }
 
-// Zt[i][j] = Zs[j][i] for i < m, j < kp (columns k..kp-1 zero): the row-major
-// X of V = B^T Z.
+// Zt[i][j] = Zs[j][i] for i < m, j < kp (columns k..kp-1 zero): the scatter's
+// Z as the row-major X of V = B^T Z (the CSR product writes Zt itself).
 __global__ void __launch_bounds__(SP_THREADS) sp_transpose_z_kernel(
     const float *__restrict__ Zs, int ldm, int m, int k, float *__restrict__ Zt, int kp,
-    const uint32_t *stop) {
-  if (*stop) return;
+    const uint32_t *gate, const uint32_t *stop) {
+  if (*stop || *gate != 0u) return;
   __shared__ float tile[SP_TILE][SP_TILE + 1];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int i0 = blockIdx.x * SP_TILE, j0 = blockIdx.y * SP_TILE;
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int j = j0 + r, i = i0 + lane;
-    tile[r][lane] = (j < k && i < m) ? Zs[(size_t)j * ldm + i] : 0.f;
-  }
-  __syncthreads();
-  for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
-    const int i = i0 + r;
-    if (i < m) Zt[(size_t)i * kp + j0 + lane] = tile[lane][r];
+  const int j0 = blockIdx.y * SP_TILE;
+  for (int i0 = blockIdx.x * SP_TILE; i0 < m; i0 += gridDim.x * SP_TILE) {
+    for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
+      const int j = j0 + r, i = i0 + lane;
+      tile[r][lane] = (j < k && i < m) ? Zs[(size_t)j * ldm + i] : 0.f;
+    }
+    __syncthreads();
+    for (int r = warp; r < SP_TILE; r += SP_THREADS / 32) {
+      const int i = i0 + r;
+      if (i < m) Zt[(size_t)i * kp + j0 + lane] = tile[lane][r];
+    }
+    __syncthreads();
   }
 }
 
@@ -407,52 +423,122 @@ __global__ void sp_zgate_kernel(const uint32_t *max_nnz, uint32_t cap,
   *max_err = 0.f;
 }
 
-// Per start j (one block), on z = Zs[j] after the centred product:
+// On z = Zt's column j (row-major, kp floats a row) after the centred product:
 //   constrained L2 variance (forms 0, 2): fz = ||z||_2, z kept;
 //   constrained L1 variance (1, 3): fz = ||z||_1, z <- sgn z;
 //   penalized L2 variance (4, 6): z <- z / ||z||_2;
 //   penalized L1 variance (5, 7): z <- sgn z
 // (gpower_commons.h:68-177 as the dense path runs it), then, when the matrix
-// is centred, zsum[j] = sum_i z_i and zdot[j] = sum_i r_i z_i of the result
-// (the corrections of V = B^T Z).  Norms and sums in FP64, fixed order.
-__global__ void __launch_bounds__(SP_THREADS) sp_zreduce_kernel(
-    float *__restrict__ Zs, int ldm, int m, int formulation, float *__restrict__ fz,
-    const float *__restrict__ row_means, double *__restrict__ zsum, double *__restrict__ zdot,
-    const uint32_t *stop) {
+// is centred (sums), zsum[j] = sum_i z_i and zdot[j] = sum_i r_i z_i of the
+// result (the corrections of V = B^T Z).  Norms and sums in FP64, fixed order.
+// A block takes `rows` rows of a tile of SP_WIDE starts, a warp every eighth of
+// them, SP_VEC starts per lane, and writes its sums to part[q][block][j] (q = 0
+// the norm's, 1 zsum's, 2 zdot's); sp_zsum_kernel adds the blocks up.
+// inv = null: the pass after the product; else (forms 4, 6) the second one, which
+// scales by inv[j].  What bounds it: the FP64 conversions and sums beside one read of
+// Z (and one write where the values change): 53 us for 40000 samples x 512 starts,
+// where a pass over start-major columns and their transposition took 92 + 140.
+__global__ void __launch_bounds__(SP_THREADS) sp_zpass_kernel(
+    float *__restrict__ Zt, int kp, int m, int rows, int formulation,
+    const float *__restrict__ inv, bool sums, const float *__restrict__ row_means,
+    double *__restrict__ part, const uint32_t *stop) {
   if (*stop) return;
-  __shared__ double red[SP_THREADS / 32];
-  const int j = blockIdx.x;
-  float *z = Zs + (size_t)j * ldm;
-  const bool l1var = formulation == 1 || formulation == 3 || formulation == 5 || formulation == 7;
-  const bool cons = formulation <= 3;
-  float inv = 1.f;
-  if (cons || !l1var) {
-    double t = 0.0;
-    for (int i = threadIdx.x; i < m; i += SP_THREADS) {
-      const double v = (double)z[i];
-      t += l1var ? fabs(v) : v * v;
+  __shared__ double red[SP_THREADS / 32][SP_WIDE];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j0 = blockIdx.y * SP_WIDE, j = j0 + SP_VEC * lane;
+  const bool l1var = formulation & 1, norm = !inv && (formulation <= 3 || !l1var);
+  const bool first_of_two = !inv && formulation > 3 && !l1var;
+  const bool write = l1var || inv;
+  sums = sums && !first_of_two;
+  double t[SP_VEC] = {}, s[SP_VEC] = {}, d[SP_VEC] = {};
+  float f[SP_VEC] = {1.f, 1.f, 1.f, 1.f};
+  const int i0 = blockIdx.x * rows, i1 = min(m, i0 + rows);
+  if (j < kp) {
+    if (inv) {
+#pragma unroll
+      for (int c = 0; c < SP_VEC; c++) f[c] = inv[j + c];
     }
-    t = sp_block_sum(t, red);
-    if (cons && threadIdx.x == 0) fz[j] = l1var ? (float)t : (float)sqrt(t);
-    if (!cons) inv = 1.0f / (float)sqrt(t);
-  }
-  double s = 0.0, d = 0.0;
-  for (int i = threadIdx.x; i < m; i += SP_THREADS) {
-    float v = z[i];
-    if (l1var)
-      v = (float)((v > 0.f) - (v < 0.f));
-    else if (!cons)
-      v *= inv;
-    if (l1var || !cons) z[i] = v;
-    if (zsum) {
-      s += (double)v;
-      if (row_means) d += (double)row_means[i] * (double)v;
+    constexpr int ROWS = 4, STEP = SP_THREADS / 32;  // rows a warp loads before it uses them
+    for (int ib = i0 + warp; ib < i1; ib += ROWS * STEP) {
+      float4 zs[ROWS];
+#pragma unroll
+      for (int u = 0; u < ROWS; u++)
+        if (ib + u * STEP < i1)
+          zs[u] = *reinterpret_cast<const float4 *>(Zt + (size_t)(ib + u * STEP) * kp + j);
+#pragma unroll
+      for (int u = 0; u < ROWS; u++) {
+        const int i = ib + u * STEP;
+        if (i >= i1) break;
+        float v[SP_VEC] = {zs[u].x, zs[u].y, zs[u].z, zs[u].w};
+        const double r = sums && row_means ? (double)row_means[i] : 0.0;
+#pragma unroll
+        for (int c = 0; c < SP_VEC; c++) {
+          if (norm) t[c] += l1var ? fabs((double)v[c]) : (double)v[c] * (double)v[c];
+          if (l1var)
+            v[c] = (float)((v[c] > 0.f) - (v[c] < 0.f));
+          else if (inv)
+            v[c] *= f[c];
+          if (sums) {
+            s[c] += (double)v[c];
+            if (row_means) d[c] += r * (double)v[c];
+          }
+        }
+        if (write)
+          *reinterpret_cast<float4 *>(Zt + (size_t)i * kp + j) =
+              make_float4(v[0], v[1], v[2], v[3]);
+      }
     }
   }
-  if (zsum) {
-    s = sp_block_sum(s, red);
-    d = sp_block_sum(d, red);
-    if (threadIdx.x == 0) {
+  // the warps' sums in warp order
+  auto put = [&](const double (&x)[SP_VEC], int q) {
+#pragma unroll
+    for (int c = 0; c < SP_VEC; c++) red[warp][SP_VEC * lane + c] = x[c];
+    __syncthreads();
+    if (threadIdx.x < SP_WIDE && j0 + (int)threadIdx.x < kp) {
+      double y = 0.0;
+      for (int w = 0; w < SP_THREADS / 32; w++) y += red[w][threadIdx.x];
+      part[((size_t)q * gridDim.x + blockIdx.x) * kp + j0 + threadIdx.x] = y;
+    }
+    __syncthreads();
+  };
+  if (norm) put(t, 0);
+  if (sums) {
+    put(s, 1);
+    put(d, 2);
+  }
+}
+
+// The blocks' sums of sp_zpass_kernel added up in a fixed order, a start per
+// lane: fz and inv as the formulation has them (when `norm`), zsum and zdot (when
+// `sums`).
+__global__ void __launch_bounds__(SP_THREADS) sp_zsum_kernel(
+    const double *__restrict__ part, int blocks, int kp, int k, int formulation, bool norm,
+    bool sums, float *__restrict__ fz, float *__restrict__ inv, double *__restrict__ zsum,
+    double *__restrict__ zdot, const uint32_t *stop) {
+  if (*stop) return;
+  __shared__ double red[SP_THREADS / 32][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j = blockIdx.x * 32 + lane;  // kp is a multiple of 32
+  auto total = [&](int q) {
+    double y = 0.0;
+#pragma unroll 8
+    for (int b = warp; b < blocks; b += SP_THREADS / 32) y += part[((size_t)q * blocks + b) * kp + j];
+    red[warp][lane] = y;
+    __syncthreads();
+    y = 0.0;
+    for (int w = 0; w < SP_THREADS / 32; w++) y += red[w][lane];
+    __syncthreads();
+    return y;
+  };
+  const bool mine = warp == 0 && j < k;
+  if (norm) {
+    const double t = total(0);
+    if (mine && formulation <= 3) fz[j] = (formulation & 1) ? (float)t : (float)sqrt(t);
+    if (warp == 0 && formulation > 3) inv[j] = j < k ? 1.0f / (float)sqrt(t) : 0.f;
+  }
+  if (sums) {
+    const double s = total(1), d = total(2);
+    if (mine) {
       zsum[j] = s;
       zdot[j] = d;
     }

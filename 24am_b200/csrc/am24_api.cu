@@ -771,13 +771,25 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
       (st = A.get(&d.Vraw, kv)) ||
       (st = A.get(&d.Z_hi, kz)) || (!d.fp16_2 && (st = A.get(&d.Z_lo, kz))) ||
       (st = A.get(&d.ws, d.ws_len)) ||
-      (st = A.get(&d.fz, k)) || (st = A.get(&d.obj_part, (size_t)k * parts)) ||
-      (st = A.get(&d.nnz_part, (size_t)k * parts)) || (st = A.get(&d.nnz, k)) ||
-      (st = A.get(&d.val, 2 * (size_t)k)) || (st = A.get(&d.max_err, 1)) ||
-      (st = A.get(&d.iters, d.log_capacity)) || (st = A.get(&d.cards, d.log_capacity)) ||
-      (st = A.get(&d.status, 1)) || (st = A.get(&d.vmask, (size_t)k * (M.ldn / 32))) ||
-      (st = A.get(&d.max_nnz, 1)) || (st = A.get(&d.planes_nnz, 1)) ||
-      (st = A.get(&d.sel_hint, k)) || (st = A.get(&d.ctl, (size_t)CTL_WORDS)) ||
+      (st = A.get(&d.obj_part, (size_t)k * parts)) ||
+      (st = A.get(&d.nnz_part, (size_t)k * parts)) || (st = A.get(&d.max_err, 1)) ||
+      // what a step or a read could see before it is written starts zeroed.  The
+      // planes need no initial contents: Vx is defined where vmask is set, every
+      // operand plane is written whole before its product, and nothing past n (m)
+      // entries of a column is used.
+      (st = A.get_filled({{&d.fz, sizeof(float) * k},
+                          {&d.nnz, sizeof(uint32_t) * k},
+                          {&d.val, 2 * sizeof(float) * k},
+                          {&d.status, sizeof(int)},
+                          {&d.planes_nnz, sizeof(uint32_t)},
+                          {&d.sel_hint, sizeof(float) * k},
+                          {&d.ctl, sizeof(uint32_t) * CTL_WORDS},
+                          {&d.vmask, sizeof(uint32_t) * k * (M.ldn / 32)}},
+                         0)) ||
+      (st = A.get_filled({{&d.max_nnz, sizeof(uint32_t)},
+                          {&d.iters, sizeof(int) * d.log_capacity},
+                          {&d.cards, sizeof(int) * d.log_capacity}},
+                         0xFF)) ||
       (lists && (st = A.get(&d.cmask, (size_t)k * (M.ldn / 32)))) ||
       (need_bf16 &&
        ((st = A.get(&d.Z_b, kz)) || (st = ensure_bf16_planes(h, mat, d.bf16_2 ? 3 : 1)))) ||
@@ -791,26 +803,10 @@ am24_status am24_batch_create(am24_handle h, am24_matrix mat, const am24_setting
     return st;
   }
   d.err = d.val + k;  // one copy reads both
-  // What a step or a read could see before it is written starts zeroed.  The
-  // planes need no initial contents: Vx is defined where vmask is set, every
-  // operand plane is written whole before its product, and nothing past n (m)
-  // entries of a column is used.
-  cudaError_t e = cudaSuccess;
-  if (!e) e = cudaMemsetAsync(d.val, 0, sizeof(float) * k, h->stream);
-  if (!e) e = cudaMemsetAsync(d.err, 0, sizeof(float) * k, h->stream);
-  if (!e) e = cudaMemsetAsync(d.fz, 0, sizeof(float) * k, h->stream);
-  if (!e) e = cudaMemsetAsync(d.nnz, 0, sizeof(uint32_t) * k, h->stream);
-  if (!e) e = cudaMemsetAsync(d.status, 0, sizeof(int), h->stream);
-  if (!e) e = cudaMemsetAsync(d.vmask, 0, sizeof(uint32_t) * k * (M.ldn / 32), h->stream);
-  if (!e) e = cudaMemsetAsync(d.max_nnz, 0xFF, sizeof(uint32_t), h->stream);
-  if (!e) e = cudaMemsetAsync(d.planes_nnz, 0, sizeof(uint32_t), h->stream);
-  if (!e) e = cudaMemsetAsync(d.sel_hint, 0, sizeof(float) * k, h->stream);
-  if (!e) e = cudaMemsetAsync(d.ctl, 0, sizeof(uint32_t) * CTL_WORDS, h->stream);
   d.row_scale = M.row_scale;
   d.bt_row_scale = M.bt_row_scale;
-  if (!e && d.mixed) e = reset_mixed(d, h->stream);
-  if (!e) e = cudaMemsetAsync(d.iters, 0xFF, sizeof(int) * d.log_capacity, h->stream);
-  if (!e) e = cudaMemsetAsync(d.cards, 0xFF, sizeof(int) * d.log_capacity, h->stream);
+  cudaError_t e = cudaSuccess;
+  if (d.mixed) e = reset_mixed(d, h->stream);
   if (!e) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
     delete b;

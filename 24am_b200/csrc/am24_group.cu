@@ -37,6 +37,10 @@ struct GroupSlot {
   std::unique_ptr<Allocs> mem;
 };
 
+// Words behind a problem's control words, in the same allocation: the device status,
+// then (on a 16-byte boundary) its k objectives and k changes.
+enum { RES_STATUS = GCTL_WORDS, RES_VAL = GCTL_WORDS + 4 };
+
 }  // namespace
 
 struct am24_group_s {
@@ -333,37 +337,37 @@ am24_status group_add_impl(am24_group g, am24_matrix mat, const am24_settings *s
   std::unique_ptr<Allocs> A(new Allocs(h->stream));
   am24_status st;
   if ((st = A->get(&P.Vx, kv)) || (st = A->get(&P.vmask, words)) ||
-      (st = A->get(&P.Vraw, kv)) || (st = A->get(&P.sel_hint, k)) || (st = A->get(&P.nnz, k)) ||
+      (st = A->get(&P.Vraw, kv)) ||
       (is_constrained(f) && (st = A->get(&P.cmask, words))) ||
       (st = A->get(&P.Z_hi, kz)) ||
       (st = A->get(&P.Z_h, zh_planes * kz)) || (st = A->get(&P.z_scale, k)) ||
       (st = A->get(&P.V_h, 2 * kv)) ||
       (st = A->get(&P.v_scale, k)) ||
       (st = A->get(&P.ws, ws_floats(P.splits1, P.m_tiles1, P.n_tiles1, P.bn))) ||
-      (st = A->get(&P.fz, k)) || (st = A->get(&P.val, k)) || (st = A->get(&P.err, k)) ||
-      (st = A->get(&P.max_err, 1)) || (st = A->get(&P.obj_part, (size_t)k * P.parts)) ||
-      (st = A->get(&P.nnz_part, (size_t)k * P.parts)) || (st = A->get(&P.ctl, GCTL_WORDS)) ||
-      (st = A->get(&P.status, 1)) ||
-      (mixed && ((st = A->get(&P.stable, k)) || (st = A->get(&P.phase, 4)) ||
-                 (st = A->get(&P.mask_hash, k)))))
+      (st = A->get(&P.obj_part, (size_t)k * P.parts)) ||
+      // a slot's memory may come back from the pool holding an earlier problem's
+      // state: what a step or a read could see before it is written starts zeroed
+      // (the planes need no contents, as a batch's do not)
+      (st = A->get_filled({{&P.sel_hint, sizeof(float) * k},
+                           {&P.nnz, sizeof(uint32_t) * k},
+                           {&P.fz, sizeof(float) * k},
+                           {&P.max_err, sizeof(float)},
+                           {&P.nnz_part, sizeof(float) * k * P.parts},
+                           {&P.ctl, sizeof(uint32_t) * (RES_VAL + 2 * (size_t)k)},
+                           {&P.stable, mixed ? sizeof(uint32_t) * k : 0},
+                           {&P.mask_hash, mixed ? sizeof(uint64_t) * k : 0}},
+                          0)) ||
+      (mixed && (st = A->get(&P.phase, 4))))
     return st;
+  // control words, status, objectives and changes side by side: a result reads them
+  // with one copy
+  P.status = reinterpret_cast<int *>(P.ctl + RES_STATUS);
+  P.val = reinterpret_cast<float *>(P.ctl + RES_VAL);
+  P.err = P.val + k;
   const cudaStream_t hs = h->stream;
-  // a slot's memory may come back from the pool holding an earlier problem's
-  // state: what a step or a read could see before it is written starts zeroed
-  // (the planes need no contents, as a batch's do not)
-  AM24_CUDA(cudaMemsetAsync(P.nnz_part, 0, sizeof(float) * k * P.parts, hs));
-  AM24_CUDA(cudaMemsetAsync(P.max_err, 0, sizeof(float), hs));
-  AM24_CUDA(cudaMemsetAsync(P.sel_hint, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.val, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.err, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.nnz, 0, sizeof(uint32_t) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.fz, 0, sizeof(float) * k, hs));
-  AM24_CUDA(cudaMemsetAsync(P.status, 0, sizeof(int), hs));
   if (mixed) {
-    AM24_CUDA(cudaMemsetAsync(P.stable, 0, sizeof(uint32_t) * k, hs));
     const uint32_t words[4] = {mixed_first_phase(s.lead_iterations), 0u, 0u, 0u};
     AM24_CUDA(cudaMemcpyAsync(P.phase, words, sizeof words, cudaMemcpyHostToDevice, hs));
-    AM24_CUDA(cudaMemsetAsync(P.mask_hash, 0, sizeof(uint64_t) * k, hs));
   }
   // control words: dense first step, and no step at all when max_iter is 0
   uint32_t ctl[GCTL_WORDS] = {};
@@ -519,19 +523,19 @@ am24_status am24_group_result(am24_group g, uint32_t problem, float *x, am24_sta
   am24_handle h = g->h;
   const cudaStream_t hs = h->stream;
   AM24_CUDA(cudaSetDevice(h->device));
-  uint32_t ctl[GCTL_WORDS];
-  AM24_TRY(read_ctl(g, sl, ctl));
-  int dev_status = 0;
-  AM24_CUDA(cudaMemcpy(&dev_status, P.status, sizeof(int), cudaMemcpyDeviceToHost));
+  const int k = P.k, n = P.n;
+  std::vector<uint32_t> ctl(RES_VAL + (size_t)k);
+  AM24_CUDA(cudaMemcpyAsync(ctl.data(), P.ctl, sizeof(uint32_t) * ctl.size(),
+                            cudaMemcpyDeviceToHost, hs));
+  AM24_CUDA(cudaStreamSynchronize(hs));
+  const int dev_status = (int)ctl[RES_STATUS];
   if (dev_status != 0) {
     char buf[96];
     snprintf(buf, sizeof buf, "device-side wait timed out (code 0x%x)", dev_status);
     return fail(AM24_ERR_DEVICE_TIMEOUT, buf);
   }
-  const int k = P.k, n = P.n;
   std::vector<float> val(k);
-  AM24_CUDA(cudaMemcpyAsync(val.data(), P.val, sizeof(float) * k, cudaMemcpyDeviceToHost, hs));
-  AM24_CUDA(cudaStreamSynchronize(hs));
+  std::memcpy(val.data(), ctl.data() + RES_VAL, sizeof(float) * k);
   // the reference's choice (sparse_PCA_solver.h:212-231): the first largest objective
   int sel = 0, degenerate = std::isnan(val[0]) ? 1 : 0;
   float bv = val[0];
@@ -543,11 +547,11 @@ am24_status am24_group_result(am24_group g, uint32_t problem, float *x, am24_sta
     }
   }
   Allocs local(hs);
-  float *xb = nullptr, *x_dev = nullptr;
-  double *ev_rows = nullptr;
-  AM24_TRY(local.get(&xb, n));
-  AM24_TRY(local.get(&x_dev, n));
-  AM24_TRY(local.get(&ev_rows, ev_partial_len(sl.mat->d)));
+  const size_t len = (size_t)round_up(n, 64);
+  float *xb = nullptr;
+  AM24_TRY(local.get(&xb, 2 * len + 2 * ev_partial_len(sl.mat->d)));
+  float *x_dev = xb + len;
+  double *ev_rows = reinterpret_cast<double *>(xb + 2 * len);
   AM24_CUDA(launch_masked_copy(P.Vx + (size_t)sel * P.ldn, P.vmask + (size_t)sel * (P.ldn / 32),
                                P.ldn, n, 1, xb, n, hs));
   AM24_CUDA(launch_finalize_x(xb, n, x_dev, hs));

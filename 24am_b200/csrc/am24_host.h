@@ -4,6 +4,8 @@
 // Not part of the public ABI.
 #pragma once
 #include <algorithm>
+#include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -74,6 +76,29 @@ struct Allocs {
     }
     ptrs.push_back(p);
     *out = static_cast<T *>(p);
+    return AM24_OK;
+  }
+  // Several arrays in one allocation, every byte `fill`, each on a 256-byte boundary: one
+  // pool request and one memset for the dozen small arrays that a batch starts defined
+  // (a call of either costs the host 2-3 us and the device as much).  Parts of no bytes
+  // are left out.
+  struct Part {
+    void *out;  // the address of the array's pointer
+    size_t bytes;
+  };
+  am24_status get_filled(std::initializer_list<Part> parts, int fill) {
+    size_t total = 0;
+    for (const Part &p : parts) total += (p.bytes + 255) / 256 * 256;
+    char *at = nullptr;
+    const am24_status st = get(&at, total);
+    if (st != AM24_OK) return st;
+    const cudaError_t e = cudaMemsetAsync(at, fill, total, stream);
+    if (e != cudaSuccess)
+      return fail(AM24_ERR_CUDA, std::string("device memset: ") + cudaGetErrorString(e));
+    for (const Part &p : parts) {
+      if (p.bytes) std::memcpy(p.out, &at, sizeof at);
+      at += (p.bytes + 255) / 256 * 256;
+    }
     return AM24_OK;
   }
 };

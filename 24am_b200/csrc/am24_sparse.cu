@@ -277,27 +277,17 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   AM24_TRY(A.get(&b.xmask, (size_t)(b.kp / 32) * (b.ldn / 32)));
   AM24_TRY(A.get(&b.Zs, (size_t)k * b.ldm));
   AM24_TRY(A.get(&b.Zt, (size_t)S.m * b.kp));
-  AM24_TRY(A.get(&b.fz, k));
   AM24_TRY(A.get(&b.val, k));
   AM24_TRY(A.get(&b.err, k));
   AM24_TRY(A.get(&b.max_err, 1));
   AM24_TRY(A.get(&b.sel_hint, k));
-  AM24_TRY(A.get(&b.obj_part, k));
-  AM24_TRY(A.get(&b.nnz_part, k));
-  AM24_TRY(A.get(&b.nnz, k));
   AM24_TRY(A.get(&b.max_nnz, 1));
   AM24_TRY(A.get(&b.ctl, CTL_WORDS));
-  AM24_TRY(A.get(&b.work, 1));
   AM24_TRY(A.get(&b.zgate, 1));
   AM24_TRY(A.get(&b.sum_v, k));
   AM24_TRY(A.get(&b.dot_mu, k));
-  AM24_TRY(A.get(&b.zsum, k));
-  AM24_TRY(A.get(&b.zdot, k));
   AM24_TRY(A.get(&b.zpart, 3 * (size_t)sparse_zblocks(S.m, b.kp) * b.kp));
   AM24_TRY(A.get(&b.zinv, b.kp));
-  AM24_TRY(A.get(&b.status, 1));
-  AM24_TRY(A.get(&b.iters, b.log_capacity));
-  AM24_TRY(A.get(&b.cards, b.log_capacity));
   AM24_TRY(A.get(&xb, n));
   AM24_TRY(A.get(&x_dev, n));
   AM24_TRY(A.get(&ev_scratch, sparse_ev_scratch(S)));
@@ -306,16 +296,18 @@ am24_status solve_sparse(am24_handle h, am24_matrix mat, float *x, am24_settings
   if (S.comps) AM24_TRY(A.get(&b.defl_a, (size_t)k * SP_DEFL_MAX));
   // what a step could see before it is written starts defined: pool memory can
   // hold an earlier call's state
-  AM24_CUDA(cudaMemsetAsync(b.work, 0, sizeof(unsigned long long), h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.fz, 0, sizeof(float) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.obj_part, 0, sizeof(float) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.nnz_part, 0, sizeof(float) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.nnz, 0, sizeof(uint32_t) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.zsum, 0, sizeof(double) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.zdot, 0, sizeof(double) * k, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.status, 0, sizeof(int), h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.iters, 0xFF, sizeof(int) * b.log_capacity, h->stream));
-  AM24_CUDA(cudaMemsetAsync(b.cards, 0xFF, sizeof(int) * b.log_capacity, h->stream));
+  AM24_TRY(A.get_filled({{&b.work, sizeof(unsigned long long)},
+                         {&b.fz, sizeof(float) * k},
+                         {&b.obj_part, sizeof(float) * k},
+                         {&b.nnz_part, sizeof(float) * k},
+                         {&b.nnz, sizeof(uint32_t) * k},
+                         {&b.zsum, sizeof(double) * k},
+                         {&b.zdot, sizeof(double) * k},
+                         {&b.status, sizeof(int)}},
+                        0));
+  AM24_TRY(A.get_filled({{&b.iters, sizeof(int) * b.log_capacity},
+                         {&b.cards, sizeof(int) * b.log_capacity}},
+                        0xFF));
   // the best loading so far starts as the caller's x (returned normalised
   // when no start ever improves on -1, as the reference returns it)
   AM24_CUDA(cudaMemcpyAsync(xb, x, sizeof(float) * n, cudaMemcpyHostToDevice, h->stream));

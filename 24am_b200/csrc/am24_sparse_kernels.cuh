@@ -435,9 +435,9 @@ __global__ void sp_zgate_kernel(const uint32_t *max_nnz, uint32_t cap,
 // them, SP_VEC starts per lane, and writes its sums to part[q][block][j] (q = 0
 // the norm's, 1 zsum's, 2 zdot's); sp_zsum_kernel adds the blocks up.
 // inv = null: the pass after the product; else (forms 4, 6) the second one, which
-// scales by inv[j].  What bounds it: the FP64 conversions and sums beside one read of
-// Z (and one write where the values change): 53 us for 40000 samples x 512 starts,
-// where a pass over start-major columns and their transposition took 92 + 140.
+// scales by inv[j].  What bounds it: one read of Z (and one write where the values
+// change): 53 us for 100000 samples x 512 starts (3.9 TB/s), where a pass over
+// start-major columns and their transposition took 92 + 140.
 __global__ void __launch_bounds__(SP_THREADS) sp_zpass_kernel(
     float *__restrict__ Zt, int kp, int m, int rows, int formulation,
     const float *__restrict__ inv, bool sums, const float *__restrict__ row_means,

@@ -22,8 +22,9 @@
 // With one MMA per K step (PairFP16x1) the loads bound the kernel: 64-byte rows
 // took 4.72 ms at 65536 x 8192 x 4096, 128-byte rows (whole L2 lines per
 // request, half the barrier traffic) take 3.59 ms; the split schemes gain 2-4 %
-// and run at the rate the power limit allows.  A stage holds a slab of PAIR_SLAB = 2 K blocks of 64 bytes, and a unit whose
-// blocks are odd in number issues the MMAs of the last slab's first block only.
+// and run at the rate the power limit allows.  A stage holds a slab of
+// PAIR_SLAB = 2 K blocks of 64 bytes, and a unit whose blocks are odd in number
+// issues the MMAs of the last slab's first block only.
 //
 // The tensor-core FP32 accumulation does not round to nearest; as in
 // gemm_tf32x3.cuh each TMEM buffer takes PROMO K slabs (S::PROMO_K elements: 48

@@ -670,18 +670,19 @@ __device__ __forceinline__ void z_store_split(const ZOut &z, int i, const float 
 __device__ __forceinline__ bool z_second_pass(const ZOut &z, int mode) {
   return mode == 2 || (mode == 0 && z.h);
 }
-// Samples i .. i + C - 1 (C = 1 or 4; beyond m they are zeros of the padding)
-// before the norm is known: their share of it into acc, and what can be stored
-// already.  KEEP: y is stored for a second pass, which reads it back.
+// Samples i .. i + C - 1 (C = 1 or 4) before the norm is known: their share of it
+// into acc, and what can be stored already.  Those beyond m are padding: stored,
+// but not of the norm (zero only while the loadings are finite: 0 x inf is NaN).
+// KEEP: y is stored for a second pass, which reads it back.
 template <int C, bool KEEP>
-__device__ __forceinline__ void z_emit(const ZOut &z, int mode, int i, const float (&y)[C],
+__device__ __forceinline__ void z_emit(const ZOut &z, int mode, int m, int i, const float (&y)[C],
                                        double &acc) {
   if (mode == 1) {
     alignas(16) uint16_t b[C], h[C];
     alignas(16) float sg[C], zero[C];
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      acc += (double)fabsf(y[c]);
+      if (C == 1 || i + c < m) acc += (double)fabsf(y[c]);
       sg[c] = sgnf(y[c]);
       zero[c] = 0.f;
       b[c] = bf16_sign(y[c]);
@@ -697,7 +698,7 @@ __device__ __forceinline__ void z_emit(const ZOut &z, int mode, int i, const flo
     alignas(16) uint16_t b[C];
 #pragma unroll
     for (int c = 0; c < C; c++) {
-      acc += (double)y[c] * (double)y[c];
+      if (C == 1 || i + c < m) acc += (double)y[c] * (double)y[c];
       b[c] = bf16_bits(y[c]);
     }
     if (z.lo) {
@@ -761,7 +762,7 @@ __device__ __forceinline__ void z_reduce_body(int mode, const float *__restrict_
       const size_t u = ((size_t)s * m_tiles + mt) * n_tiles + nt;
       y += ws[u * unit_stride + (size_t)c * BM + r];
     }
-    z_emit<1, true>(z, mode, i, {y}, acc);
+    z_emit<1, true>(z, mode, m, i, {y}, acc);
   }
   const double tot = block_sum(acc, red);
   if (z_second_pass(z, mode)) {
@@ -781,7 +782,7 @@ __device__ __forceinline__ void z_finish_body(int mode, int m, const ZOut &z) {
   double acc = 0.0;
   for (int i = 4 * threadIdx.x; i < m; i += 4 * blockDim.x) {
     const float4 y = *reinterpret_cast<const float4 *>(z.hi + i);
-    z_emit<4, true>(z, mode, i, {y.x, y.y, y.z, y.w}, acc);
+    z_emit<4, true>(z, mode, m, i, {y.x, y.y, y.z, y.w}, acc);
   }
   const double tot = block_sum(acc, red);
   if (z_second_pass(z, mode)) {
@@ -986,7 +987,7 @@ __device__ __forceinline__ void gather_narrow_body(int mode, const float *__rest
   }
   const float e[4] = {y.x, y.y, y.z, y.w};
   double acc = 0.0;
-  if (on) z_emit<4, false>(z, mode, 4 * i4, e, acc);
+  if (on) z_emit<4, false>(z, mode, m, 4 * i4, e, acc);
   const double tot = block_sum(acc, red);
   if (on && z_second_pass(z, mode)) z_emit2<4>(z, mode, z_scales(mode, tot), 4 * i4, e);
   if (threadIdx.x == 0) z_close(z, mode, tot);

@@ -35,14 +35,33 @@ namespace am24host {
 thread_local std::string g_last_error;
 }  // namespace am24host
 
-// Whether p lies in memory of the handle's own device, which its kernels can read.
-static bool own_memory(am24_handle h, const void *p) {
+// A caller's device array of `bytes` bytes from p: *in_place when a kernel can read
+// it as it stands, that is when it is floats of the handle's own device inside one
+// allocation; else (another device's or managed memory, an odd address, several
+// mappings in a row) the copies take it, which check their ranges themselves.  An
+// array that runs past what is mapped is refused here: a kernel would fault on it.
+static am24_status device_source(am24_handle h, const void *p, size_t bytes, bool *in_place) {
+  *in_place = false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    return AM24_OK;
   }
-  return at.type == cudaMemoryTypeDevice && at.device == h->device;
+  if (at.type != cudaMemoryTypeDevice || at.device != h->device || !h->range) return AM24_OK;
+  AM24_CUDA(cudaSetDevice(h->device));
+  const CUdeviceptr first = (CUdeviceptr)p, end = first + bytes;
+  for (CUdeviceptr a = first; a < end;) {
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUresult r = h->range(&base, &size, a);
+    if (a != first && (r == CUDA_ERROR_NOT_FOUND || r == CUDA_ERROR_INVALID_VALUE))
+      return fail(AM24_ERR_INVALID_ARG, "the device array ends " + std::to_string(end - a) +
+                                            " bytes past its allocation");
+    if (r != CUDA_SUCCESS || base + size <= a) return AM24_OK;
+    if (a == first) *in_place = base + size >= end && first % sizeof(float) == 0;
+    a = base + size;
+  }
+  return AM24_OK;
 }
 
 namespace am24host {
@@ -464,6 +483,9 @@ am24_status am24_create(am24_handle *out, int device) {
     return fail(AM24_ERR_CUDA, "cuTensorMapEncodeTiled entry point not available");
   }
   h->encode = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
+  if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) == cudaSuccess &&
+      q == cudaDriverEntryPointSuccess)
+    h->range = reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(fn);
   am24_status st = h->scratch.get(&h->ev_out, 1);
   if (st == AM24_OK && cudaMallocHost(reinterpret_cast<void **>(&h->flags),
                                       sizeof(uint32_t) * am24_handle_s::AHEAD) != cudaSuccess)
@@ -536,6 +558,9 @@ static am24_status create_matrix(am24_handle h, const float *B, int32_t ldB, uin
   if (ldB < (int32_t)m) return fail(AM24_ERR_INVALID_ARG, "ldB must be >= m");
   if (m > (1u << 30) || n > (1u << 30)) return fail(AM24_ERR_INVALID_ARG, "matrix too large");
   AM24_CUDA(cudaSetDevice(h->device));
+  bool in_place = false;
+  if (on_device)
+    AM24_TRY(device_source(h, B, sizeof(float) * ((size_t)(n - 1) * ldB + m), &in_place));
   auto *mat = new am24_matrix_s();
   if (ordered) {
     mat->mem.stream = h->stream;
@@ -553,12 +578,10 @@ static am24_status create_matrix(am24_handle h, const float *B, int32_t ldB, uin
     return st;
   }
   // one copy straight into Bc's layout, pad rows zeroed: a kernel for a source in
-  // this device's own memory, a 2-D copy otherwise (host, or another device's
-  // memory, which a kernel may not reach); the other layouts are made from Bc when
-  // a batch first needs them
+  // this device's own memory, a 2-D copy otherwise; the other layouts are made from
+  // Bc when a batch first needs them
   cudaError_t e = cudaSuccess;
-  const bool own = on_device && own_memory(h, B);
-  if (own) {
+  if (in_place) {
     e = launch_copy_matrix(M, B, ldB, h->stream);
   } else {
     if (M.ldm > (int)m)
@@ -882,7 +905,9 @@ am24_status am24_batch_load(am24_handle h, am24_batch b, const float *V, int32_t
   const int k = b->d.k;
   // read in place where a kernel can (this device's own memory), else staged in
   // Vraw by one contiguous copy
-  if (on_device && own_memory(h, V)) return load_from(h, b, V);
+  bool in_place = false;
+  if (on_device) AM24_TRY(device_source(h, V, sizeof(float) * (size_t)M.n * k, &in_place));
+  if (in_place) return load_from(h, b, V);
   AM24_CUDA(cudaMemcpyAsync(b->d.Vraw, V, sizeof(float) * (size_t)M.n * k,
                             on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                             h->stream));

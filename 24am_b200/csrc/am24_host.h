@@ -115,6 +115,7 @@ struct am24_handle_s {
   uint32_t *flags = nullptr;
   cudaEvent_t run_ev[AHEAD] = {};
   PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
+  PFN_cuMemGetAddressRange_v3020 range = nullptr;  // null: device arrays are always copied
   am24host::Allocs scratch;  // small per-handle buffers
   double *ev_out = nullptr;
 };

@@ -157,18 +157,14 @@ am24_status ensure_tf32_planes(am24_handle h, am24_matrix mat) {
 am24_status ensure_fp16_planes(am24_handle h, am24_matrix mat) {
   MatrixDev &M = mat->d;
   if (M.Bc_h2) return AM24_OK;
-  auto pad = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
-  const size_t c_bytes = pad(2 * sizeof(uint16_t) * (size_t)M.n * M.ldm);
-  const size_t t_bytes = pad(2 * sizeof(uint16_t) * (size_t)M.m * M.ldn);
-  const size_t n_bytes = pad(sizeof(float) * M.n), m_bytes = pad(sizeof(float) * M.m);
+  const Fp16Block at((size_t)M.m, (size_t)M.n);
   char *p = nullptr;
-  AM24_TRY(mat->mem.get(&p, c_bytes + t_bytes + n_bytes + m_bytes +
-                                sizeof(uint32_t) * ((size_t)M.n + M.m)));
+  AM24_TRY(mat->mem.get(&p, at.bytes));
   M.Bc_h2 = reinterpret_cast<uint16_t *>(p);
-  M.Bt_h2 = reinterpret_cast<uint16_t *>(p + c_bytes);
-  M.row_scale = reinterpret_cast<float *>(p + c_bytes + t_bytes);
-  M.bt_row_scale = reinterpret_cast<float *>(p + c_bytes + t_bytes + n_bytes);
-  M.fp16_keys = reinterpret_cast<uint32_t *>(p + c_bytes + t_bytes + n_bytes + m_bytes);
+  M.Bt_h2 = reinterpret_cast<uint16_t *>(p + at.bt);
+  M.row_scale = reinterpret_cast<float *>(p + at.row_scale);
+  M.bt_row_scale = reinterpret_cast<float *>(p + at.bt_row_scale);
+  M.fp16_keys = reinterpret_cast<uint32_t *>(p + at.keys);
   cudaError_t e = launch_prep_fp16(M, h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {

@@ -152,6 +152,19 @@ am24_status make_map_bf16(am24_handle h, CUtensorMap *map, const uint16_t *base,
 am24_status ensure_bf16_planes(am24_handle h, am24_matrix mat, int planes);
 am24_status ensure_tf32_planes(am24_handle h, am24_matrix mat);
 am24_status ensure_fp16_planes(am24_handle h, am24_matrix mat);
+// The one allocation of a matrix's FP16 planes: where each part begins, and its size.
+struct Fp16Block {
+  size_t bt, row_scale, bt_row_scale, keys, bytes;  // (the planes of B begin it)
+  Fp16Block(size_t m, size_t n) {
+    auto pad = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t ldm = (m + 31) / 32 * 32, ldn = (n + 31) / 32 * 32;
+    bt = pad(2 * sizeof(uint16_t) * n * ldm);
+    row_scale = bt + pad(2 * sizeof(uint16_t) * m * ldn);
+    bt_row_scale = row_scale + pad(sizeof(float) * n);
+    keys = bt_row_scale + pad(sizeof(float) * m);
+    bytes = keys + sizeof(uint32_t) * (n + m);
+  }
+};
 void choose_splits(int tiles, int kb_total, int sms, int *splits, int *kbps);
 am24_status validate_settings(const am24_settings *s);
 // The phase word a MIXED batch or problem starts in (lead_iterations > 0: the FP32 lead-in).

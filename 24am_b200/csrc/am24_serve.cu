@@ -59,11 +59,10 @@ struct ServeRequest {
 using RequestPtr = std::shared_ptr<ServeRequest>;
 
 // Device bytes of a matrix's layouts: FP32 B and the two FP16 planes of B and
-// of B^T with their scales, all made when the matrix is added.
+// of B^T with their scales and scratch, all made when the matrix is added.
 uint64_t matrix_bytes(uint32_t m, uint32_t n) {
-  const uint64_t ldm = (m + 31) / 32 * 32, ldn = (n + 31) / 32 * 32;
-  return 4ull * n * ldm + 2ull * 2 * n * ldm + 4ull * n + 2ull * 2 * m * ldn + 4ull * m +
-         4ull * m;
+  const uint64_t ldm = ((uint64_t)m + 31) / 32 * 32;
+  return 4ull * n * ldm + Fp16Block(m, n).bytes;
 }
 
 }  // namespace

@@ -2014,6 +2014,10 @@ __device__ uint32_t resolve_stop(uint32_t best, double bw, uint32_t *res,
 // predicates evaluated rank by rank.  lo_end is the largest value below the
 // set (0 for the whole column).  Returns the stopping rank and sets *w; NONE
 // when the set ran out first (len < n), and the caller walks the column.
+// It begins behind the ranks that a sorted candidate set has shown not to stop:
+// misc[SEEN] of them (0: none; below len), all the entries with keys of at least
+// misc[SEEN_KEY], their S1 and S2 at w_sh[1] and w_sh[2].
+enum { SEEN = 4, SEEN_KEY = 5, SET_KEY = 6 };  // words of misc
 template <bool EXACT, class Src>
 __device__ __noinline__ uint32_t exact_walk(Src src, uint32_t len, uint32_t n, double lo_end, float *cand,
                                double *p1, double *p2, uint32_t *hist, uint32_t *res,
@@ -2024,8 +2028,8 @@ __device__ __noinline__ uint32_t exact_walk(Src src, uint32_t len, uint32_t n, d
   uint32_t brk = NONE;
   const SelResult top = block_select_src(src, (int)len, 1u, hist, res);
   const double lim = __dsub_rn((double)__uint_as_float(top.key), 0.000001);
-  uint32_t consumed = 0, khi = NONE, ge_hi = 0;
-  double S1 = 0.0, S2 = 0.0;
+  uint32_t consumed = misc[SEEN], khi = consumed ? misc[SEEN_KEY] : NONE, ge_hi = consumed;
+  double S1 = w_sh[1], S2 = w_sh[2];
   while (true) {
     const uint32_t R = min(consumed + (uint32_t)SOFT_C, len);
     const uint32_t total = R - consumed;
@@ -2103,9 +2107,9 @@ __device__ __forceinline__ void soft_select_body(
   __shared__ uint32_t res[32];
   __shared__ double red[32];
   __shared__ uint32_t misc_raw[16];
-  __shared__ double w_shared;
+  __shared__ double w_shared[3];
   volatile uint32_t *misc = misc_raw;
-  double *w_sh = &w_shared;
+  double *w_sh = w_shared;
 
   const float *colg = Vraw + (size_t)j * ldv;
   // sqrt(s), sqrt(s)^2 as the double-precision reference forms them
@@ -2119,7 +2123,6 @@ __device__ __forceinline__ void soft_select_body(
   bool sparse = false;     // ... and the gathered pairs hold every kept entry
   uint32_t c_pairs = 0;
   double ss = 0.0, cnt = 0.0;
-  float new_hint = 0.f;
   // ---- candidate sets (1024 columns of 50000, s = 128: 186 us on the first
   // step where the histogram and the chunked walk took 780; 90 to 190 later,
   // where columns that outran the hint took 690): the (key, index) pairs with
@@ -2128,9 +2131,16 @@ __device__ __forceinline__ void soft_select_body(
   // hinted set; when that is empty, too large or ends before the stop, attempts
   // 1 and 2 take bounds from a sample of the column (4 s + 64 entries or twice
   // the set that was too small; then as many as fit)
+  // A set of attempts 1 and 2 that ends before the stop is not lost: the walks below
+  // begin behind it (256 columns of 9000, exact, supports of 4650: 317 us a select,
+  // 504 when they began at the first rank, 424 without the attempts)
+  constexpr uint32_t MOST = SOFT_HINT_CAP;
   const float hint = hints[j];
   uint32_t c_hint = 0;  // entries at or above the hinted bound
-  constexpr uint32_t MOST = SOFT_HINT_CAP;
+  if (threadIdx.x == 0) {
+    misc[SEEN] = 0;
+    w_sh[1] = w_sh[2] = 0.0;
+  }
   uint32_t want = s < MOST / 4u ? 4u * s + 64u : MOST;
   for (int attempt = hint > 0.f ? 0 : 1; attempt < 3 && brk == NONE; attempt++) {
     uint32_t c = 0, below_key = 0;
@@ -2150,6 +2160,7 @@ __device__ __forceinline__ void soft_select_body(
       if (bound) {
         c = gather_pairs_above<true>(colg, n, bound, pairs, SOFT_HINT_CAP, res);
         below_key = res[1];
+        if (threadIdx.x == 0) misc[SET_KEY] = bound;
       }
     }
     if (attempt == 0) c_hint = c;
@@ -2208,9 +2219,16 @@ __device__ __forceinline__ void soft_select_body(
         have_norm = true;
         sparse = true;
         c_pairs = c;
-        new_hint = next_hint(pairs, c, brk + 1u, brk + brk / 2u + 32u, SOFT_HINT_CAP, (float)w);
+        if (threadIdx.x == 0)
+          hints[j] = next_hint(pairs, c, brk + 1u, brk + brk / 2u + 32u, SOFT_HINT_CAP, (float)w);
       } else {
         want = max(want, 2u * c);
+        if (!listed && threadIdx.x == 0) {
+          misc[SEEN] = c;
+          misc[SEEN_KEY] = misc[SET_KEY];
+          w_sh[1] = p1[c - 1 - q0];
+          w_sh[2] = p2[c - 1 - q0];
+        }
       }
     }
     __syncthreads();
@@ -2227,12 +2245,15 @@ __device__ __forceinline__ void soft_select_body(
                             misc, w_sh, sq, sq2, &w);
   }
 
-  // ---- fast path: the highest bins holding at most SOFT_C values
+  // ---- fast path: the highest bins holding at most SOFT_C values (unless as many
+  // ranks are seen already)
   uint32_t c = 0, bstar = 0;
   bool hist_ok = false;  // hist holds the column's top-bit histogram
-  if (brk == NONE) {
+  if (brk == NONE && (misc[SEEN] < (uint32_t)SOFT_C || n > 8 * SOFT_C)) {
     key_histogram(colg, n, hist);
     hist_ok = true;
+  }
+  if (brk == NONE && misc[SEEN] < (uint32_t)SOFT_C) {
     find_rank_bin(hist, 2048, (uint32_t)SOFT_C + 1u, res);
     const bool whole = (uint32_t)n <= (uint32_t)SOFT_C;
     bstar = whole ? 0u : res[0] + 1u;  // gather bins >= bstar
@@ -2310,7 +2331,7 @@ __device__ __forceinline__ void soft_select_body(
     brk = exact_walk<EXACT>(ColumnSrc{colg}, (uint32_t)n, (uint32_t)n, 0.0, cand, p1, p2, hist,
                             res, red, misc, w_sh, sq, sq2, &w);
 
-  if (threadIdx.x == 0) hints[j] = sparse ? new_hint : (float)w;
+  if (threadIdx.x == 0 && !sparse) hints[j] = (float)w;
   // x = sgn(v)(|v| - w)_+ with w kept in double: a level that lands within
   // rounding of the largest |v| still leaves that entry non-zero, as in the
   // reference's double arithmetic.

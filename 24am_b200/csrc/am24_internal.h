@@ -277,7 +277,7 @@ struct GroupDev {
 // One grouped AM step of every live, unstopped problem; the plan kernel first.
 // grids: per-kernel persistent grid sizes (from grouped_grids()).
 struct GroupGrids {
-  int plan_threads, col, select_hard, select_soft, gather, gather_tile, fin, pairs;
+  int col, select_hard, select_soft, gather, gather_tile, fin;
 };
 cudaError_t grouped_grids(GroupGrids *g);
 // The streams and events of a step's branches.

@@ -2545,10 +2545,6 @@ __global__ void deflate_kernel(float *__restrict__ Bc, int ldm, int m,
 }
 
 // ------------------------------------------------------------ GEMM launch
-struct GemmCfg {
-  int bn, stages;
-};
-
 // Co-resident clusters of two CTAs for a pair kernel.
 template <class K>
 cudaError_t pair_clusters(K kern, int threads, int smem, int *out) {
@@ -3222,8 +3218,6 @@ cudaError_t grouped_grids(GroupGrids *gr) {
   if ((e = grouped_gemms_setup<GE_PARTIAL>(&c)) || (e = grouped_gemms_setup<GE_RAW>(&c)) ||
       (e = grouped_gemms_setup<GE_PL1>(&c)) || (e = grouped_gemms_setup<GE_PL0>(&c)))
     return e;
-  gr->plan_threads = PLAN_THREADS;
-  gr->pairs = c;
   if ((e = persistent_grid(g_z_reduce_kernel, 256, 0, &gr->col)) ||
       (e = persistent_grid(g_hard_select_kernel, HARD_THREADS, 0, &gr->select_hard)) ||
       (e = kernel_setup(g_soft_select_kernel<false>, SOFT_SMEM)) ||

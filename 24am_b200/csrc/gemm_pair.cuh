@@ -220,10 +220,13 @@ struct PairSmem {
 // The epilogue warps of a pair kernel: four per 32-lane quarter of tensor memory
 // (two for the narrowest tile), each with BN / PARTS columns of its 32 rows.  With
 // two per quarter the epilogue's instructions ran one per 7.5 cycles and warp, two
-// warps a scheduler.  With four, and tensor memory read 16 columns at a time (112
-// registers a thread in place of 168): 202 x 33654, 1005 starts 122 -> 100 us a
-// launch with the L1 penalty, 90 -> 62 with raw output; 2000 x 50000, 1024 starts
-// 430 -> 405.
+// warps a scheduler.  With four, and tensor memory read 16 columns at a time: 202 x
+// 33654, 1005 starts 122 -> 100 us a launch with the L1 penalty, 90 -> 62 with raw
+// output; 2000 x 50000, 1024 starts 430 -> 405.  Eighteen warps put five on two of a
+// multiprocessor's four register files, which leaves a thread 96 registers (168 with
+// ten warps) and costs spills at an N tile of 256: 64 bytes stored and 44 loaded a
+// thread with raw output, 48 to 68 and 108 to 144 with a penalty, 188 and 236 in the
+// grouped kernel's penalties.
 template <int BN>
 struct PairEpi {
   static constexpr int PARTS = BN >= 128 ? 4 : 2;

@@ -55,6 +55,7 @@ N_SAMPLES, P_FEATURES, RANK, NNZ_V, STARTS = SIZES["config1"]
 S_CONS, GAMMA_C, SEED = 16, 0.1, 1
 E2E_MAX_IT, E2E_TOL = 200, 1e-6
 CPU_SAMPLE_STARTS, CPU_SAMPLE_ITERS = 64, 3
+CPU_SAMPLE_STARTS_PORT = 4  # the one-core port takes 0.65 s a start-iteration: a minute
 def workload_name():
     tag = "config-1" if (N_SAMPLES, P_FEATURES) == SIZES["config1"][:2] else "profiling case"
     return (f"{tag} AM step: n={N_SAMPLES} samples x p={P_FEATURES} features (r={RANK}, "
@@ -191,6 +192,22 @@ def cpu_reference(B_host, steps, per_step_iters, starts, forms_per_step=8, first
                 cores = 1
             total_its += starts * int(r["it"])
     return total_its / total_s, cores, kind, total_its, total_s
+
+
+def cpu_sample(B_host):
+    """cpu_reference on the bounded sample of the full matrix that fits the code at
+    hand: the reference's where it was built, else this repository's port of it on one
+    core.  Its results, the starts sampled and the name of the code that ran."""
+    sys.path.insert(0, os.path.join(ROOT, "oracle"))
+    import pyoracle as po
+    if po.ref_available("openblas"):
+        code = "reference denseDataSolver<float> + OpenBLAS"
+    elif po.ref_available("naive"):
+        code = "reference denseDataSolver<float> + plain C BLAS"
+    else:
+        code = "one-core C port of the reference's solver"
+    starts = CPU_SAMPLE_STARTS_PORT if code.startswith("one-core") else CPU_SAMPLE_STARTS
+    return (*cpu_reference(B_host, 1, CPU_SAMPLE_ITERS, starts), starts, code)
 
 
 def fp64_oracle_check(am, M, B_host, gam, starts=64, iters=3):
@@ -910,11 +927,11 @@ def run_ours(args):
         Bnp = Dt.cpu().numpy().T  # n x p view, column-major
         import numpy as np
         Bnp = np.asfortranarray(Bnp)
-        v, cores, kind, its, secs = cpu_reference(Bnp, 1, CPU_SAMPLE_ITERS, CPU_SAMPLE_STARTS)
+        v, cores, kind, its, secs, starts, code = cpu_sample(Bnp)
         cpu = {"value": v, "unit": "start-it/s", "cores": cores, "kind": kind,
                "sample": f"8 formulations x {CPU_SAMPLE_ITERS} iterations x "
-                         f"{CPU_SAMPLE_STARTS} starts on the full matrix ({its} start-iterations, "
-                         f"{secs:.1f} s compute, reference denseDataSolver<float> + OpenBLAS)"}
+                         f"{starts} starts on the full matrix ({its} start-iterations, "
+                         f"{secs:.1f} s compute, {code})"}
         if not args.no_oracle_check:
             t0 = time.perf_counter()
             cpu["fp64_oracle_check"] = {

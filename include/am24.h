@@ -199,7 +199,8 @@ am24_status am24_solve_dense_f64(am24_handle h, const double *B, int32_t ldB, do
 
 /* ---- resident data matrices ---------------------------------------------- */
 /* Copies B (host, or device when on_device != 0) into the handle's layout and
- * keeps it until am24_matrix_destroy. */
+ * keeps it until am24_matrix_destroy.  A device array that runs past what is
+ * allocated is AM24_ERR_INVALID_ARG, here and in am24_batch_load. */
 am24_status am24_matrix_create_f32(am24_handle h, const float *B, int32_t ldB, uint32_t m,
                                    uint32_t n, int32_t on_device, am24_matrix *out);
 /* A resident matrix from compressed sparse columns, the input of the

@@ -508,6 +508,10 @@ am24_status am24_destroy(am24_handle h) {
   cudaStreamSynchronize(h->copy);
   cudaStreamSynchronize(h->stream);
   for (int i = 0; i < am24_handle_s::AHEAD; i++) cudaEventDestroy(h->run_ev[i]);
+  for (cudaEvent_t ev : h->branches.ev)
+    if (ev) cudaEventDestroy(ev);
+  for (cudaStream_t st : h->branches.side)
+    if (st) cudaStreamDestroy(st);
   cudaFreeHost(h->flags);
   cudaStreamDestroy(h->copy);
   cudaStreamDestroy(h->stream);

